@@ -20,6 +20,7 @@ struct Grid {
     int n[3];       // ghost-inclusive sizes (n[2] == 1 in 2D)
     long long s[3]; // strides (1, n0, n0*n1)
     long long N;    // cells per scalar field
+    int pr[3] = {0, 0, 0};   // multigrid: the first pr[e] cells along e cover two cells of the next finer level
 
     __host__ __device__ bool isper(int d) const { return (per >> d) & 1; }
 };

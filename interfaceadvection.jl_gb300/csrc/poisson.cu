@@ -6,10 +6,11 @@
 // + D_I x_I with D_I = -Σ_i (L[I,i] + L[I+δi,i]); L = μ₀ = 1/ρ on faces, zero
 // on wall faces, periodic dimensions wrap.  The solver is this library's own:
 //
-//  * geometric multigrid on cell-centred levels (2x coarsening while every
-//    interior extent is even and >= 4); coarse face coefficient = ½ Σ of the
-//    2^(D-1) fine faces it covers; restriction sums the 2^D children,
-//    prolongation injects; red-black Gauss-Seidel, ν₁ sweeps red→black
+//  * geometric multigrid on cell-centred levels of any size (a dimension halves,
+//    an odd one with a single cell left at its end); coarse face coefficient =
+//    Σ of the fine faces it covers times the ratio of the cell distances (½ away
+//    from single cells); restriction sums the children, prolongation injects;
+//    red-black Gauss-Seidel, ν₁ sweeps red→black
 //    before and ν₂ black→red after, so the V-cycle is a symmetric
 //    preconditioner; the coarsest level is solved by one block with a fixed
 //    number of symmetric sweeps on the mean-free right-hand side;
@@ -28,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "capi_internal.cuh"
@@ -41,23 +43,6 @@ namespace {
 
 inline dim3 blk() { return dim3(32, 8, 1); }
 inline dim3 grd(const Grid& g) { return dim3((g.n[0] + 31) / 32, (g.n[1] + 7) / 8, g.n[2]); }
-
-// neighbour offset of interior cell coordinate ci along dimension i (periodic wrap;
-// on a wall the ghost is read but its face coefficient is zero)
-__device__ __forceinline__ long long lo_off(const Grid& g, int i, int ci) {
-    return (g.isper(i) && ci == 1) ? (long long)(g.n[i] - 3) * g.s[i] : -g.s[i];
-}
-__device__ __forceinline__ long long hi_off(const Grid& g, int i, int ci) {
-    return (g.isper(i) && ci == g.n[i] - 2) ? -(long long)(g.n[i] - 3) * g.s[i] : g.s[i];
-}
-
-template <class T>
-__device__ __forceinline__ T offdiag(const Grid& g, const T* L, const T* x, long long I, const int c[3]) {
-    T a = T(0);
-    for (int i = 0; i < g.D; ++i)
-        a += L[I + i * g.N] * x[I + lo_off(g, i, c[i])] + L[I + g.s[i] + i * g.N] * x[I + hi_off(g, i, c[i])];
-    return a;
-}
 
 // face coefficient as the arithmetic type of the sweep (the finest mixed level may store them as FP16)
 __device__ __forceinline__ float cf(float v) { return v; }
@@ -83,7 +68,7 @@ __device__ __forceinline__ Nb nb_of(const Grid& g, int x, int y, int z) {
     }
     return o;
 }
-// Σ_i L[I,i] v[I-δi] + L[I+δi,i] v[I+δi]  (same order as offdiag)
+// Σ_i L[I,i] v[I-δi] + L[I+δi,i] v[I+δi]
 template <int D, class T, class TL>
 __device__ __forceinline__ T off7(const Grid& g, const TL* __restrict__ L, const T* v, int I, const Nb& o) {
     const int s1 = int(g.s[1]), s2 = int(g.s[2]);
@@ -145,10 +130,48 @@ __global__ void set_diag_k(Grid g, const T* __restrict__ L, T* __restrict__ iD) 
     iD[I] = (dd * dd < T(2) * eps) ? T(0) : T(1) / dd;
 }
 
-// Coarse face coefficients: ½ Σ over the fine faces covering each coarse face
-// (all coarse faces 1..n-1 along i, interior elsewhere).
+// Coarsening along a dimension e of n cells: the first pr[e] coarse cells cover two fine cells each, the
+// others one.  A dimension between walls takes (n+1)/2 coarse cells (one single when n is odd); a periodic
+// one the next even number of them, so that the red-black colouring closes across the wrap on every coarse
+// level (2 singles when n/2 is odd), and one cell after two (its faces then join the cell to itself and
+// carry no coefficient).
+// Fine cell c lies in coarse cell mg_parent; coarse cell c covers mg_children fine cells from mg_child on.
+__device__ __forceinline__ int mg_parent(const Grid& gc, int e, int c) { return max((c + 1) >> 1, c - gc.pr[e]); }
+__device__ __forceinline__ int mg_child(const Grid& gc, int e, int c) { return c <= gc.pr[e] ? 2 * c - 1 : c + gc.pr[e]; }
+__device__ __forceinline__ int mg_children(const Grid& gc, int e, int c) { return c <= gc.pr[e] ? 2 : 1; }
+// REG: every coarse cell covers two fine ones along each dimension, so that the parent is (c+1)/2; on the finest
+// levels of a large grid the general form's extra index arithmetic costs 8 to 16 % of a kernel's time.
+template <bool REG>
+__device__ __forceinline__ int mg_up(const Grid& gc, int e, int c) { return REG ? (c + 1) >> 1 : mg_parent(gc, e, c); }
+template <bool REG>
+__device__ __forceinline__ long long mg_parent_cell(const Grid& gc, int x, int y, int z) {
+    return lin(gc, mg_up<REG>(gc, 0, x), mg_up<REG>(gc, 1, y), gc.D == 3 ? mg_up<REG>(gc, 2, z) : 0);
+}
+inline bool mg_regular(const Grid& g, const Grid& gc) {
+    for (int e = 0; e < g.D; ++e)
+        if (2 * gc.pr[e] != g.n[e] - 2) return false;
+    return true;
+}
+// A periodic dimension with an odd number of cells (possible on the finest level only) puts two cells of one
+// colour next to each other across the wrap.  A half-sweep there runs in passes: cells are told apart by the
+// set of such dimensions in whose last plane they lie, and neighbours across a wrap differ in that set.
+__host__ __device__ inline int wrap_conflicts(const Grid& g) {
+    int m = 0;
+    for (int e = 0; e < g.D; ++e)
+        if (g.isper(e) && (g.n[e] & 1) && g.n[e] > 3) m |= 1 << e;
+    return m;
+}
+__device__ __forceinline__ int wrap_class(const Grid& g, int conflicts, int x, int y, int z) {
+    return (((conflicts & 1) && x == g.n[0] - 2) ? 1 : 0) | (((conflicts & 2) && y == g.n[1] - 2) ? 2 : 0) |
+           (((conflicts & 4) && z == g.n[2] - 2) ? 4 : 0);
+}
+
+// Coarse face coefficients: Σ over the fine faces covering each coarse face times ratio[e][c], the distance of
+// the fine cells beside face c along e over that of the coarse cells (½ between coarse cells of two fine ones);
+// all coarse faces 1..n-1 along i, interior elsewhere.
 template <class T>
-__global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, T* __restrict__ Lc) {
+__global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, const double* __restrict__ ratio,
+                             T* __restrict__ Lc) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
     if (x >= gc.n[0] || y >= gc.n[1]) return;
@@ -161,11 +184,11 @@ __global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, T* __re
             if (c[e] < 1 || c[e] > hi) ok = false;
         }
         if (!ok) continue;
-        // fine base cell of the face: coordinate 2c-1 in every dimension
-        int fb[3] = {2 * c[0] - 1, 2 * c[1] - 1, gc.D == 3 ? 2 * c[2] - 1 : 0};
+        // fine base cell of the face: the first child in every dimension
+        int fb[3] = {mg_child(gc, 0, c[0]), mg_child(gc, 1, c[1]), gc.D == 3 ? mg_child(gc, 2, c[2]) : 0};
         T s = T(0);
         const int o1 = (i == 0) ? 1 : 0, o2 = (i == 2) ? 1 : 2;   // the other dimensions
-        const int n1 = 2, n2 = (gc.D == 3) ? 2 : 1;
+        const int n1 = mg_children(gc, o1, c[o1]), n2 = (gc.D == 3) ? mg_children(gc, o2, c[o2]) : 1;
         for (int b = 0; b < n2; ++b)
             for (int a = 0; a < n1; ++a) {
                 int q[3] = {fb[0], fb[1], fb[2]};
@@ -173,7 +196,7 @@ __global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, T* __re
                 if (gc.D == 3) q[o2] += b;
                 s += Lf[lin(gf, q[0], q[1], q[2]) + i * gf.N];
             }
-        Lc[Ic + i * gc.N] = T(0.5) * s;
+        Lc[Ic + i * gc.N] = T(ratio[(i > 0 ? gc.n[0] : 0) + (i > 1 ? gc.n[1] : 0) + c[i]]) * s;
     }
 }
 
@@ -196,9 +219,9 @@ inline dim3 pair_tile_grid(const Grid& g) {
     const int pairs = (g.n[0] - 2 + 1) / 2;
     return dim3((pairs + 31) / 32, (g.n[1] - 2 + 7) / 8, g.D == 3 ? (g.n[2] - 2 + RB_ZT - 1) / RB_ZT : 1);
 }
-template <class T, int D, bool PROL = false, class TL = T>
+template <class T, int D, bool PROL = false, class TL = T, bool REG = true>
 __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, const T* __restrict__ b,
-                            T* __restrict__ xv, int color, T omega, Grid gc = Grid(),
+                            T* __restrict__ xv, int color, T omega, int conflicts, int cls, Grid gc = Grid(),
                             const T* __restrict__ xc = nullptr) {
     const int y = y0 + int(blockIdx.y * blockDim.y + threadIdx.y);   // rows [y0, y1) of the interior
     if (y >= y1) return;
@@ -210,6 +233,8 @@ __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, co
     auto cell_of = [&](int z) {
         int x = xp;
         if (((x + y + z) & 1) != color) ++x;
+        // with wrap conflicts, a pass takes the cells of its class alone (any x past the row is no cell)
+        if (conflicts && wrap_class(g, conflicts, x, y, z) != cls) x = g.n[0];
         return x;
     };
     auto load = [&](int x, int z, int& I, T& off, T& dd, T& bv, T& xo) {
@@ -220,7 +245,7 @@ __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, co
         bv = b[I];
         if (omega != T(1)) {
             xo = xv[I];
-            if (PROL) xo += xc[lin(gc, (x + 1) / 2, (y + 1) / 2, D == 3 ? (z + 1) / 2 : 0)];
+            if (PROL) xo += xc[mg_parent_cell<REG>(gc, x, y, z)];
         }
     };
     auto store = [&](int I, T off, T dd, T bv, T xo) {
@@ -264,7 +289,7 @@ __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, co
 // pre-smoothing from x = 0 (the first red sweep, whose neighbours are zero) and x + the
 // injected coarse correction for the post-smoothing (prolong_k's values, interior cells only).  The red cells are written only for
 // a pre-smoothing of one sweep (write_red), whose red values are part of its result.
-template <class T, bool PROL>
+template <class T, bool PROL, bool REG>
 __device__ __forceinline__ T first_nb(const Grid& g, const Grid& gc, const T* __restrict__ b,
                                       const T* __restrict__ iD, const T* __restrict__ xc, const T* xv, int J,
                                       int cx, int cy, int cz, T omega) {
@@ -272,11 +297,11 @@ __device__ __forceinline__ T first_nb(const Grid& g, const Grid& gc, const T* __
     const bool in = cx >= 1 && cx <= g.n[0] - 2 && cy >= 1 && cy <= g.n[1] - 2 &&
                     (g.D == 2 || (cz >= 1 && cz <= g.n[2] - 2));
     if (!in) return xv[J];
-    if (PROL) return xv[J] + xc[lin(gc, (cx + 1) / 2, (cy + 1) / 2, g.D == 3 ? (cz + 1) / 2 : 0)];
+    if (PROL) return xv[J] + xc[mg_parent_cell<REG>(gc, cx, cy, cz)];
     return omega == T(1) ? b[J] * iD[J] : omega * (b[J] * iD[J]);
 }
 
-template <class T, int D, bool PROL, class TL = T>
+template <class T, int D, bool PROL, class TL = T, bool REG = true>
 __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restrict__ L, const T* __restrict__ b,
                              const T* __restrict__ iD, const T* __restrict__ xc, T* __restrict__ xv, int write_red,
                              T omega) {
@@ -299,14 +324,28 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
     // whichever way the values were found)
     T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
     if (x >= 2 && x <= g.n[0] - 3 && y >= 2 && y <= g.n[1] - 3 && (D == 2 || (z >= 2 && z <= g.n[2] - 3))) {
-        // every neighbour interior, no wrap: the coarse parent of the neighbour below (above) along
-        // e is the cell's own parent, or the one below (above) when the coordinate is odd (even)
+        // every neighbour interior, no wrap
         const int J[6] = {I - 1, I + 1, I - s1, I + s1, I - s2, I + s2};
         if (PROL) {
             const int g1 = int(gc.s[1]), g2 = int(gc.s[2]);
-            const int P = (x + 1) / 2 + ((y + 1) / 2) * g1 + (D == 3 ? ((z + 1) / 2) * g2 : 0);
-            const int Pn[6] = {P - ((x & 1) ? 1 : 0), P + ((x & 1) ? 0 : 1), P - ((y & 1) ? g1 : 0),
-                               P + ((y & 1) ? 0 : g1), P - ((z & 1) ? g2 : 0), P + ((z & 1) ? 0 : g2)};
+            const int px = mg_up<REG>(gc, 0, x), py = mg_up<REG>(gc, 1, y) * g1, pz = D == 3 ? mg_up<REG>(gc, 2, z) * g2 : 0;
+            const int P = px + py + pz;
+            int Pn[6];
+            if (REG) {   // the cell's own parent, or the one below (above) when the coordinate is odd (even)
+                Pn[0] = P - ((x & 1) ? 1 : 0);
+                Pn[1] = P + ((x & 1) ? 0 : 1);
+                Pn[2] = P - ((y & 1) ? g1 : 0);
+                Pn[3] = P + ((y & 1) ? 0 : g1);
+                Pn[4] = P - ((z & 1) ? g2 : 0);
+                Pn[5] = P + ((z & 1) ? 0 : g2);
+            } else {
+                Pn[0] = P - px + mg_up<REG>(gc, 0, x - 1);
+                Pn[1] = P - px + mg_up<REG>(gc, 0, x + 1);
+                Pn[2] = P - py + mg_up<REG>(gc, 1, y - 1) * g1;
+                Pn[3] = P - py + mg_up<REG>(gc, 1, y + 1) * g1;
+                Pn[4] = P - pz + (D == 3 ? mg_up<REG>(gc, 2, z - 1) * g2 : 0);
+                Pn[5] = P - pz + (D == 3 ? mg_up<REG>(gc, 2, z + 1) * g2 : 0);
+            }
 #pragma unroll
             for (int q = 0; q < 2 * D; ++q) v[q] = xv[J[q]] + xc[Pn[q]];
         } else {
@@ -317,14 +356,14 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
         const Nb o = nb_of<D>(g, x, y, z);
         const int xl = (g.isper(0) && x == 1) ? g.n[0] - 2 : x - 1, xh = (g.isper(0) && x == g.n[0] - 2) ? 1 : x + 1;
         const int yl = (g.isper(1) && y == 1) ? g.n[1] - 2 : y - 1, yh = (g.isper(1) && y == g.n[1] - 2) ? 1 : y + 1;
-        v[0] = first_nb<T, PROL>(g, gc, b, iD, xc, xv, I + o.xl, xl, y, z, omega);
-        v[1] = first_nb<T, PROL>(g, gc, b, iD, xc, xv, I + o.xh, xh, y, z, omega);
-        v[2] = first_nb<T, PROL>(g, gc, b, iD, xc, xv, I + o.yl, x, yl, z, omega);
-        v[3] = first_nb<T, PROL>(g, gc, b, iD, xc, xv, I + o.yh, x, yh, z, omega);
+        v[0] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.xl, xl, y, z, omega);
+        v[1] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.xh, xh, y, z, omega);
+        v[2] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.yl, x, yl, z, omega);
+        v[3] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.yh, x, yh, z, omega);
         if (D == 3) {
             const int zl = (g.isper(2) && z == 1) ? g.n[2] - 2 : z - 1, zh = (g.isper(2) && z == g.n[2] - 2) ? 1 : z + 1;
-            v[4] = first_nb<T, PROL>(g, gc, b, iD, xc, xv, I + o.zl, x, y, zl, omega);
-            v[5] = first_nb<T, PROL>(g, gc, b, iD, xc, xv, I + o.zh, x, y, zh, omega);
+            v[4] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.zl, x, y, zl, omega);
+            v[5] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.zh, x, y, zh, omega);
         }
     }
     T a = cf(L[I]) * v[0] + cf(L[I + 1]) * v[1];
@@ -337,7 +376,7 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
     if (omega == T(1)) {
         xv[I] = gs;
     } else if (PROL) {   // over-relaxation from the prolongated value of this (black) cell
-        const T xo = xv[I] + xc[lin(gc, (x + 1) / 2, (y + 1) / 2, D == 3 ? (z + 1) / 2 : 0)];
+        const T xo = xv[I] + xc[mg_parent_cell<REG>(gc, x, y, z)];
         xv[I] = xo + omega * (gs - xo);
     } else {             // from x = 0
         xv[I] = omega * gs;
@@ -543,9 +582,9 @@ __global__ void residual_k(Grid g, const T* __restrict__ L, const T* __restrict_
     r[I] = b[I] - (off7<D>(g, L, xv, I, o) + diag7<D>(g, L, I) * xv[I]);
 }
 
-// residual of the 2^D fine children of each coarse cell, summed straight into the coarse
+// residual of the (at most 2^D) fine children of each coarse cell, summed straight into the coarse
 // right-hand side (residual_k + restrict_k without the fine residual array; same sums, same order)
-template <class T, int D, class TL = T>
+template <class T, int D, class TL = T, bool REG = true>
 __global__ void resid_restrict_k(Grid gc, int yc0, int yc1, Grid gf, const TL* __restrict__ L,
                                  const T* __restrict__ b, const T* __restrict__ xv, T* __restrict__ bc) {
     const int xc = 1 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -554,10 +593,14 @@ __global__ void resid_restrict_k(Grid gc, int yc0, int yc1, Grid gf, const TL* _
     if (xc > gc.n[0] - 2 || yc >= yc1) return;
     const int s1 = int(gf.s[1]), s2 = int(gf.s[2]);
     T sum = T(0);
-    for (int k = 0; k < (D == 3 ? 2 : 1); ++k)
-        for (int j = 0; j < 2; ++j)
-            for (int i = 0; i < 2; ++i) {
-                const int x = 2 * xc - 1 + i, y = 2 * yc - 1 + j, z = D == 3 ? 2 * zc - 1 + k : 0;
+    const int fx = REG ? 2 * xc - 1 : mg_child(gc, 0, xc), fy = REG ? 2 * yc - 1 : mg_child(gc, 1, yc);
+    const int fz = D == 3 ? (REG ? 2 * zc - 1 : mg_child(gc, 2, zc)) : 0;
+    const int mx = REG ? 2 : mg_children(gc, 0, xc), my = REG ? 2 : mg_children(gc, 1, yc);
+    const int mz = D == 3 ? (REG ? 2 : mg_children(gc, 2, zc)) : 1;
+    for (int k = 0; k < mz; ++k)
+        for (int j = 0; j < my; ++j)
+            for (int i = 0; i < mx; ++i) {
+                const int x = fx + i, y = fy + j, z = fz + k;
                 const int I = x + y * s1 + z * s2;
                 const Nb o = nb_of<D>(gf, x, y, z);
                 sum += b[I] - (off7<D>(gf, L, xv, I, o) + diag7<D>(gf, L, I) * xv[I]);
@@ -569,64 +612,149 @@ template <class T>
 __global__ void prolong_k(Grid gf, Grid gc, const T* __restrict__ xc, T* __restrict__ xf) {
     const Grid& g = gf;
     INTERIOR_XYZ
-    const long long P = lin(gc, (c[0] + 1) / 2, (c[1] + 1) / 2, g.D == 3 ? (c[2] + 1) / 2 : 0);
-    xf[I] += xc[P];
+    xf[I] += xc[mg_parent_cell<false>(gc, c[0], c[1], c[2])];
 }
 
-// Coarsest level: one block, mean-free right-hand side, nuc symmetric red-black sweeps from zero.
+// The small levels of the V-cycle in one launch: a single block runs the whole cycle below (and on) the first
+// level of at most tail_pairs<T>() pairs of cells, with x and b of every such level in shared memory and a block barrier
+// between the stages.  The stages are those of the levels above (first red half-sweep from zero, relaxed red-black
+// half-sweeps, residual restriction, prolongation); the coarsest level is solved by nuc symmetric sweeps on its
+// mean-free right-hand side (a colour swept twice in a row keeps its values, so those sweeps are skipped).
+// What bounds it: the chain of barriers and shared-memory latencies, about 0.3 us a stage, where a launch of its
+// own takes 2 to 3 us whatever the size.
+constexpr int TAIL_MAX = 16, TAIL_THREADS = 1024, TAIL_PAIRS = 2;
 template <class T>
-__global__ void coarse_k(Grid g, const T* __restrict__ L, const T* __restrict__ iD, T* __restrict__ b,
-                         T* __restrict__ xv, int nuc) {
-    // the sweeps run on a shared-memory copy of x when the level fits (it holds at most a few
-    // hundred cells), with 32-bit cell coordinates
-    constexpr int SMAX = 4096;
-    __shared__ double red[1024];
-    __shared__ T xs[SMAX];
-    const int total = int(g.N);
-    const bool sm = total <= SMAX;
-    T* xw = sm ? xs : xv;
-    auto coords = [&](int q, int c[3]) {
-        c[0] = q % g.n[0];
-        const int r = q / g.n[0];
-        c[1] = r % g.n[1];
-        c[2] = r / g.n[1];
+struct TailArgs {
+    int nl;                                          // levels; 0 is the largest
+    Grid g[TAIL_MAX];
+    const T* L[TAIL_MAX];
+    const T* iD[TAIL_MAX];
+    int off[TAIL_MAX];                               // x of the level in shared memory; b follows it
+    int nu1[TAIL_MAX], nu2[TAIL_MAX];
+    int nuc, total;                                  // total: shared values in all
+    T omega;
+    const T* b;                                      // right-hand side and result of level 0
+    T* x;
+};
+
+template <class T, int D>
+__global__ void __launch_bounds__(TAIL_THREADS) mg_tail_k(const __grid_constant__ TailArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char tail_raw[];
+    T* sm = reinterpret_cast<T*>(tail_raw);
+    __shared__ T mean_s;
+    const int tid = threadIdx.x;
+    // every interior cell of a level, as f(x, y, z, index)
+    auto cells = [&](const Grid& g, auto&& f) {
+        const int nx = g.n[0] - 2, ny = g.n[1] - 2, nz = D == 3 ? g.n[2] - 2 : 1, n = nx * ny * nz;
+        for (int t = tid; t < n; t += TAIL_THREADS) {
+            const int r = t / nx, x = 1 + t - r * nx, rz = r / ny, y = 1 + r - rz * ny, z = D == 3 ? 1 + rz : 0;
+            f(x, y, z, x + y * int(g.s[1]) + z * int(g.s[2]));
+        }
     };
-    double acc = 0.0;
-    for (int q = threadIdx.x; q < total; q += blockDim.x) {
-        int c[3];
-        coords(q, c);
-        if (is_interior(g, c)) acc += double(b[q]);
-    }
-    red[threadIdx.x] = acc;
+    // nh half-sweeps x += omega (x_GS - x) of alternating colours from color0 on, after x += P(x of level l + 1)
+    // when prol.  A thread keeps its (at most TAIL_PAIRS) pairs of cells in x, decoded once: the divisions would
+    // otherwise be most of a stage's instructions.
+    auto sweeps = [&](int l, int nh, int color0, T om, bool prol) {
+        const Grid& g = a.g[l];
+        T* xv = sm + a.off[l];
+        const T* b = xv + g.N;
+        const T* __restrict__ L = a.L[l];
+        const T* __restrict__ iD = a.iD[l];
+        const int N = int(g.N), s1 = int(g.s[1]), s2 = int(g.s[2]);
+        const int nx = g.n[0] - 2, ny = g.n[1] - 2, nz = D == 3 ? g.n[2] - 2 : 1;
+        const int hx = (nx + 1) / 2, n = hx * ny * nz, conflicts = wrap_conflicts(g);
+        int px[TAIL_PAIRS], py[TAIL_PAIRS], pz[TAIL_PAIRS];   // px = 0: no pair
+#pragma unroll
+        for (int k = 0; k < TAIL_PAIRS; ++k) {
+            const int t = tid + k * TAIL_THREADS, r = t / hx, rz = r / ny;
+            px[k] = t < n ? 1 + 2 * (t - r * hx) : 0;
+            py[k] = 1 + r - rz * ny;
+            pz[k] = D == 3 ? 1 + rz : 0;
+        }
+        if (prol) {
+            const Grid& gc = a.g[l + 1];
+            const T* xc = sm + a.off[l + 1];
+#pragma unroll
+            for (int k = 0; k < TAIL_PAIRS; ++k) {
+                if (!px[k]) continue;
+                const int row = py[k] * s1 + pz[k] * s2;
+                const int up = mg_parent(gc, 1, py[k]) * int(gc.s[1]) + (D == 3 ? mg_parent(gc, 2, pz[k]) * int(gc.s[2]) : 0);
+                xv[row + px[k]] += xc[up + mg_parent(gc, 0, px[k])];
+                if (px[k] < nx) xv[row + px[k] + 1] += xc[up + mg_parent(gc, 0, px[k] + 1)];
+            }
+            __syncthreads();
+        }
+        for (int s = 0; s < nh; ++s) {
+            const int color = (color0 + s) & 1;
+            for (int cls = 0; cls <= conflicts; ++cls) {
+                if (cls & ~conflicts) continue;
+#pragma unroll
+                for (int k = 0; k < TAIL_PAIRS; ++k) {
+                    const int x = px[k] + (((px[k] + py[k] + pz[k]) & 1) != color), y = py[k], z = pz[k];
+                    if (!px[k] || x > nx || (conflicts && wrap_class(g, conflicts, x, y, z) != cls)) continue;
+                    const int I = x + y * s1 + z * s2;
+                    const Nb o = nb_of<D>(g, x, y, z);
+                    T off = __ldg(L + I) * xv[I + o.xl] + __ldg(L + I + 1) * xv[I + o.xh];
+                    off += __ldg(L + N + I) * xv[I + o.yl] + __ldg(L + N + I + s1) * xv[I + o.yh];
+                    if (D == 3) off += __ldg(L + 2 * N + I) * xv[I + o.zl] + __ldg(L + 2 * N + I + s2) * xv[I + o.zh];
+                    const T gs = (b[I] - off) * __ldg(iD + I);
+                    xv[I] = om == T(1) ? gs : xv[I] + om * (gs - xv[I]);
+                }
+                __syncthreads();
+            }
+        }
+    };
+    // level 0's right-hand side (its ghost entries are zero); everything else from zero
+    const int N0 = int(a.g[0].N);
+    for (int q = tid; q < a.total; q += TAIL_THREADS) sm[q] = q >= N0 && q < 2 * N0 ? a.b[q - N0] : T(0);
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    const int last = a.nl - 1;
+    for (int l = 0; l < last; ++l) {
+        const Grid &g = a.g[l], &gc = a.g[l + 1];
+        T* xv = sm + a.off[l];
+        const T* b = xv + g.N;
+        sweeps(l, 2 * a.nu1[l], 0, a.omega, false);
+        T* bc = sm + a.off[l + 1] + gc.N;
+        cells(gc, [&](int X, int Y, int Z, int Ic) {
+            const int fx = mg_child(gc, 0, X), fy = mg_child(gc, 1, Y), fz = D == 3 ? mg_child(gc, 2, Z) : 0;
+            const int mx = mg_children(gc, 0, X), my = mg_children(gc, 1, Y), mz = D == 3 ? mg_children(gc, 2, Z) : 1;
+            T sum = T(0);
+            for (int k = 0; k < mz; ++k)
+                for (int j = 0; j < my; ++j)
+                    for (int i = 0; i < mx; ++i) {
+                        const int x = fx + i, y = fy + j, z = fz + k, I = x + y * int(g.s[1]) + z * int(g.s[2]);
+                        sum += b[I] - (off7<D>(g, a.L[l], xv, I, nb_of<D>(g, x, y, z)) + diag7<D>(g, a.L[l], I) * xv[I]);
+                    }
+            bc[Ic] = sum;
+        });
         __syncthreads();
     }
-    long long ninner = 1;
-    for (int e = 0; e < g.D; ++e) ninner *= (g.n[e] - 2);
-    const T mean = T(red[0] / double(ninner));
-    __syncthreads();
-    for (int q = threadIdx.x; q < total; q += blockDim.x) {
-        int c[3];
-        coords(q, c);
-        if (is_interior(g, c)) b[q] -= mean;
-        xw[q] = T(0);
-    }
-    __syncthreads();
-    for (int it = 0; it < 2 * nuc; ++it) {
-        const int color = (it & 1) ^ ((it >> 1) & 1);   // R B, B R, R B, ...
-        for (int q = threadIdx.x; q < total; q += blockDim.x) {
-            int c[3];
-            coords(q, c);
-            if (!is_interior(g, c) || ((c[0] + c[1] + c[2]) & 1) != color) continue;
-            xw[q] = (b[q] - offdiag(g, L, xw, q, c)) * iD[q];
+    {
+        const Grid& g = a.g[last];
+        T* b = sm + a.off[last] + g.N;
+        // FP64 sum by one warp (ghost entries are zero): an FP64 instruction occupies the pipe for 16 cycles
+        // a warp, whatever its lanes do
+        if (tid < 32) {
+            double acc = 0.0;
+            for (int q = tid; q < int(g.N); q += 32) acc += double(b[q]);
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (tid == 0) mean_s = T(acc / double((g.n[0] - 2) * (g.n[1] - 2) * (D == 3 ? g.n[2] - 2 : 1)));
         }
         __syncthreads();
+        const T mean = mean_s;
+        cells(g, [&](int, int, int, int I) { b[I] -= mean; });
+        __syncthreads();
+        // R B, B R, R B, ...: a colour following itself changes nothing
+        sweeps(last, a.nuc + 1, 0, T(1), false);
     }
-    if (sm)
-        for (int q = threadIdx.x; q < total; q += blockDim.x) xv[q] = xs[q];
+    for (int l = last - 1; l >= 0; --l) sweeps(l, 2 * a.nu2[l], 1, a.omega, true);
+    for (int q = tid; q < N0; q += TAIL_THREADS) a.x[q] = sm[q];   // the ghost entries stay zero
 }
+
+// Pairs of cells in the largest level that the one-block kernel takes.  FP32: TAIL_PAIRS for each thread (16^3
+// cells).  FP64: 256, since a multiprocessor issues FP64 at 1/64 of the FP32 rate and a half-sweep on more cells is
+// faster spread over the device.
+template <class T> constexpr long long tail_pairs() { return sizeof(T) == 4 ? TAIL_PAIRS * TAIL_THREADS : 256; }
 
 template <class T>
 __global__ void zero_k(long long n, T* a) {
@@ -678,6 +806,12 @@ constexpr int KBLOCKS = 1216;   // 8 blocks on each of 152 SMs
             for (int x = 1 + threadIdx.x; x <= nxi_; x += blockDim.x) {                    \
                 const int I = row_ + x;
 
+// Blocks of the whole-array FP32 vector kernels: two float4 a thread on small grids (every further block only adds
+// a partial to the last block's sum), the row loops' grid on large ones.
+inline int vblocks(const Grid& g) {
+    const long long b = (g.N / 4 + 2 * KTHREADS - 1) / (2 * KTHREADS);
+    return int(std::max<long long>(1, std::min<long long>(b, KBLOCKS)));
+}
 inline int kblocks(const Grid& g) {
     const long long rows = (long long)(g.n[1] - 2) * (g.D == 3 ? g.n[2] - 2 : 1);
     return int(rows < KBLOCKS ? rows : KBLOCKS);
@@ -792,10 +926,25 @@ __global__ void setup_fine_k(Grid g, const double* __restrict__ L, double* __res
     iD32[I] = (df * df < 2.0f * eps) ? 0.0f : 1.0f / df;
 }
 
-constexpr int MV_ZT = 8;   // z planes per block of the tiled stencil kernels
-inline dim3 mv_tile_grid(const Grid& g) {
-    return dim3((g.n[0] - 2 + 31) / 32, (g.n[1] - 2 + 7) / 8, g.D == 3 ? (g.n[2] - 2 + MV_ZT - 1) / MV_ZT : 1);
+// z planes per block of the tiled stencil kernels: 8, and 1 where 8 would leave fewer than two blocks for a
+// multiprocessor (a thread's planes are then a chain of loads on an idle device)
+constexpr int MV_ZT = 8;
+inline int mv_planes(const Grid& g, int nsm) {
+    const long long tiles = ((g.n[0] - 2 + 31) / 32) * (long long)((g.n[1] - 2 + 7) / 8);
+    return g.D == 3 && tiles * ((g.n[2] - 2 + MV_ZT - 1) / MV_ZT) < 2ll * nsm ? 1 : MV_ZT;
 }
+inline dim3 mv_tile_grid(const Grid& g, int zt) {
+    return dim3((g.n[0] - 2 + 31) / 32, (g.n[1] - 2 + 7) / 8, g.D == 3 ? (g.n[2] - 2 + zt - 1) / zt : 1);
+}
+// launch K<D, planes per block> for the grid's dimension and the solver's tile depth
+#define LAUNCH_TILE(gg, K, ...)                                                                      \
+    do {                                                                                             \
+        const dim3 tg_ = mv_tile_grid(gg, mg->zt);                                                   \
+        if ((gg).D == 2) K<2, MV_ZT><<<tg_, KTHREADS, 0, st>>>(__VA_ARGS__);                         \
+        else if (mg->zt == 1) K<3, 1><<<tg_, KTHREADS, 0, st>>>(__VA_ARGS__);                        \
+        else K<3, MV_ZT><<<tg_, KTHREADS, 0, st>>>(__VA_ARGS__);                                     \
+        ia::note_launch();                                                                           \
+    } while (0)
 
 // z_I - D_I x_I - Σ L x_nb as one FMA chain: 2D + 1 FP64 operations where pairwise sums take 3D + 1
 // (the residual kernels are bound by the FP64 pipe)
@@ -842,7 +991,7 @@ __global__ void true_resid_k(Grid g, const double* __restrict__ L, const double*
 // With r32 given, also the next inner solve's start: r32 = float(r) (integer rounding, no FP64-pipe
 // conversion in this FP64-bound kernel) and e32 = 0 on the same interior cells (their ghost entries stay
 // zero from the allocation: the whole-array vector updates only ever add zero there).
-template <int D>
+template <int D, int ZT>
 __global__ void __launch_bounds__(256) true_resid_tile_k(Grid g, const double* __restrict__ L,
                                                          const double* __restrict__ diag,
                                                          const double* __restrict__ zz,
@@ -850,7 +999,7 @@ __global__ void __launch_bounds__(256) true_resid_tile_k(Grid g, const double* _
                                                          unsigned long long* __restrict__ pmax,
                                                          float* __restrict__ r32, float* __restrict__ e32) {
     const int x = 1 + int(blockIdx.x) * 32 + int(threadIdx.x & 31), y = 1 + int(blockIdx.y) * 8 + int(threadIdx.x >> 5);
-    const int z0 = D == 3 ? 1 + MV_ZT * int(blockIdx.z) : 0;
+    const int z0 = D == 3 ? 1 + ZT * int(blockIdx.z) : 0;
     unsigned long long m = 0ull;
     auto cell = [&](int z) {
         const int I = x + y * int(g.s[1]) + z * int(g.s[2]);
@@ -865,11 +1014,11 @@ __global__ void __launch_bounds__(256) true_resid_tile_k(Grid g, const double* _
         m = b > m ? b : m;
     };
     if (x <= g.n[0] - 2 && y <= g.n[1] - 2) {
-        if (D == 3 && z0 + MV_ZT - 1 <= g.n[2] - 2) {
+        if (D == 3 && z0 + ZT - 1 <= g.n[2] - 2) {
 #pragma unroll
-            for (int k = 0; k < MV_ZT; ++k) cell(z0 + k);   // a full tile (see matvec32_tile_k)
+            for (int k = 0; k < ZT; ++k) cell(z0 + k);   // a full tile (see matvec32_tile_k)
         } else {
-            for (int k = 0; k < (D == 3 ? MV_ZT : 1); ++k) {
+            for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
                 if (D == 3 && z0 + k > g.n[2] - 2) break;
                 cell(z0 + k);
             }
@@ -937,35 +1086,34 @@ __global__ void finalize_k(const double* __restrict__ partial, long long n, int 
         if (threadIdx.x == 0) out[qd] = v;
     }
 }
-// finalize_sum's value (its 1024 strided partial sums, then its pairwise tree, so the same roundings)
-// computed by a block of 256 threads, four strands each; valid in every thread.  sm: 1024 shared doubles.
+// Σ p[i] and Σ q[i] over n partials by one block of 256 threads in a fixed order, valid in thread 0: strands of
+// 256, a shuffle tree in each warp, then the eight warp sums by the first thread.  One barrier instead of the ten
+// of a tree over shared memory: with few partials the barriers were most of the reduction's tail.
 // Out of line: only the last block of a reduction calls it, and inlined it would raise the streaming
 // loop's register count.
-__device__ __noinline__ double sum1024_by256(const double* partial, long long n, int qd, double* sm) {
-    // the four strands advance together (each still in increasing index order), so that their loads
-    // are in flight at the same time
-    const double* p = partial + qd * n;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 2
-    for (long long i0 = threadIdx.x; i0 < n; i0 += 1024) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (i0 + 256 * k < n) acc[k] += __ldcg(p + i0 + 256 * k);
+__device__ __noinline__ void sum2_by256(const double* p, const double* q, long long n, double& sp, double& sq) {
+    __shared__ double wp[8], wq[8];
+    double a = 0.0, b = 0.0;
+#pragma unroll 4
+    for (long long i = threadIdx.x; i < n; i += 256) {
+        a += __ldcg(p + i);
+        if (q) b += __ldcg(q + i);
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) sm[int(threadIdx.x) + 256 * k] = acc[k];
+    a = warp_sum(a);
+    if (q) b = warp_sum(b);
+    if ((threadIdx.x & 31) == 0) {
+        wp[threadIdx.x >> 5] = a;
+        wq[threadIdx.x >> 5] = b;
+    }
     __syncthreads();
-    for (int w = 512; w > 0; w >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int v = int(threadIdx.x) + 256 * k;
-            if (v < w) sm[v] += sm[v + w];
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            a += wp[w];
+            if (q) b += wq[w];
         }
-        __syncthreads();
+        sp = a;
+        sq = b;
     }
-    const double r = sm[0];
-    __syncthreads();
-    return r;
 }
 // After thread 0 of every block has written the block's partials: true in the last block to finish,
 // which then sees every partial (each block's write is fenced before its count); the counter is reset
@@ -1032,12 +1180,12 @@ __global__ void update_k(Grid g, double alpha, const double* __restrict__ pv, co
 // are summed in a fixed order.  Four blocks per SM (64 registers) let a thread keep more of its planes'
 // loads in flight: 0.180 against 0.194 ms per launch at 256x512x256 with the default 32 registers.
 
-template <int D>
+template <int D, int ZT>
 __global__ void __launch_bounds__(256, 4) matvec32_tile_k(Grid g, const float* __restrict__ L,
                                                        const float* __restrict__ pv, float* __restrict__ q,
                                                        double* __restrict__ partial, FcgDev* S) {
     const int x = 1 + int(blockIdx.x) * 32 + int(threadIdx.x & 31), y = 1 + int(blockIdx.y) * 8 + int(threadIdx.x >> 5);
-    const int z0 = D == 3 ? 1 + MV_ZT * int(blockIdx.z) : 0;
+    const int z0 = D == 3 ? 1 + ZT * int(blockIdx.z) : 0;
     float acc = 0.f;
     auto cell = [&](int z) {
         const int I = x + y * int(g.s[1]) + z * int(g.s[2]);
@@ -1047,13 +1195,13 @@ __global__ void __launch_bounds__(256, 4) matvec32_tile_k(Grid g, const float* _
         acc += pv[I] * v;
     };
     if (x <= g.n[0] - 2 && y <= g.n[1] - 2) {
-        if (D == 3 && z0 + MV_ZT - 1 <= g.n[2] - 2) {
+        if (D == 3 && z0 + ZT - 1 <= g.n[2] - 2) {
             // a full tile: no bound test between the planes, so that their loads can be issued early
             // and a plane's values reused as the next plane's z neighbours
 #pragma unroll
-            for (int k = 0; k < MV_ZT; ++k) cell(z0 + k);
+            for (int k = 0; k < ZT; ++k) cell(z0 + k);
         } else {
-            for (int k = 0; k < (D == 3 ? MV_ZT : 1); ++k) {
+            for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
                 if (D == 3 && z0 + k > g.n[2] - 2) break;
                 cell(z0 + k);
             }
@@ -1073,8 +1221,8 @@ __global__ void __launch_bounds__(256, 4) matvec32_tile_k(Grid g, const float* _
     }
     // the last block: p·q in a fixed order, then α
     if (!last_block(&S->done_mv, nb)) return;
-    __shared__ double sm[1024];
-    const double pq = sum1024_by256(partial, nb, 0, sm);
+    double pq = 0.0, unused = 0.0;
+    sum2_by256(partial, nullptr, nb, pq, unused);
     if (threadIdx.x == 0) fcg_alpha(S, pq);
 }
 
@@ -1108,9 +1256,8 @@ __global__ void dot2_32_k(long long n, const float* __restrict__ sv, const float
     }
     // the last block: s·q and s·r in a fixed order, then β
     if (!last_block(&S->done_dot, gridDim.x)) return;
-    __shared__ double sm[1024];
-    const double sq = sum1024_by256(partial, gridDim.x, 0, sm);
-    const double sr = sum1024_by256(partial, gridDim.x, 1, sm);
+    double sq = 0.0, sr = 0.0;
+    sum2_by256(partial, partial + gridDim.x, gridDim.x, sq, sr);
     if (threadIdx.x == 0) fcg_beta(S, sq, sr, first);
 }
 
@@ -1218,13 +1365,13 @@ __device__ __forceinline__ double widen_exact(float v) {
 }
 
 // x += e over interior cells, on the tiles of matvec32_tile_k (one cell per thread and plane)
-template <int D>
+template <int D, int ZT>
 __global__ void __launch_bounds__(256) add_correction_k(Grid g, const float* __restrict__ e, double* __restrict__ xv) {
     const int x = 1 + int(blockIdx.x) * 32 + int(threadIdx.x & 31), y = 1 + int(blockIdx.y) * 8 + int(threadIdx.x >> 5);
-    const int z0 = D == 3 ? 1 + MV_ZT * int(blockIdx.z) : 0;
+    const int z0 = D == 3 ? 1 + ZT * int(blockIdx.z) : 0;
     if (x > g.n[0] - 2 || y > g.n[1] - 2) return;
 #pragma unroll
-    for (int k = 0; k < (D == 3 ? MV_ZT : 1); ++k) {
+    for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
         const int z = z0 + k;
         if (D == 3 && z > g.n[2] - 2) break;
         const int I = x + y * int(g.s[1]) + z * int(g.s[2]);
@@ -1264,14 +1411,12 @@ static int tb_zchunk(const Grid& g, int S, int nsm) {
     return std::max(zc, 1);
 }
 
-// the blocked smoother runs the FP32 V-cycle of a 3D level with an even number of interior
-// cells in every dimension (every level but the coarsest), for nu1, nu2 in {1, 2}
-static bool tb_usable(const PoissonMG* mg, const Grid& g) {
+// the blocked smoother runs the FP32 V-cycle of a 3D level whose next coarser level (gc) halves every
+// dimension, for nu1, nu2 in {1, 2}
+static bool tb_usable(const PoissonMG* mg, const Grid& g, const Grid& gc) {
     if (mg->smoother != IA_SMOOTHER_BLOCKED || g.D != 3 || mg->omega != 1.0) return false;
     if (mg->nu1 < 1 || mg->nu1 > 2 || mg->nu2 < 1 || mg->nu2 > 2) return false;
-    for (int e = 0; e < 3; ++e)
-        if ((g.n[e] - 2) % 2 != 0) return false;
-    return true;
+    return mg_regular(g, gc);
 }
 
 static void tb_launch(const PoissonMG* mg, const TbArgs& a, int S, cudaStream_t st) {
@@ -1290,6 +1435,47 @@ static void tb_launch(const PoissonMG* mg, const TbArgs& a, int S, cudaStream_t 
     ia::note_launch();
 }
 
+// shared values of the one-block V-cycle from level l on: x and b of each level
+static long long tail_values(const PoissonMG* mg, int l) {
+    long long n = 0;
+    for (; l < mg->nlev; ++l) n += 2 * mg->lev[l].g.N;
+    return n;
+}
+constexpr long long TAIL_BYTES = 160 * 1024;   // the rest of the 228 KB caches the coefficients in L1
+// first level of the one-block V-cycle; the coarsest level (at most 512 cells) always fits
+template <class T>
+static int tail_level(const PoissonMG* mg) {
+    int l = mg->nlev - 1;
+    while (l > 0 && mg->nlev - l < TAIL_MAX) {
+        const Grid& g = mg->lev[l - 1].g;
+        const long long pairs = (long long)((g.n[0] - 1) / 2) * (g.n[1] - 2) * (g.D == 3 ? g.n[2] - 2 : 1);
+        if (pairs > tail_pairs<T>() || tail_values(mg, l - 1) * (long long)sizeof(T) > TAIL_BYTES) break;
+        --l;
+    }
+    return l;
+}
+template <class T>
+static TailArgs<T> tail_args(PoissonMG* mg, int l0, int nu1, int nu2, int nuc) {
+    TailArgs<T> a;
+    a.nl = mg->nlev - l0;
+    a.total = 0;
+    for (int k = 0; k < a.nl; ++k) {
+        MGLevel& L = mg->lev[l0 + k];
+        a.g[k] = L.g;
+        a.L[k] = L.template L_<T>();
+        a.iD[k] = L.template iD_<T>();
+        a.off[k] = a.total;
+        a.total += 2 * int(L.g.N);
+        a.nu1[k] = (l0 + k == 0 && mg->nu1f > 0) ? mg->nu1f : nu1;
+        a.nu2[k] = (l0 + k == 0 && mg->nu2f > 0) ? mg->nu2f : nu2;
+    }
+    a.nuc = nuc;
+    a.omega = T(mg->omega);
+    a.b = mg->lev[l0].template b_<T>();
+    a.x = mg->lev[l0].template x_<T>();
+    return a;
+}
+
 template <class T>
 static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, int nu1, int nu2, int nuc) {
     auto& L = mg->lev[l];
@@ -1297,12 +1483,16 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     T* b = L.template b_<T>();
     const T* Lc = L.template L_<T>();
     const T* iD = L.template iD_<T>();
-    if (l == mg->nlev - 1) {
-        { coarse_k<T><<<1, 1024, 0, st>>>(L.g, Lc, iD, b, x, nuc); ia::note_launch(); }
+    if (l >= tail_level<T>(mg)) {
+        const TailArgs<T> a = tail_args<T>(mg, l, nu1, nu2, nuc);
+        const size_t bytes = sizeof(T) * (size_t)a.total;
+        if (L.g.D == 3) mg_tail_k<T, 3><<<1, TAIL_THREADS, bytes, st>>>(a);
+        else mg_tail_k<T, 2><<<1, TAIL_THREADS, bytes, st>>>(a);
+        ia::note_launch();
         return cudaGetLastError();
     }
     if constexpr (sizeof(T) == 4) {
-        if (tb_usable(mg, L.g)) {
+        if (tb_usable(mg, L.g, mg->lev[l + 1].g)) {
             // pre-smoothing from zero into the level's scratch vector, residual restriction
             // from it, then post-smoothing of scratch + prolongated correction into x
             auto& C = mg->lev[l + 1];
@@ -1342,22 +1532,30 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     if constexpr (sizeof(T) == 4) L16 = (l == 0 && mg->coef16) ? L.L16 : nullptr;
     auto& C = mg->lev[l + 1];
     const T om = T(mg->omega);
+    const bool reg = mg_regular(L.g, C.g);
     // each launch takes the interior rows [y0, y1)
     auto rows = [](dim3 gr, int y0, int y1) {
         gr.y = unsigned((y1 - y0 + 7) / 8);
         return gr;
     };
+    // cells of one colour that touch across a wrap are updated in passes, one per class of such cells
+    const int conf = wrap_conflicts(L.g);
     auto half = [&](int color, int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
         const dim3 gr = rows(pair_tile_grid(L.g), y0, y1);
-        if (L16) {
-            if (L.g.D == 3) rbgs_pair_k<T, 3, false, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, L16, b, x, color, om);
-            else rbgs_pair_k<T, 2, false, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, L16, b, x, color, om);
-        } else {
-            if (L.g.D == 3) rbgs_pair_k<T, 3><<<gr, blk(), 0, st>>>(L.g, y0, y1, Lc, b, x, color, om);
-            else rbgs_pair_k<T, 2><<<gr, blk(), 0, st>>>(L.g, y0, y1, Lc, b, x, color, om);
+        for (int cls = 0; cls <= conf; ++cls) {
+            if (cls & ~conf) continue;
+            auto go = [&](const auto* coef) {
+                using TL = std::decay_t<decltype(*coef)>;
+                if (L.g.D == 3) rbgs_pair_k<T, 3, false, TL><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, color, om, conf, cls);
+                else rbgs_pair_k<T, 2, false, TL><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, color, om, conf, cls);
+            };
+            if constexpr (sizeof(T) == 4) {
+                if (L16) go(L16);
+            }
+            if (!L16) go(Lc);
+            ia::note_launch();
         }
-        ia::note_launch();
         timing_end(h, tk);
     };
     // the relaxed first red half-sweep of a post-smoothing: the red cells still hold x without the
@@ -1366,10 +1564,16 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
         const dim3 gr = rows(pair_tile_grid(L.g), y0, y1);
         const T* xc = C.template x_<T>();
-        if (L16 && L.g.D == 3) rbgs_pair_k<T, 3, true, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, L16, b, x, 0, om, C.g, xc);
-        else if (L16) rbgs_pair_k<T, 2, true, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, L16, b, x, 0, om, C.g, xc);
-        else if (L.g.D == 3) rbgs_pair_k<T, 3, true><<<gr, blk(), 0, st>>>(L.g, y0, y1, Lc, b, x, 0, om, C.g, xc);
-        else rbgs_pair_k<T, 2, true><<<gr, blk(), 0, st>>>(L.g, y0, y1, Lc, b, x, 0, om, C.g, xc);
+        auto go = [&](auto REG, const auto* coef) {
+            using TL = std::decay_t<decltype(*coef)>;
+            constexpr bool R = decltype(REG)::value;
+            if (L.g.D == 3) rbgs_pair_k<T, 3, true, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, 0, om, 0, 0, C.g, xc);
+            else rbgs_pair_k<T, 2, true, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, 0, om, 0, 0, C.g, xc);
+        };
+        if constexpr (sizeof(T) == 4) {
+            if (L16) reg ? go(std::true_type{}, L16) : go(std::false_type{}, L16);
+        }
+        if (!L16) reg ? go(std::true_type{}, Lc) : go(std::false_type{}, Lc);
         ia::note_launch();
         timing_end(h, tk);
     };
@@ -1384,19 +1588,21 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
         const dim3 gr = rows(pair_grid(L.g), y0, y1);
         const T* xc = C.template x_<T>();
         const int wr = prol ? 0 : write_red;
-        if (L16 && L.g.D == 3) {
-            if (prol) rbgs_first_k<T, 3, true, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, L16, b, iD, xc, x, wr, om);
-            else rbgs_first_k<T, 3, false, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, L16, b, iD, xc, x, wr, om);
-        } else if (L16) {
-            if (prol) rbgs_first_k<T, 2, true, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, L16, b, iD, xc, x, wr, om);
-            else rbgs_first_k<T, 2, false, __half><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, L16, b, iD, xc, x, wr, om);
-        } else if (L.g.D == 3) {
-            if (prol) rbgs_first_k<T, 3, true><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, Lc, b, iD, xc, x, wr, om);
-            else rbgs_first_k<T, 3, false><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, Lc, b, iD, xc, x, wr, om);
-        } else {
-            if (prol) rbgs_first_k<T, 2, true><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, Lc, b, iD, xc, x, wr, om);
-            else rbgs_first_k<T, 2, false><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, Lc, b, iD, xc, x, wr, om);
+        auto go = [&](auto PROL, auto REG, const auto* coef) {
+            using TL = std::decay_t<decltype(*coef)>;
+            constexpr bool P = decltype(PROL)::value, R = decltype(REG)::value;
+            if (L.g.D == 3) rbgs_first_k<T, 3, P, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, coef, b, iD, xc, x, wr, om);
+            else rbgs_first_k<T, 2, P, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, C.g, coef, b, iD, xc, x, wr, om);
+        };
+        auto pick = [&](const auto* coef) {
+            if (!prol) go(std::false_type{}, std::true_type{}, coef);   // no coarse parent is read
+            else if (reg) go(std::true_type{}, std::true_type{}, coef);
+            else go(std::true_type{}, std::false_type{}, coef);
+        };
+        if constexpr (sizeof(T) == 4) {
+            if (L16) pick(L16);
         }
+        if (!L16) pick(Lc);
         ia::note_launch();
         timing_end(h, tk);
     };
@@ -1404,10 +1610,16 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto restrict_rows = [&](int yc0, int yc1) {
         const dim3 gr = rows(cell_grid(C.g), yc0, yc1);
         T* bc = C.template b_<T>();
-        if (L16 && L.g.D == 3) resid_restrict_k<T, 3, __half><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, L16, b, x, bc);
-        else if (L16) resid_restrict_k<T, 2, __half><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, L16, b, x, bc);
-        else if (L.g.D == 3) resid_restrict_k<T, 3><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, Lc, b, x, bc);
-        else resid_restrict_k<T, 2><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, Lc, b, x, bc);
+        auto go = [&](auto REG, const auto* coef) {
+            using TL = std::decay_t<decltype(*coef)>;
+            constexpr bool R = decltype(REG)::value;
+            if (L.g.D == 3) resid_restrict_k<T, 3, TL, R><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, coef, b, x, bc);
+            else resid_restrict_k<T, 2, TL, R><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, coef, b, x, bc);
+        };
+        if constexpr (sizeof(T) == 4) {
+            if (L16) reg ? go(std::true_type{}, L16) : go(std::false_type{}, L16);
+        }
+        if (!L16) reg ? go(std::true_type{}, Lc) : go(std::false_type{}, Lc);
         ia::note_launch();
     };
     // A smoothing is a chain of stages, each a half-sweep of one colour that reads the previous
@@ -1418,7 +1630,7 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     // updates read only the other colour).  The results are those of whole-level half-sweeps, bit for
     // bit, while a slab's rows are still in L2 for the next stage.  The restriction follows with the
     // coarse rows whose fine rows (and their neighbours) are final.
-    const bool slab = sizeof(T) == 4 && l == 0 && mg->slab_rows > 0 && L.g.D == 3 && !L.g.isper(1) &&
+    const bool slab = sizeof(T) == 4 && l == 0 && mg->slab_rows > 0 && L.g.D == 3 && !L.g.isper(1) && !conf &&
                       L.g.n[1] - 2 > mg->slab_rows;
     auto chain = [&](int S, auto&& stage, bool with_restrict) {
         const int ny = L.g.n[1] - 2, yend = L.g.n[1] - 1;
@@ -1448,8 +1660,11 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     }, true);
     cudaError_t e = vcycle<T>(h, mg, l + 1, st, nu1, nu2, nuc);
     if (e != cudaSuccess) return e;
-    if (nu2_here == 0) {
+    if (nu2_here == 0 || conf) {
         { prolong_k<T><<<grd(L.g), blk(), 0, st>>>(L.g, C.g, C.template x_<T>(), x); ia::note_launch(); }
+        // with wrap conflicts the fused prolongation would read cells that it writes: the half-sweeps
+        // (black, red) nu2 times follow the separate pass
+        for (int s = 0; s < 2 * nu2_here; ++s) half((s & 1) ? 0 : 1, 1, L.g.n[1] - 1);
         return cudaGetLastError();
     }
     // post-smoothing: first (black from x + P(x_coarse)), red (adding the correction when relaxed),
@@ -1515,6 +1730,13 @@ bool coef16_fits(double lrho) {
     return lo > 0.0 && 1.0 / lo <= 60000.0 && 1.0 / hi >= 1e-4;
 }
 
+// Cells of the next coarser level along a dimension of n: half of them rounded up, for a periodic dimension to
+// an even number (the red-black colouring has to close across the wrap), or to one.
+static long long mg_coarse_cells(long long n, bool periodic) {
+    const long long c = (n + 1) / 2;
+    return periodic && c > 1 ? c + (c & 1) : c;
+}
+
 // Rows per slab of the finest-level wavefront: the bytes a stage touches per interior row (x, b, the
 // inverse diagonal and the coefficients) times the rows of a slab within about 3/5 of L2, a multiple of
 // 8 rows (measured at 256x512x256: 64 rows 45.7 ms per step, 32 rows 47.0, 16 rows 49.9, whole-level
@@ -1528,10 +1750,15 @@ int mg_create(ia_handle* h) {
     const bool mixed = h->cfg.poisson_mode != IA_POISSON_FP64;
     mg->coef16 = (mixed && coef16_fits(h->cfg.lrho)) ? 1 : 0;
     int nl = 0;
+    int pr[3] = {0, 0, 0};
+    std::vector<double> width[3];   // cell widths of the current level in finest cells
+    for (int d = 0; d < g0.D; ++d) width[d].assign((size_t)Nint[d], 1.0);
+    std::vector<double> ratio;
     while (nl < MG_MAX_LEVELS) {
         int64_t N[3] = {Nint[0], Nint[1], Nint[2]};
         MGLevel& L = mg->lev[nl];
         L.g = make_grid(g0.D, g0.per, N);
+        for (int d = 0; d < 3; ++d) L.g.pr[d] = pr[d];
         const size_t n = (size_t)L.g.N;
         cudaError_t e = cudaSuccess;
         // FP64 levels always exist for level 0 (fine operator copies) and for the FP64 mode
@@ -1563,17 +1790,52 @@ int mg_create(ia_handle* h) {
                 cudaMemset(L.L32, 0, 4 * n * g0.D);
             }
         }
+        if (nl > 0) {
+            e = e ? e : cudaMalloc(&L.ratio, 8 * ratio.size());
+            if (!e) e = cudaMemcpy(L.ratio, ratio.data(), 8 * ratio.size(), cudaMemcpyHostToDevice);
+        }
         if (e != cudaSuccess) return IA_ERR_CUDA;
         ++nl;
-        bool can = true;
-        for (int d = 0; d < g0.D; ++d)
-            if (Nint[d] % 2 != 0 || Nint[d] < 4) can = false;
         long long cells = 1;
         for (int d = 0; d < g0.D; ++d) cells *= Nint[d];
-        if (!can || cells <= 512) break;
-        for (int d = 0; d < g0.D; ++d) Nint[d] /= 2;
+        // the coarsest level: few cells, and short enough that its sweeps reach across it
+        long long side = 0;
+        for (int d = 0; d < g0.D; ++d) side = std::max(side, Nint[d]);
+        if (cells <= 512 && side <= 8) break;
+        bool coarser = false;
+        ratio.clear();
+        for (int d = 0; d < g0.D; ++d) {
+            const long long n = Nint[d], nc = mg_coarse_cells(n, g0.isper(d));
+            pr[d] = int(n - nc);
+            coarser = coarser || nc < n;
+            // widths of the coarse cells and, for coarse face c = 1 .. nc + 1 (entry c, entry 0 unused), the
+            // distance of the cell centres beside it on this level over that on the coarse one
+            std::vector<double> wc;
+            for (long long c = 0, q = 0; c < nc; ++c, ++q) {
+                double w = width[d][(size_t)q];
+                if (c < pr[d]) w += width[d][(size_t)++q];
+                wc.push_back(w);
+            }
+            auto dist = [](const std::vector<double>& w, long long lo, long long hi) { return 0.5 * (w[(size_t)lo] + w[(size_t)hi]); };
+            ratio.push_back(0.5);
+            for (long long c = 0; c <= nc; ++c) {
+                const long long q = c < pr[d] ? 2 * c : c + pr[d];   // first child of coarse cell c (0-based)
+                // the outer faces: across the wrap, or a wall (whose coefficient is zero)
+                const bool edge = c == 0 || c == nc;
+                if (nc == 1) ratio.push_back(0.0);
+                else ratio.push_back(dist(width[d], edge ? n - 1 : q - 1, edge ? 0 : q) / dist(wc, edge ? nc - 1 : c - 1, edge ? 0 : c));
+            }
+            width[d] = wc;
+            Nint[d] = nc;
+        }
+        if (!coarser) break;
     }
     mg->nlev = nl;
+    if (cudaFuncSetAttribute(mg_tail_k<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess ||
+        cudaFuncSetAttribute(mg_tail_k<float, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess ||
+        cudaFuncSetAttribute(mg_tail_k<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess ||
+        cudaFuncSetAttribute(mg_tail_k<double, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess)
+        return IA_ERR_CUDA;
     const size_t N = (size_t)g0.N;
     cudaError_t e = cudaSuccess;
     e = e ? e : cudaMalloc(&mg->r, 8 * N);
@@ -1581,8 +1843,13 @@ int mg_create(ia_handle* h) {
     e = e ? e : cudaMalloc(&mg->p, 8 * N);
     e = e ? e : cudaMalloc(&mg->q, 8 * N);
     mg->kb = kblocks(g0);
+    mg->vb = vblocks(g0);
     {
-        const dim3 mv = mv_tile_grid(g0);
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&mg->nsm, cudaDevAttrMultiProcessorCount, dev);
+        mg->zt = mv_planes(g0, mg->nsm);
+        const dim3 mv = mv_tile_grid(g0, mg->zt);
         mg->mvb = (long long)mv.x * mv.y * mv.z;
     }
     e = e ? e : cudaMalloc(&mg->partial, 8 * std::max<size_t>(2 * (size_t)KBLOCKS, (size_t)mg->mvb));
@@ -1620,14 +1887,9 @@ int mg_create(ia_handle* h) {
     mg->nu1 = 2;
     mg->nu2 = 2;
     mg->nuc = 16;
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&mg->nsm, cudaDevAttrMultiProcessorCount, dev);
-        // whole-level half-sweeps by default: with two z planes per half-sweep thread the y-slab wavefront
-        // (ia_poisson_slab_rows) no longer shortens the step
-        mg->slab_rows = 0;
-    }
+    // whole-level half-sweeps by default: with two z planes per half-sweep thread the y-slab wavefront
+    // (ia_poisson_slab_rows) no longer shortens the step
+    mg->slab_rows = 0;
     return IA_OK;
 }
 
@@ -1638,6 +1900,7 @@ void mg_destroy(ia_handle* h) {
         MGLevel& L = mg->lev[l];
         cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.L); cudaFree(L.iD);
         cudaFree(L.x32); cudaFree(L.b32); cudaFree(L.r32); cudaFree(L.L32); cudaFree(L.iD32); cudaFree(L.L16);
+        cudaFree(L.ratio);
     }
     cudaFree(mg->r); cudaFree(mg->s); cudaFree(mg->p); cudaFree(mg->q);
     cudaFree(mg->p32); cudaFree(mg->q32); cudaFree(mg->e32);
@@ -1664,7 +1927,7 @@ static cudaError_t mg_setup(ia_handle* h, const double* L0) {
         { set_diag_k<double><<<grd(F.g), blk(), 0, st>>>(F.g, F.L, F.iD); ia::note_launch(); }
         for (int l = 1; l < mg->nlev; ++l) {
             { restrict_L_k<double><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l - 1].g,
-                                                                       mg->lev[l - 1].L, mg->lev[l].L); ia::note_launch(); }
+                                                                       mg->lev[l - 1].L, mg->lev[l].ratio, mg->lev[l].L); ia::note_launch(); }
             { set_diag_k<double><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l].L, mg->lev[l].iD); ia::note_launch(); }
         }
     } else {
@@ -1674,7 +1937,7 @@ static cudaError_t mg_setup(ia_handle* h, const double* L0) {
         LAUNCH_D(F.g, setup_fine_k, gg, blk(), F.g, L0, mg->diag64, F.L32, l16, F.iD32);
         for (int l = 1; l < mg->nlev; ++l) {
             { restrict_L_k<float><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l - 1].g,
-                                                                      mg->lev[l - 1].L32, mg->lev[l].L32); ia::note_launch(); }
+                                                                      mg->lev[l - 1].L32, mg->lev[l].ratio, mg->lev[l].L32); ia::note_launch(); }
             { set_diag_k<float><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l].L32, mg->lev[l].iD32); ia::note_launch(); }
         }
     }
@@ -1713,7 +1976,7 @@ static cudaError_t mg_precondition(ia_handle* h) {
 static void true_residual(PoissonMG* mg, const Grid& g, const double* L, const double* zz, const double* xv,
                           unsigned long long* dlinf, cudaStream_t st, float* r32 = nullptr, float* e32 = nullptr) {
     unsigned long long* pmax = reinterpret_cast<unsigned long long*>(mg->partial);
-    LAUNCH_D(g, true_resid_tile_k, mv_tile_grid(g), KTHREADS, g, L, mg->diag64, zz, xv, mg->r, pmax, r32, e32);
+    LAUNCH_TILE(g, true_resid_tile_k, g, L, mg->diag64, zz, xv, mg->r, pmax, r32, e32);
     { finalize_max_k<<<1, 1024, 0, st>>>(pmax, mg->mvb, dlinf); ia::note_launch(); }
 }
 
@@ -1807,10 +2070,10 @@ static int poisson_solve_mixed(ia_handle* h, double* xv, const double* zz, const
             // β, the direction, q = A p, α and the update without a host round trip; one read-back of
             // the inner residual and the breakdown flag per step
             tk = timing_begin(h, TK_KRYLOV);
-            { dot2_32_k<<<mg->kb, KTHREADS, 0, st>>>(N, sv, mg->q32, rr, mg->partial, S, it == 0 ? 1 : 0); ia::note_launch(); }
-            { xpby32_k<<<mg->kb, KTHREADS, 0, st>>>(N, sv, S, mg->p32); ia::note_launch(); }
-            LAUNCH_D(g, matvec32_tile_k, mv_tile_grid(g), KTHREADS, g, F.L32, mg->p32, mg->q32, mg->partial, S);
-            { update32_k<<<mg->kb, KTHREADS, 0, st>>>(N, S, mg->p32, mg->q32, mg->e32, rr); ia::note_launch(); }
+            { dot2_32_k<<<mg->vb, KTHREADS, 0, st>>>(N, sv, mg->q32, rr, mg->partial, S, it == 0 ? 1 : 0); ia::note_launch(); }
+            { xpby32_k<<<mg->vb, KTHREADS, 0, st>>>(N, sv, S, mg->p32); ia::note_launch(); }
+            LAUNCH_TILE(g, matvec32_tile_k, g, F.L32, mg->p32, mg->q32, mg->partial, S);
+            { update32_k<<<mg->vb, KTHREADS, 0, st>>>(N, S, mg->p32, mg->q32, mg->e32, rr); ia::note_launch(); }
             timing_end(h, tk);
             cudaMemcpyAsync(mg->hsc + 2, &S->rin, 8, cudaMemcpyDeviceToHost, st);
             if (cudaStreamSynchronize(st) != cudaSuccess) return IA_ERR_CUDA;
@@ -1826,7 +2089,7 @@ static int poisson_solve_mixed(ia_handle* h, double* xv, const double* zz, const
             if (double(rinf) <= target) break;
         }
         tk = timing_begin(h, TK_KRYLOV);
-        LAUNCH_D(g, add_correction_k, mv_tile_grid(g), KTHREADS, g, mg->e32, xv);
+        LAUNCH_TILE(g, add_correction_k, g, mg->e32, xv);
         true_residual(mg, g, L, zz, xv, dlinf, st, rr, mg->e32);
         timing_end(h, tk);
         const double res_old = res;

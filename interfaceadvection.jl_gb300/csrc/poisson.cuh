@@ -9,7 +9,7 @@ struct ia_handle;
 
 namespace ia {
 
-constexpr int MG_MAX_LEVELS = 12;
+constexpr int MG_MAX_LEVELS = 32;   // a dimension has less than 2^31 cells
 
 // Step scalars of the mixed solver's inner FCG, kept on the device so that only the convergence test
 // is read back each iteration: β and α in FP64 (and as the FP32 values the vector kernels use), the
@@ -30,6 +30,8 @@ struct MGLevel {
     float *x32 = nullptr, *b32 = nullptr, *r32 = nullptr, *L32 = nullptr, *iD32 = nullptr;
     // finest level of the mixed V-cycle: FP16 copy of L32 for the smoother and the residual restriction
     __half* L16 = nullptr;
+    // coarse levels: per dimension and face, cell distance on the finer level over this level's (restrict_L_k)
+    double* ratio = nullptr;
     template <class T> T* x_();
     template <class T> T* b_();
     template <class T> T* r_();
@@ -62,6 +64,8 @@ struct PoissonMG {
     double* partial = nullptr;                                        // per-block dot partials
     long long mvb = 0;                                                // blocks (partials) of the tiled FP32 matvec
     int kb = 0;                                                       // blocks of the Krylov row loops
+    int vb = 0;                                                       // blocks of the FP32 vector kernels
+    int zt = 8;                                                       // z planes per block of the tiled stencils
     double* diag64 = nullptr;                                         // FP64 operator diagonal
     double* dsc = nullptr;                                            // device scalars
     ia::FcgDev* fcg = nullptr;                                        // the inner FCG's step scalars
