@@ -1,8 +1,7 @@
 // Learned Poisson preconditioner (see nn.cuh for the network).
 //
-//  * Training kernels (FP32, CUDA cores): direct 3x3x3 convolution forward,
-//    backward-data (flipped, transposed taps), backward-weight (per-tap block
-//    reductions), pooling / upsampling / ReLU / skip adjoints, MSE loss, Adam.
+//  * Training kernels (FP32, CUDA cores; the convolutions and their gradients in
+//    nn_train.cuh): MSE and energy losses, Adam.
 //  * Inference kernel (BF16 weights and activations, FP32 accumulation on the
 //    5th-generation tensor cores): implicit GEMM with M = 128 output cells,
 //    N = Cout, K = 27 taps x Cin.  Per tap the 128 x Cin im2col tile is staged in
@@ -16,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -58,180 +58,14 @@ __device__ __forceinline__ long long child_pos(const Dims& f, int b, int X, int 
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (D).cells();                \
          q += (long long)gridDim.x * blockDim.x)
 
-// ------------------------------------------------------------------ FP32 training kernels
-template <int CI, int CO>
-__global__ void conv_fwd_f32(Dims d, const float* __restrict__ X, const float* __restrict__ W,
-                             const float* __restrict__ bias, float* __restrict__ Z, float* __restrict__ A,
-                             const float* __restrict__ skip, int relu) {
-    FOR_CELLS(d) {
-        int b, x, y, z;
-        d.decode(q, b, x, y, z);
-        const long long p = d.pos(b, x, y, z);
-        float acc[CO];
-#pragma unroll
-        for (int o = 0; o < CO; ++o) acc[o] = __ldg(bias + o);
-        for (int t = 0; t < 27; ++t) {
-            const float* xp = X + (p + d.tap(t)) * CI;
-            const float* wt = W + (long long)t * CO * CI;
-#pragma unroll 4
-            for (int c = 0; c < CI; ++c) {
-                const float xv = xp[c];
-#pragma unroll
-                for (int o = 0; o < CO; ++o) acc[o] = fmaf(__ldg(wt + o * CI + c), xv, acc[o]);
-            }
-        }
-#pragma unroll
-        for (int o = 0; o < CO; ++o) {
-            if (Z) Z[p * CO + o] = acc[o];
-            float v = relu ? fmaxf(acc[o], 0.f) : acc[o];
-            if (skip) v += skip[p * CO + o];
-            A[p * CO + o] = v;
-        }
-    }
-}
+}  // namespace nn
+}  // namespace ia
+#include "nn_train.cuh"
 
-// dX[p] = Σ_t W[t]^T dY[p - off(t)]
-template <int CI, int CO>
-__global__ void conv_bwd_data_f32(Dims d, const float* __restrict__ dY, const float* __restrict__ W,
-                                  float* __restrict__ dX) {
-    FOR_CELLS(d) {
-        int b, x, y, z;
-        d.decode(q, b, x, y, z);
-        const long long p = d.pos(b, x, y, z);
-        float acc[CI];
-#pragma unroll
-        for (int c = 0; c < CI; ++c) acc[c] = 0.f;
-        for (int t = 0; t < 27; ++t) {
-            const float* yp = dY + (p - d.tap(t)) * CO;
-            const float* wt = W + (long long)t * CO * CI;
-#pragma unroll 4
-            for (int o = 0; o < CO; ++o) {
-                const float g = yp[o];
-#pragma unroll
-                for (int c = 0; c < CI; ++c) acc[c] = fmaf(__ldg(wt + o * CI + c), g, acc[c]);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < CI; ++c) dX[p * CI + c] = acc[c];
-    }
-}
+namespace ia {
+namespace nn {
 
-// dW[t][o][c] += Σ_p X[p+off(t)][c] dY[p][o] over a chunk of cells (one tap per blockIdx.y);
-// the tap-0 blocks also accumulate the bias gradient db[o] += Σ_p dY[p][o].
-template <int CI, int CO>
-__global__ void conv_bwd_w_f32(Dims d, const float* __restrict__ X, const float* __restrict__ dY,
-                               float* __restrict__ dW, float* __restrict__ db, long long chunk) {
-    constexpr int TILE = 32;
-    constexpr int PAIRS = CI * CO;
-    constexpr int PER = (PAIRS + 255) / 256;
-    __shared__ float xs[TILE][CI];
-    __shared__ float ys[TILE][CO];
-    const int t = blockIdx.y;
-    const long long toff = d.tap(t);
-    const long long c0 = (long long)blockIdx.x * chunk;
-    const long long c1 = min(d.cells(), c0 + chunk);
-    float acc[PER];
-#pragma unroll
-    for (int k = 0; k < PER; ++k) acc[k] = 0.f;
-    float bacc = 0.f;
-    for (long long base = c0; base < c1; base += TILE) {
-        for (int e = threadIdx.x; e < TILE * (CI + CO); e += blockDim.x) {
-            const int r = e / (CI + CO), c = e % (CI + CO);
-            const long long qq = base + r;
-            float v = 0.f;
-            if (qq < c1) {
-                int b, x, y, z;
-                d.decode(qq, b, x, y, z);
-                const long long p = d.pos(b, x, y, z);
-                v = (c < CI) ? X[(p + toff) * CI + c] : dY[p * CO + (c - CI)];
-            }
-            if (c < CI) xs[r][c] = v;
-            else ys[r][c - CI] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            const int pr = threadIdx.x + 256 * k;
-            if (pr < PAIRS) {
-                const int o = pr / CI, c = pr % CI;
-                float sacc = acc[k];
-                for (int r = 0; r < TILE; ++r) sacc = fmaf(xs[r][c], ys[r][o], sacc);
-                acc[k] = sacc;
-            }
-        }
-        if (t == 0 && threadIdx.x < CO)
-            for (int r = 0; r < TILE; ++r) bacc += ys[r][threadIdx.x];
-        __syncthreads();
-    }
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        const int pr = threadIdx.x + 256 * k;
-        if (pr < PAIRS) atomicAdd(dW + (long long)t * PAIRS + pr, acc[k]);
-    }
-    if (t == 0 && threadIdx.x < CO) atomicAdd(db + threadIdx.x, bacc);
-}
-
-// dZ = dA · [Z > 0]
-__global__ void relu_bwd_f32(Dims d, int C, const float* __restrict__ Z, const float* __restrict__ dA,
-                             float* __restrict__ dZ) {
-    FOR_CELLS(d) {
-        int b, x, y, z;
-        d.decode(q, b, x, y, z);
-        const long long p = d.pos(b, x, y, z) * C;
-        for (int c = 0; c < C; ++c) dZ[p + c] = Z[p + c] > 0.f ? dA[p + c] : 0.f;
-    }
-}
-
-// out (coarse dims dc) = mean of the 8 children of in (fine dims 2dc)
-__global__ void pool_fwd_f32(Dims dc, int C, const float* __restrict__ in, float* __restrict__ out) {
-    const Dims df{dc.B, 2 * dc.nx, 2 * dc.ny, 2 * dc.nz};
-    FOR_CELLS(dc) {
-        int b, x, y, z;
-        dc.decode(q, b, x, y, z);
-        const long long P = dc.pos(b, x, y, z) * C;
-        for (int c = 0; c < C; ++c) {
-            float s = 0.f;
-            for (int k = 0; k < 8; ++k) s += in[child_pos(df, b, x, y, z, k) * C + c];
-            out[P + c] = s * 0.125f;
-        }
-    }
-}
-// dIn[child] += dOut[parent] / 8   (fine dims df)
-__global__ void pool_bwd_add_f32(Dims df, int C, const float* __restrict__ dout, float* __restrict__ din) {
-    const Dims dc = df.half();
-    FOR_CELLS(df) {
-        int b, x, y, z;
-        df.decode(q, b, x, y, z);
-        const long long p = df.pos(b, x, y, z) * C, P = dc.pos(b, x / 2, y / 2, z / 2) * C;
-        for (int c = 0; c < C; ++c) din[p + c] += 0.125f * dout[P + c];
-    }
-}
-// out[child] = in[parent] (+ skip[child])  (fine dims df)
-__global__ void up_fwd_f32(Dims df, int C, const float* __restrict__ in, const float* __restrict__ skip,
-                           float* __restrict__ out) {
-    const Dims dc = df.half();
-    FOR_CELLS(df) {
-        int b, x, y, z;
-        df.decode(q, b, x, y, z);
-        const long long p = df.pos(b, x, y, z) * C, P = dc.pos(b, x / 2, y / 2, z / 2) * C;
-        for (int c = 0; c < C; ++c) out[p + c] = in[P + c] + (skip ? skip[p + c] : 0.f);
-    }
-}
-// dIn[parent] = Σ children dOut  (coarse dims dc)
-__global__ void up_bwd_f32(Dims dc, int C, const float* __restrict__ dout, float* __restrict__ din) {
-    const Dims df{dc.B, 2 * dc.nx, 2 * dc.ny, 2 * dc.nz};
-    FOR_CELLS(dc) {
-        int b, x, y, z;
-        dc.decode(q, b, x, y, z);
-        const long long P = dc.pos(b, x, y, z) * C;
-        for (int c = 0; c < C; ++c) {
-            float s = 0.f;
-            for (int k = 0; k < 8; ++k) s += dout[child_pos(df, b, x, y, z, k) * C + c];
-            din[P + c] = s;
-        }
-    }
-}
-
+// ------------------------------------------------------------------ FP32 training kernels: loss and optimiser
 // dOut = 2 (out - tgt) / n ; loss partials
 __global__ void mse_k(Dims d, const float* __restrict__ out, const float* __restrict__ tgt, float* __restrict__ dout,
                       double* __restrict__ loss) {
@@ -299,11 +133,6 @@ __global__ void adam_k(long long n, float* __restrict__ w, const float* __restri
         v[i] = vi;
         w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     }
-}
-
-__global__ void zero_f32(long long n, float* a) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        a[i] = 0.f;
 }
 
 // ------------------------------------------------------------------ tcgen05 inference convolution
@@ -680,6 +509,8 @@ struct NNState {
     float* buf = nullptr;
     size_t buf_bytes = 0;
     nn::Dims buf_dims{0, 0, 0, 0};
+    float* part = nullptr;                                           // the blocks' weight gradients, one layer's at a time
+    int sms = 152;                                                   // multiprocessors of the device
     // inference activations (BF16), same rule
     __nv_bfloat16* ibuf = nullptr;
     size_t ibuf_bytes = 0;
@@ -716,6 +547,7 @@ NNState* nn_state(ia_handle* h) {
         e = cudaMalloc(&s->wtc[l], (size_t)27 * co * ci * 2);
     }
     if (e != cudaSuccess) return nullptr;
+    cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, h->device);
     cudaMemset(s->w, 0, 4 * n);
     cudaMemset(s->m, 0, 4 * n);
     cudaMemset(s->v, 0, 4 * n);
@@ -734,14 +566,14 @@ float* take(float*& cur, long long n) {
 struct Graph {
     nn::Dims f, hf, qt;
     float *x0, *z1, *a1, *p1, *z2, *a2, *p2, *z3, *a3, *u2, *z4, *a4, *u1, *z5, *a5, *out, *tgt;
-    float *dout, *da5, *dz5, *du1, *da4, *dz4, *du2, *da3, *dz3, *dp2, *da2, *dz2, *dp1, *da1, *dz1;
+    float *dout, *da5, *dz5, *du1, *dz4, *du2, *dz3, *dp2, *dz2, *dp1, *dz1;
 };
 
 size_t graph_floats(const nn::Dims& f) {
     const nn::Dims hf = f.half(), qt = hf.half();
     const long long F = f.padded(), H = hf.padded(), Q = qt.padded();
     const long long per = F * (4 + 16 * 3 + 32 + 16 * 2 + 1 + 1) + H * (16 + 32 * 5) + Q * (32 * 3) +
-                          F * (1 + 16 * 2 + 32 + 16 * 2) + H * (16 + 32 * 5) + Q * (32 * 3);
+                          F * (1 + 16 * 2 + 32 + 16) + H * (16 + 32 * 3) + Q * (32 * 2);
     return (size_t)per + 64 * 40;
 }
 
@@ -773,16 +605,12 @@ Graph carve(float* base, const nn::Dims& f) {
     G.da5 = take(c, F * 16);
     G.dz5 = take(c, F * 16);
     G.du1 = take(c, F * 32);
-    G.da4 = take(c, H * 32);
     G.dz4 = take(c, H * 32);
     G.du2 = take(c, H * 32);
-    G.da3 = take(c, Q * 32);
     G.dz3 = take(c, Q * 32);
     G.dp2 = take(c, Q * 32);
-    G.da2 = take(c, H * 32);
     G.dz2 = take(c, H * 32);
     G.dp1 = take(c, H * 16);
-    G.da1 = take(c, F * 16);
     G.dz1 = take(c, F * 16);
     return G;
 }
@@ -810,58 +638,85 @@ inline int nblk(long long n) {
     return int(b < 4096 ? (b < 1 ? 1 : b) : 4096);
 }
 
-template <int CI, int CO>
-void fwd(const nn::Dims& d, const float* X, const float* W, const float* b, float* Z, float* A, const float* skip,
-         int relu, cudaStream_t st) {
-    { nn::conv_fwd_f32<CI, CO><<<nblk(d.cells()), 256, 0, st>>>(d, X, W, b, Z, A, skip, relu); ia::note_launch(); }
+// a convolution (flip: a data gradient) on the tile that fills the device: 32 x 8 x 4 cells, 2 planes where 4 leave
+// fewer than two blocks for a multiprocessor, 16 cells along x on short rows
+template <int CI, int CO, int TX, int TZ>
+cudaError_t conv32_tile(const nn::Dims& d, const float* X, const float* W, int flip, const float* b, float* Z, float* A,
+                        const float* skip, int relu, cudaStream_t st) {
+    using C = nn::Conv32<CI, CO, TX, TZ>;
+    const long long blocks = (long long)((d.nx + TX - 1) / TX) * ((d.ny + nn::CONV_TY - 1) / nn::CONV_TY) * ((d.nz + TZ - 1) / TZ) * d.B;
+    const cudaError_t e = cudaFuncSetAttribute(nn::conv32_k<CI, CO, TX, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES);
+    if (e != cudaSuccess) return e;
+    { nn::conv32_k<CI, CO, TX, TZ><<<unsigned(blocks), C::THREADS, C::BYTES, st>>>(d, X, W, flip, b, Z, A, skip, relu); ia::note_launch(); }
+    return cudaGetLastError();
 }
 template <int CI, int CO>
-void bwd(const nn::Dims& d, const float* X, const float* dY, const float* W, float* dW, float* db, float* dX,
-         cudaStream_t st) {
-    // about 96 chunks per tap (27 x 96 blocks), at least 1024 cells each
-    long long chunk = (d.cells() + 95) / 96;
-    chunk = chunk < 1024 ? 1024 : (chunk + 31) / 32 * 32;
-    const dim3 grid((unsigned)((d.cells() + chunk - 1) / chunk), 27);
-    { nn::conv_bwd_w_f32<CI, CO><<<grid, 256, 0, st>>>(d, X, dY, dW, db, chunk); ia::note_launch(); }
-    if (dX) { nn::conv_bwd_data_f32<CI, CO><<<nblk(d.cells()), 256, 0, st>>>(d, dY, W, dX); ia::note_launch(); }
+cudaError_t conv32(const NNState* s, const nn::Dims& d, const float* X, const float* W, int flip, const float* b, float* Z,
+                   float* A, const float* skip, int relu, cudaStream_t st) {
+    if (d.nx <= 16) return conv32_tile<CI, CO, 16, 2>(d, X, W, flip, b, Z, A, skip, relu, st);
+    const long long blocks = (long long)((d.nx + 31) / 32) * ((d.ny + nn::CONV_TY - 1) / nn::CONV_TY) * ((d.nz + 3) / 4) * d.B;
+    if (blocks < 2 * s->sms) return conv32_tile<CI, CO, 32, 2>(d, X, W, flip, b, Z, A, skip, relu, st);
+    return conv32_tile<CI, CO, 32, 4>(d, X, W, flip, b, Z, A, skip, relu, st);
 }
+// gradients of the weights and the bias of a layer into g (W[27][CO][CI], then b[CO])
+template <int CI, int CO>
+cudaError_t wgrad(const NNState* s, const nn::Dims& d, const float* X, const float* dY, float* g, cudaStream_t st) {
+    using G = nn::Wgrad<CI, CO>;
+    const long long tiles = (long long)((d.nx + nn::WG_X - 1) / nn::WG_X) * ((d.ny + nn::WG_Y - 1) / nn::WG_Y) *
+                            ((d.nz + nn::WG_Z - 1) / nn::WG_Z) * d.B;
+    const int blocks = int(std::min<long long>(tiles, nn::WG_BLOCKS * s->sms));
+    const cudaError_t e = cudaFuncSetAttribute(nn::wgrad_k<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * G::SM);
+    if (e != cudaSuccess) return e;
+    { nn::wgrad_k<CI, CO><<<blocks, G::THREADS, 4 * G::SM, st>>>(d, X, dY, s->part, int(tiles)); ia::note_launch(); }
+    { nn::wgrad_sum_k<<<(G::N + 31) / 32, 256, 0, st>>>(s->part, blocks, G::N, g); ia::note_launch(); }
+    return cudaGetLastError();
+}
+
+inline const float4* v4(const float* p) { return reinterpret_cast<const float4*>(p); }
+inline float4* v4(float* p) { return reinterpret_cast<float4*>(p); }
 
 // forward of the training graph (inputs already in G.x0)
-void forward_f32(const Graph& G, const float* w, cudaStream_t st) {
+cudaError_t forward_f32(const NNState* s, const Graph& G, cudaStream_t st) {
     using namespace nn;
-    fwd<4, 16>(G.f, G.x0, w + layer_w(0), w + layer_b(0), G.z1, G.a1, nullptr, 1, st);
-    { pool_fwd_f32<<<nblk(G.hf.cells()), 256, 0, st>>>(G.hf, 16, G.a1, G.p1); ia::note_launch(); }
-    fwd<16, 32>(G.hf, G.p1, w + layer_w(1), w + layer_b(1), G.z2, G.a2, nullptr, 1, st);
-    { pool_fwd_f32<<<nblk(G.qt.cells()), 256, 0, st>>>(G.qt, 32, G.a2, G.p2); ia::note_launch(); }
-    fwd<32, 32>(G.qt, G.p2, w + layer_w(2), w + layer_b(2), G.z3, G.a3, nullptr, 1, st);
-    { up_fwd_f32<<<nblk(G.hf.cells()), 256, 0, st>>>(G.hf, 32, G.a3, G.a2, G.u2); ia::note_launch(); }
-    fwd<32, 32>(G.hf, G.u2, w + layer_w(3), w + layer_b(3), G.z4, G.a4, nullptr, 1, st);
-    { up_fwd_f32<<<nblk(G.f.cells()), 256, 0, st>>>(G.f, 32, G.a4, nullptr, G.u1); ia::note_launch(); }
-    fwd<32, 16>(G.f, G.u1, w + layer_w(4), w + layer_b(4), G.z5, G.a5, G.a1, 1, st);
-    fwd<16, 1>(G.f, G.a5, w + layer_w(5), w + layer_b(5), nullptr, G.out, nullptr, 0, st);
+    const float* w = s->w;
+    cudaError_t e = conv32<4, 16>(s, G.f, G.x0, w + layer_w(0), 0, w + layer_b(0), G.z1, G.a1, nullptr, 1, st);
+    { pool_fwd_k<<<nblk(G.hf.cells() * 4), 256, 0, st>>>(G.hf, 4, v4(G.a1), v4(G.p1)); ia::note_launch(); }
+    e = e ? e : conv32<16, 32>(s, G.hf, G.p1, w + layer_w(1), 0, w + layer_b(1), G.z2, G.a2, nullptr, 1, st);
+    { pool_fwd_k<<<nblk(G.qt.cells() * 8), 256, 0, st>>>(G.qt, 8, v4(G.a2), v4(G.p2)); ia::note_launch(); }
+    e = e ? e : conv32<32, 32>(s, G.qt, G.p2, w + layer_w(2), 0, w + layer_b(2), G.z3, G.a3, nullptr, 1, st);
+    { up_fwd_k<<<nblk(G.hf.cells() * 8), 256, 0, st>>>(G.hf, 8, v4(G.a3), v4(G.a2), v4(G.u2)); ia::note_launch(); }
+    e = e ? e : conv32<32, 32>(s, G.hf, G.u2, w + layer_w(3), 0, w + layer_b(3), G.z4, G.a4, nullptr, 1, st);
+    { up_fwd_k<<<nblk(G.f.cells() * 8), 256, 0, st>>>(G.f, 8, v4(G.a4), nullptr, v4(G.u1)); ia::note_launch(); }
+    e = e ? e : conv32<32, 16>(s, G.f, G.u1, w + layer_w(4), 0, w + layer_b(4), G.z5, G.a5, G.a1, 1, st);
+    e = e ? e : conv32<16, 1>(s, G.f, G.a5, w + layer_w(5), 0, w + layer_b(5), nullptr, G.out, nullptr, 0, st);
+    return e ? e : cudaGetLastError();
 }
 
-void backward_f32(const Graph& G, const float* w, float* g, cudaStream_t st) {
+cudaError_t backward_f32(const NNState* s, const Graph& G, cudaStream_t st) {
     using namespace nn;
-    bwd<16, 1>(G.f, G.a5, G.dout, w + layer_w(5), g + layer_w(5), g + layer_b(5), G.da5, st);
-    { relu_bwd_f32<<<nblk(G.f.cells()), 256, 0, st>>>(G.f, 16, G.z5, G.da5, G.dz5); ia::note_launch(); }
-    bwd<32, 16>(G.f, G.u1, G.dz5, w + layer_w(4), g + layer_w(4), g + layer_b(4), G.du1, st);
-    { up_bwd_f32<<<nblk(G.hf.cells()), 256, 0, st>>>(G.hf, 32, G.du1, G.da4); ia::note_launch(); }
-    { relu_bwd_f32<<<nblk(G.hf.cells()), 256, 0, st>>>(G.hf, 32, G.z4, G.da4, G.dz4); ia::note_launch(); }
-    bwd<32, 32>(G.hf, G.u2, G.dz4, w + layer_w(3), g + layer_w(3), g + layer_b(3), G.du2, st);
-    { up_bwd_f32<<<nblk(G.qt.cells()), 256, 0, st>>>(G.qt, 32, G.du2, G.da3); ia::note_launch(); }
-    { relu_bwd_f32<<<nblk(G.qt.cells()), 256, 0, st>>>(G.qt, 32, G.z3, G.da3, G.dz3); ia::note_launch(); }
-    bwd<32, 32>(G.qt, G.p2, G.dz3, w + layer_w(2), g + layer_w(2), g + layer_b(2), G.dp2, st);
-    // da2 = du2 (skip) + pool adjoint of dp2
-    cudaMemcpyAsync(G.da2, G.du2, sizeof(float) * G.hf.padded() * 32, cudaMemcpyDeviceToDevice, st);
-    { pool_bwd_add_f32<<<nblk(G.hf.cells()), 256, 0, st>>>(G.hf, 32, G.dp2, G.da2); ia::note_launch(); }
-    { relu_bwd_f32<<<nblk(G.hf.cells()), 256, 0, st>>>(G.hf, 32, G.z2, G.da2, G.dz2); ia::note_launch(); }
-    bwd<16, 32>(G.hf, G.p1, G.dz2, w + layer_w(1), g + layer_w(1), g + layer_b(1), G.dp1, st);
-    // da1 = da5 (skip) + pool adjoint of dp1
-    cudaMemcpyAsync(G.da1, G.da5, sizeof(float) * G.f.padded() * 16, cudaMemcpyDeviceToDevice, st);
-    { pool_bwd_add_f32<<<nblk(G.f.cells()), 256, 0, st>>>(G.f, 16, G.dp1, G.da1); ia::note_launch(); }
-    { relu_bwd_f32<<<nblk(G.f.cells()), 256, 0, st>>>(G.f, 16, G.z1, G.da1, G.dz1); ia::note_launch(); }
-    bwd<4, 16>(G.f, G.x0, G.dz1, w + layer_w(0), g + layer_w(0), g + layer_b(0), nullptr, st);
+    const float* w = s->w;
+    float* g = s->g;
+    // data gradient of layer l
+    auto W = [&](int l) { return w + layer_w(l); };
+    cudaError_t e = wgrad<16, 1>(s, G.f, G.a5, G.dout, g + layer_w(5), st);
+    e = e ? e : conv32<1, 16>(s, G.f, G.dout, W(5), 1, nullptr, nullptr, G.da5, nullptr, 0, st);
+    { relu_bwd_k<<<nblk(G.f.cells() * 4), 256, 0, st>>>(G.f, 4, v4(G.z5), v4(G.da5), v4(G.dz5)); ia::note_launch(); }
+    e = e ? e : wgrad<32, 16>(s, G.f, G.u1, G.dz5, g + layer_w(4), st);
+    e = e ? e : conv32<16, 32>(s, G.f, G.dz5, W(4), 1, nullptr, nullptr, G.du1, nullptr, 0, st);
+    { up_bwd_relu_k<<<nblk(G.hf.cells() * 8), 256, 0, st>>>(G.hf, 8, v4(G.du1), v4(G.z4), v4(G.dz4)); ia::note_launch(); }
+    e = e ? e : wgrad<32, 32>(s, G.hf, G.u2, G.dz4, g + layer_w(3), st);
+    e = e ? e : conv32<32, 32>(s, G.hf, G.dz4, W(3), 1, nullptr, nullptr, G.du2, nullptr, 0, st);
+    { up_bwd_relu_k<<<nblk(G.qt.cells() * 8), 256, 0, st>>>(G.qt, 8, v4(G.du2), v4(G.z3), v4(G.dz3)); ia::note_launch(); }
+    e = e ? e : wgrad<32, 32>(s, G.qt, G.p2, G.dz3, g + layer_w(2), st);
+    e = e ? e : conv32<32, 32>(s, G.qt, G.dz3, W(2), 1, nullptr, nullptr, G.dp2, nullptr, 0, st);
+    // a2 feeds the skip connection (du2) and the pooling (dp2)
+    { pool_bwd_relu_k<<<nblk(G.hf.cells() * 8), 256, 0, st>>>(G.hf, 8, v4(G.du2), v4(G.dp2), v4(G.z2), v4(G.dz2)); ia::note_launch(); }
+    e = e ? e : wgrad<16, 32>(s, G.hf, G.p1, G.dz2, g + layer_w(1), st);
+    e = e ? e : conv32<32, 16>(s, G.hf, G.dz2, W(1), 1, nullptr, nullptr, G.dp1, nullptr, 0, st);
+    // a1 feeds the skip connection (da5) and the pooling (dp1)
+    { pool_bwd_relu_k<<<nblk(G.f.cells() * 4), 256, 0, st>>>(G.f, 4, v4(G.da5), v4(G.dp1), v4(G.z1), v4(G.dz1)); ia::note_launch(); }
+    e = e ? e : wgrad<4, 16>(s, G.f, G.x0, G.dz1, g + layer_w(0), st);
+    return e ? e : cudaGetLastError();
 }
 
 int loss_grad(ia_handle* h, NNState* s, const float* x0, const float* tgt, const nn::Dims& f, double* loss_out) {
@@ -870,13 +725,14 @@ int loss_grad(ia_handle* h, NNState* s, const float* x0, const float* tgt, const
     if (ensure_graph(h, s, f, G) != IA_OK) return IA_ERR_CUDA;
     cudaMemcpyAsync(G.x0, x0, sizeof(float) * f.padded() * 4, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(G.tgt, tgt, sizeof(float) * f.padded(), cudaMemcpyDeviceToDevice, st);
-    forward_f32(G, s->w, st);
+    if (forward_f32(s, G, st) != cudaSuccess) return IA_ERR_CUDA;
     cudaMemsetAsync(s->dloss, 0, 8, st);
     const int nbl = nblk(f.cells()) < 1024 ? nblk(f.cells()) : 1024;
     if (s->loss_kind == 1) { nn::energy_k<<<nbl, 256, 0, st>>>(f, G.out, G.tgt, G.x0, G.dout, s->dloss); ia::note_launch(); }
     else { nn::mse_k<<<nbl, 256, 0, st>>>(f, G.out, G.tgt, G.dout, s->dloss); ia::note_launch(); }
-    { nn::zero_f32<<<256, 256, 0, st>>>(nn::NPARAM, s->g); ia::note_launch(); }
-    backward_f32(G, s->w, s->g, st);
+    if (!s->part && cudaMalloc(&s->part, sizeof(float) * (size_t)(nn::WG_BLOCKS * s->sms) * nn::Wgrad<32, 32>::N) != cudaSuccess)
+        return IA_ERR_CUDA;
+    if (backward_f32(s, G, st) != cudaSuccess) return IA_ERR_CUDA;
     if (loss_out) {
         cudaMemcpyAsync(loss_out, s->dloss, 8, cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) return IA_ERR_CUDA;
@@ -1042,7 +898,7 @@ void nn_destroy(ia_handle* h) {
     if (!s) return;
     cudaFree(s->w); cudaFree(s->g); cudaFree(s->m); cudaFree(s->v);
     for (int l = 0; l < nn::NLAYER; ++l) cudaFree(s->wtc[l]);
-    cudaFree(s->bias_tc); cudaFree(s->buf); cudaFree(s->ibuf); cudaFree(s->x16);
+    cudaFree(s->bias_tc); cudaFree(s->buf); cudaFree(s->part); cudaFree(s->ibuf); cudaFree(s->x16);
     cudaFree(s->dloss); cudaFree(s->derr); cudaFree(s->dscale);
     delete s;
     h->nn = nullptr;
@@ -1095,7 +951,7 @@ int ia_nn_forward(ia_handle* h, const float* x0, float* out, int32_t B, int32_t 
         Graph G;
         if (ensure_graph(h, s, f, G) != IA_OK) return IA_ERR_CUDA;
         cudaMemcpyAsync(G.x0, x0, sizeof(float) * f.padded() * 4, cudaMemcpyDeviceToDevice, st);
-        forward_f32(G, s->w, st);
+        if (forward_f32(s, G, st) != cudaSuccess) return IA_ERR_CUDA;
         cudaMemcpyAsync(out, G.out, sizeof(float) * f.padded(), cudaMemcpyDeviceToDevice, st);
         return cuda_fail(cudaStreamSynchronize(st));
     }
