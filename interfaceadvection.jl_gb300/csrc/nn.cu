@@ -3,14 +3,11 @@
 //  * Training kernels (FP32, CUDA cores; the convolutions and their gradients in
 //    nn_train.cuh): MSE and energy losses, Adam.
 //  * Inference kernel (BF16 weights and activations, FP32 accumulation on the
-//    5th-generation tensor cores): implicit GEMM with M = 128 output cells,
-//    N = Cout, K = 27 taps x Cin.  Per tap the 128 x Cin im2col tile is staged in
-//    shared memory in the canonical K-major core-matrix layout; one elected
-//    thread issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32 in TMEM) and
-//    tcgen05.commit to a per-stage mbarrier; the four warps read the 128 x Cout
-//    accumulator back with tcgen05.ld for the bias / ReLU / skip epilogue.
-//    Every mbarrier wait is bounded; on timeout the kernel raises an error flag,
-//    releases its TMEM and returns.
+//    5th-generation tensor cores): implicit GEMM with M = 128 output cells, a
+//    patch marched through z, fed by TMA; tcgen05.mma (kind::f16, BF16 x BF16 ->
+//    FP32 in TMEM) from one elected thread, tcgen05.ld for the bias / ReLU /
+//    skip epilogue.  Every mbarrier wait is bounded; on timeout the kernel
+//    raises an error flag, waits for its copies, releases its TMEM and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -158,9 +155,10 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
-// Poll an mbarrier phase for at most ~1 s of wall time (and a fixed number of polls).
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    const uint64_t t0 = global_ns();
+// Poll an mbarrier phase for at most ~1 s of wall time (and a fixed number of polls), or until *fail (another
+// wait of the block has given up).
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, const volatile int* fail) {
+    uint64_t t0 = 0;
     for (uint32_t i = 0; i < (1u << 28); ++i) {
         uint32_t ok = 0;
         asm volatile(
@@ -169,7 +167,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
             : "r"(mbar), "r"(parity)
             : "memory");
         if (ok) return true;
-        if ((i & 255u) == 255u && global_ns() - t0 > 1000000000ull) return false;
+        if ((i & 255u) == 255u) {
+            if (fail && *fail) return false;
+            const uint64_t t = global_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > 1000000000ull) return false;
+        }
     }
     return false;
 }
@@ -188,60 +191,105 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 
 // ------------------------------------------------------------------ TMA-fed tensor-core convolution
 // Inference activations are stored as 8-channel planes: plane j holds channels 8j..8j+7 of every
-// (padded, halo-included) cell, 16 B per cell, so a run of cells of one plane is contiguous.
-// A tile is M = 128 consecutive cells of one x-row (rows shorter than 128 leave the tail masked).
-// For each of the 9 (dy, dz) neighbour rows and each plane, one TMA box of WR = 136 consecutive
-// cells (2176 contiguous bytes) lands in shared memory as 136 rows of 16 B: the chunk column of a
-// K-major no-swizzle operand whose 8-row core matrices are contiguous (SBO 128 B) and whose
-// K-neighbour chunks are one box apart (LBO = 2176 B).  The A operand of tap (dx, dy, dz) is the
-// (dy, dz) window started dx + 1 rows in, so all 27 taps are read from one set of 9·Cin/8 boxes.
-// Two stages: thread 0 issues the next tile's boxes before the MMAs of this one; one commit per
-// tile releases the epilogue (all four warps, tcgen05.ld) and the stage.
-constexpr int kM = 128;   // output cells per tile (the MMA M)
-constexpr int WR = 136;
-constexpr int BOX_BYTES = WR * 16;
+// (padded, halo-included) cell, 16 B per cell.
+// A block marches a patch of 8 x 16 cells (x, y: the MMA's M = 128 rows) through up to ZP planes of z.  One TMA box
+// brings one z plane of the patch with its halo, all channels: 10 x 18 cells of 16 B for each 8 channels, the
+// 160 B of a row as one run.  In
+// shared memory that is a K-major no-swizzle operand: 8 cells of a row are a core matrix of 128 B, the next row is
+// 160 B on (SBO), the next 8 channels one box on (LBO), and the A operand of tap (dx, dy) starts (dy+1)·10 + dx+1
+// cells in.  A plane is loaded once and multiplied once for its three output planes: the B operand of a tap has
+// the weights of dz = +1, 0, -1 side by side (N = 3·Cout) and the accumulators of the output planes z-1, z, z+1
+// are neighbouring column blocks of TMEM.  An output's 27·Cin products are added in the order of the taps
+// (dz, then dy, dx, then channels), as one tap after the other into one accumulator would.
+// Warp 4 issues the loads, warp 5 the MMAs, warps 0-3 read finished planes with tcgen05.ld and clear their columns
+// for the next patch; a ring of NS stages and per-plane barriers let the three run independently, also from one
+// patch to the next.  The MMAs of a plane have one accumulator and one shape; the next plane's, one column block on,
+// are issued when they have finished (the order of MMAs on overlapping accumulators of another base or shape is not
+// specified), while the other block of the multiprocessor keeps the tensor cores busy.
+// What bounds it: an MMA takes about 50 ns whatever its N (16 more of them a plane cost 110 us more over 242 planes
+// a multiprocessor: the A operand's rows, not the products), so the 9·Cin/16 MMAs a plane, a third of a tap-by-tap
+// N = Cout form's.  A plane is fetched from L2 1.4 times (halo) instead of 9 times.  Measured, 32 -> 16 channels on
+// 128 x 256 x 128 cells: 1334 us with the tap-by-tap kernel (one 128-cell row a tile, 9 windows each), 213 us here;
+// 16 -> 16 channels 389 and 103 us.
+constexpr int kM = 128;                  // output cells per patch plane (the MMA M)
+constexpr int kPX = 8, kPY = 16;         // patch
+constexpr int kBX = kPX + 2, kBY = kPY + 2;
+constexpr int BOX_BYTES = kBX * kBY * 16;   // one plane of a patch, 8 channels
+constexpr int kTmemCols = 256;           // two blocks share a multiprocessor's 512
+constexpr int kConvThreads = 192;
 
 template <int CI, int COP>
 struct TmaSmem {
     static constexpr int W_BYTES = 27 * COP * CI * 2;
-    static constexpr int NBOX = 9 * (CI / 8);
-    static constexpr int STAGE_BYTES = NBOX * BOX_BYTES;
+    static constexpr int STAGE_BYTES = CI / 8 * BOX_BYTES;
+    static constexpr int NS = COP > 16 ? 4 : 6;
+    static constexpr int ZP = kTmemCols / COP;                       // output planes in flight
     static constexpr int A_OFF = (W_BYTES + 1023) / 1024 * 1024;
-    static constexpr int BAR_OFF = A_OFF + 2 * STAGE_BYTES;
-    static constexpr int TOTAL = BAR_OFF + 64;
+    static constexpr int BAR_OFF = A_OFF + NS * STAGE_BYTES;
+    static constexpr int USED = BAR_OFF + 8 * (2 * NS + 2 * ZP + 1);
+    // at least 80 KB, so that no third block waits for TMEM on a multiprocessor
+    static constexpr int TOTAL = USED > 80 * 1024 ? USED : 80 * 1024;
+    static_assert(STAGE_BYTES % 128 == 0, "TMA destination");
 };
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+// box at (x, y, z) of the padded grid: the innermost dimension runs over the 8 channels of the cells of a row
+__device__ __forceinline__ void tma_load_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar)
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(8 * x), "r"(y), "r"(z), "r"(0), "r"(bar)
         : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc) {   // D += A B
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(1u));
+}
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+                 "r"(0u)
+                 : "memory");
 }
 
 template <int CI, int CO, bool RELU, bool OUTF32>
-__global__ void __launch_bounds__(128) conv_tma_kernel(const __grid_constant__ CUtensorMap tmap, Dims d,
-                                                       const uint8_t* __restrict__ Wg, const float* __restrict__ bias,
-                                                       const __nv_bfloat16* __restrict__ skip,
-                                                       __nv_bfloat16* __restrict__ Y, float* __restrict__ Yf,
-                                                       int* __restrict__ err) {
+__global__ void __launch_bounds__(kConvThreads) conv_tma_kernel(const __grid_constant__ CUtensorMap tmap, Dims d,
+                                                                int zc, const uint8_t* __restrict__ Wg,
+                                                                const float* __restrict__ bias,
+                                                                const __nv_bfloat16* __restrict__ skip,
+                                                                __nv_bfloat16* __restrict__ Y, float* __restrict__ Yf,
+                                                                int* __restrict__ err) {
     constexpr int COP = CO < 16 ? 16 : CO;
     using S = TmaSmem<CI, COP>;
+    constexpr int NS = S::NS;
     static_assert(CI % 16 == 0 && COP % 16 == 0 && COP <= 32, "tile shape");
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t tmem_holder;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    for (int i = tid; i < S::W_BYTES / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(smem)[i] = __ldg(reinterpret_cast<const uint4*>(Wg) + i);
-    const uint32_t full0 = smem_u32(smem + S::BAR_OFF), mdone = full0 + 16;
+    __shared__ int fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // weights: chunk (tap of the plane q, block k) holds dz = 1 - k
+    constexpr int CHUNK = COP * CI * 2 / 16;
+    for (int i = tid; i < S::W_BYTES / 16; i += blockDim.x) {
+        const int q = i / (3 * CHUNK), k = i / CHUNK % 3;
+        reinterpret_cast<uint4*>(smem)[i] = __ldg(reinterpret_cast<const uint4*>(Wg) + ((2 - k) * 9 + q) * CHUNK + i % CHUNK);
+    }
+    const uint32_t full0 = smem_u32(smem + S::BAR_OFF), empty0 = full0 + 8 * NS, out0 = empty0 + 8 * NS,
+                   free0 = out0 + 8 * S::ZP, drain = free0 + 8 * S::ZP;
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mdone));
+        fail = 0;
+        for (int k = 0; k < 2 * NS + S::ZP; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * k));
+        for (int k = 0; k < S::ZP; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(free0 + 8 * k));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drain));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
-                     "r"(32));
+                     "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // weights: generic writes, async reads
@@ -249,139 +297,154 @@ __global__ void __launch_bounds__(128) conv_tma_kernel(const __grid_constant__ C
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_holder;
-    const uint32_t wbase = smem_u32(smem), abase = smem_u32(smem + S::A_OFF);
-    constexpr uint32_t idesc = idesc_bf16(kM, COP);
-    const int xtiles = (d.nx + kM - 1) / kM;
-    const long long ntiles = (long long)xtiles * d.ny * d.nz * d.B;
-    const int rowp = d.nx + 2;
-    const long long planep = (long long)(d.nx + 2) * (d.ny + 2);
-    const long long plane = d.padded() * 8;   // elements per 8-channel plane
-    float bias_r[CO];
-#pragma unroll
-    for (int o = 0; o < CO; ++o) bias_r[o] = __ldg(bias + o);
-
-    auto tile_origin = [&](long long t, int& x0) -> long long {
-        x0 = int(t % xtiles) * kM;
-        long long r = t / xtiles;
-        const int y = int(r % d.ny);
-        r /= d.ny;
-        const int z = int(r % d.nz);
-        const int b = int(r / d.nz);
-        return d.pos(b, x0, y, z);
-    };
-    auto issue = [&](long long t, int s) {   // thread 0
-        int x0;
-        const long long p0 = tile_origin(t, x0);
-        const uint32_t bar = full0 + 8 * s;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(S::STAGE_BYTES)
-                     : "memory");
-        for (int w = 0; w < 9; ++w) {
-            const long long row = p0 - 1 + (long long)(w % 3 - 1) * rowp + (long long)(w / 3 - 1) * planep;
-#pragma unroll
-            for (int j = 0; j < CI / 8; ++j)
-                tma_load_2d(abase + s * S::STAGE_BYTES + (w * (CI / 8) + j) * BOX_BYTES, &tmap, 0,
-                            int(row + (long long)j * d.padded()), bar);
-        }
-    };
-    int issued[2] = {0, 0}, waited[2] = {0, 0}, commits = 0, commits_waited = 0;
-    if (tid == 0 && (long long)blockIdx.x < ntiles) issue(blockIdx.x, 0);
-    if ((long long)blockIdx.x < ntiles) issued[0] = 1;
-    bool failed = false;
-    int i = 0;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i) {
-        const int s = i & 1;
-        const long long next = tile + gridDim.x;
-        if (next < ntiles) {
-            if (tid == 0) issue(next, s ^ 1);
-            issued[s ^ 1] += 1;
-        }
-        bool ok = mbar_wait(full0 + 8 * s, uint32_t((i >> 1) & 1));
-        if (__syncthreads_or(!ok)) {
-            failed = true;
-            break;
-        }
-        waited[s] += 1;
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t st = abase + s * S::STAGE_BYTES;
-#pragma unroll 1
-            for (int t = 0; t < 27; ++t) {
-                const int w = t / 3, dx1 = t % 3;   // window (dy, dz) and dx + 1
-#pragma unroll
-                for (int ks = 0; ks < CI / 16; ++ks) {
-                    const uint64_t ad =
-                        smem_desc(st + (w * (CI / 8) + 2 * ks) * BOX_BYTES + dx1 * 16, BOX_BYTES, 128);
-                    const uint64_t bd = smem_desc(wbase + t * COP * CI * 2 + ks * 256, 128, CI * 16);
-                    const uint32_t acc = (t > 0 || ks > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-                }
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mdone)
-                         : "memory");
-        }
-        ++commits;
-        ok = mbar_wait(mdone, uint32_t(i & 1));
-        if (__syncthreads_or(!ok)) {
-            failed = true;
-            break;
-        }
-        ++commits_waited;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        int x0;
-        const long long p0 = tile_origin(tile, x0);
-        const bool valid = x0 + tid < d.nx;
-        const long long p = p0 + tid;
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-        if (OUTF32) {
-            float v[16];
-            tmem_ld16(trow, v);
-            if (valid) Yf[p] = v[0] + bias_r[0];
-        } else {
-#pragma unroll
-            for (int c0 = 0; c0 < CO; c0 += 16) {
-                float v[16];
-                tmem_ld16(trow + c0, v);
-                if (valid) {
-                    uint32_t packed[8];
-#pragma unroll
-                    for (int k = 0; k < 16; k += 2) {
-                        float a = v[k] + bias_r[c0 + k], b2 = v[k + 1] + bias_r[c0 + k + 1];
-                        if (RELU) {
-                            a = fmaxf(a, 0.f);
-                            b2 = fmaxf(b2, 0.f);
-                        }
-                        if (skip) {
-                            const long long sp = (long long)((c0 + k) / 8) * plane + p * 8 + (k % 8);
-                            const __nv_bfloat162 sk = *reinterpret_cast<const __nv_bfloat162*>(skip + sp);
-                            a += __low2float(sk);
-                            b2 += __high2float(sk);
-                        }
-                        const __nv_bfloat162 o2 = __floats2bfloat162_rn(a, b2);
-                        packed[k / 2] = *reinterpret_cast<const uint32_t*>(&o2);
-                    }
-                    *reinterpret_cast<uint4*>(Y + (long long)(c0 / 8) * plane + p * 8) =
-                        make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    *reinterpret_cast<uint4*>(Y + (long long)(c0 / 8 + 1) * plane + p * 8) =
-                        make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                }
-            }
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-    }
-    if (failed) {
-        if (tid == 0) atomicExch(err, 1);
-        // bounded drain: the last commit and every box load still in flight
-        if (commits > commits_waited) mbar_wait(mdone, uint32_t((commits - 1) & 1));
-        for (int s = 0; s < 2; ++s)
-            if (issued[s] > waited[s]) mbar_wait(full0 + 8 * s, uint32_t((issued[s] - 1) & 1));
+    if (warp < 4) {
+        for (int c0 = 0; c0 < kTmemCols; c0 += 16) tmem_zero16(tmem + c0 + ((uint32_t)(warp * 32) << 16));
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32));
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t wbase = smem_u32(smem), abase = smem_u32(smem + S::A_OFF);
+    const int npx = (d.nx + kPX - 1) / kPX, npy = (d.ny + kPY - 1) / kPY, npz = (d.nz + zc - 1) / zc;
+    const int items = npx * npy * npz * d.B;
+    // item -> patch origin and output planes [z0, z1)
+    auto item_of = [&](int it, int& x0, int& y0, int& z0, int& z1, int& b) {
+        x0 = it % npx * kPX;
+        it /= npx;
+        y0 = it % npy * kPY;
+        it /= npy;
+        z0 = it % npz * zc;
+        z1 = min(z0 + zc, d.nz);
+        b = it / npz;
+    };
+    // a wait gives up when another role has, or after about a second; the kernel then raises err and ends
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        const bool ok = mbar_wait(bar, parity, &fail);
+        if (!ok) atomicExch(&fail, 1);
+        return ok;
+    };
+    if (warp == 4 && lane == 0) {   // loads
+        int n = 0;   // planes issued
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            int x0, y0, z0, z1, b;
+            item_of(it, x0, y0, z0, z1, b);
+            for (int zi = z0 - 1; zi <= z1; ++zi, ++n) {
+                const int s = n % NS;
+                if (n >= NS && !(ok = wait(empty0 + 8 * s, uint32_t(n / NS - 1) & 1))) break;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s), "r"(S::STAGE_BYTES)
+                             : "memory");
+                // padded coordinates of the box's first cell: x0 - 1 + 1, ...
+                tma_load_box(abase + s * S::STAGE_BYTES, &tmap, x0, y0, b * (d.nz + 2) + zi + 1, full0 + 8 * s);
+            }
+        }
+        // a block must not end with copies in flight
+        if (!ok)
+            for (int k = n > NS ? n - NS : 0; k < n; ++k) mbar_wait(full0 + 8 * (k % NS), uint32_t(k / NS) & 1, nullptr);
+    } else if (warp == 5 && lane == 0) {   // MMAs
+        int n = 0;
+        uint32_t used = 0, par = 0;   // per TMEM block: used before, parity of its uses
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            int x0, y0, z0, z1, b;
+            item_of(it, x0, y0, z0, z1, b);
+            for (int zi = z0 - 1; zi <= z1; ++zi, ++n) {
+                const int s = n % NS;
+                if (!(ok = wait(full0 + 8 * s, uint32_t(n / NS) & 1))) break;
+                if (n > 0 && !(ok = wait(empty0 + 8 * ((n - 1) % NS), uint32_t((n - 1) / NS) & 1))) break;   // the last plane's MMAs
+                // weight blocks k0..k1: output planes zi-1+k0 .. zi-1+k1 inside [z0, z1)
+                const int k0 = zi - 1 < z0 ? z0 - zi + 1 : 0, k1 = zi + 1 >= z1 ? z1 - zi : 2;
+                if (k1 == 2) {   // the first products of plane zi + 1: its block has to be free and cleared
+                    const int slot = zi + 1 - z0;
+                    if ((used >> slot) & 1)
+                        if (!(ok = wait(free0 + 8 * slot, ((par >> slot) & 1) ^ 1))) break;
+                    used |= 1u << slot;
+                    par ^= 1u << slot;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t st = abase + s * S::STAGE_BYTES, dcol = tmem + (zi - 1 + k0 - z0) * COP;
+                const uint32_t nb = k1 - k0 + 1, idesc = idesc_bf16(kM, 0) | (nb * COP >> 3 << 17);
+                // one thread issues: descriptors by constant steps from the plane's first (addresses are below 2^18,
+                // so a step never leaves the 14-bit address field), or the issue takes longer than the MMA
+                const uint64_t ad = smem_desc(st, BOX_BYTES, kBX * 16);
+                const uint64_t bd = smem_desc(wbase + k0 * COP * CI * 2, 128, CI * 16);
+#pragma unroll
+                for (int q = 0; q < 9; ++q)
+#pragma unroll
+                    for (int ks = 0; ks < CI / 16; ++ks)
+                        mma_bf16(dcol, ad + ((2 * ks * BOX_BYTES + (q / 3 * kBX + q % 3) * 16) >> 4),
+                                 bd + ((q * 3 * COP * CI * 2 + ks * 256) >> 4), idesc);
+                mma_commit(empty0 + 8 * s);
+                if (zi - 1 >= z0) mma_commit(out0 + 8 * (zi - 1 - z0));
+            }
+        }
+        mma_commit(drain);
+        mbar_wait(drain, 0, nullptr);
+    } else if (warp < 4) {   // finished planes
+        uint32_t par = 0;
+        float bias_r[CO];
+#pragma unroll
+        for (int o = 0; o < CO; ++o) bias_r[o] = __ldg(bias + o);
+        const long long plane = d.padded() * 8;   // elements per 8-channel plane
+        const int px = tid & 7, py = tid >> 3;    // row of the accumulator: cell (px, py) of the patch
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            int x0, y0, z0, z1, b;
+            item_of(it, x0, y0, z0, z1, b);
+            const bool valid = x0 + px < d.nx && y0 + py < d.ny;
+            for (int z = z0; z < z1; ++z) {
+                const int slot = z - z0;
+                ok = wait(out0 + 8 * slot, (par >> slot) & 1);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                par ^= 1u << slot;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const long long p = d.pos(b, x0 + px, y0 + py, z);
+                const uint32_t trow = tmem + slot * COP + ((uint32_t)(warp * 32) << 16);
+                float v[COP];
+#pragma unroll
+                for (int c0 = 0; c0 < COP; c0 += 16) tmem_ld16(trow + c0, *reinterpret_cast<float(*)[16]>(v + c0));
+#pragma unroll
+                for (int c0 = 0; c0 < COP; c0 += 16) tmem_zero16(trow + c0);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(free0 + 8 * slot);
+                if (!valid) continue;
+                if (OUTF32) {
+                    Yf[p] = v[0] + bias_r[0];
+                } else {
+#pragma unroll
+                    for (int c0 = 0; c0 < CO; c0 += 8) {
+                        uint32_t packed[4];
+                        uint4 sk4 = make_uint4(0u, 0u, 0u, 0u);
+                        if (skip) sk4 = __ldg(reinterpret_cast<const uint4*>(skip + (long long)(c0 / 8) * plane + p * 8));
+                        const uint32_t* skp = reinterpret_cast<const uint32_t*>(&sk4);
+#pragma unroll
+                        for (int k = 0; k < 8; k += 2) {
+                            float a = v[c0 + k] + bias_r[(c0 + k) % CO], b2 = v[c0 + k + 1] + bias_r[(c0 + k + 1) % CO];
+                            if (RELU) {
+                                a = fmaxf(a, 0.f);
+                                b2 = fmaxf(b2, 0.f);
+                            }
+                            if (skip) {
+                                const __nv_bfloat162 sk = *reinterpret_cast<const __nv_bfloat162*>(&skp[k / 2]);
+                                a += __low2float(sk);
+                                b2 += __high2float(sk);
+                            }
+                            const __nv_bfloat162 o2 = __floats2bfloat162_rn(a, b2);
+                            packed[k / 2] = *reinterpret_cast<const uint32_t*>(&o2);
+                        }
+                        *reinterpret_cast<uint4*>(Y + (long long)(c0 / 8) * plane + p * 8) =
+                            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0 && fail) atomicExch(err, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
 // ------------------------------------------------------------------ BF16 glue kernels (inference)
@@ -518,6 +581,7 @@ struct NNState {
     // preconditioner input (BF16, 16 channels, grid-shaped) and its scale
     __nv_bfloat16* x16 = nullptr;
     size_t x16_bytes = 0;
+    nn::Dims x16_dims{0, 0, 0, 0};
     unsigned int* dscale = nullptr;
     double* dloss = nullptr;
     int* derr = nullptr;
@@ -672,7 +736,6 @@ cudaError_t wgrad(const NNState* s, const nn::Dims& d, const float* X, const flo
     return cudaGetLastError();
 }
 
-inline const float4* v4(const float* p) { return reinterpret_cast<const float4*>(p); }
 inline float4* v4(float* p) { return reinterpret_cast<float4*>(p); }
 
 // forward of the training graph (inputs already in G.x0)
@@ -784,16 +847,17 @@ EncodeTiled encode_tiled() {
     return fn;
 }
 
-// tensor map of a BF16 activation stored as Cin/8 planes of 8 channels: a 2D view of
-// (Cin/8)·rows cells x 8 channels, box = 8 channels x WR cells; loads past either end read zeros
-bool make_act_map(CUtensorMap* m, const __nv_bfloat16* X, int CI, long long rows) {
+// tensor map of a BF16 activation stored as Cin/8 planes of 8 channels: (channel and x, y, z and batch, plane) of
+// the padded cells, box = one z plane of a patch with its halo, every plane; loads past an end read zeros
+bool make_act_map(CUtensorMap* m, const __nv_bfloat16* X, int CI, const nn::Dims& d) {
     EncodeTiled enc = encode_tiled();
     if (!enc) return false;
-    const cuuint64_t dims[2] = {8, (cuuint64_t)rows * (CI / 8)};
-    const cuuint64_t strides[1] = {16};
-    const cuuint32_t box[2] = {8, (cuuint32_t)nn::WR};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(X), dims, strides, box, estr,
+    const cuuint64_t nx = d.nx + 2, ny = d.ny + 2, nz = (cuuint64_t)(d.nz + 2) * d.B;
+    const cuuint64_t dims[4] = {8 * nx, ny, nz, (cuuint64_t)(CI / 8)};
+    const cuuint64_t strides[3] = {16 * nx, 16 * nx * ny, 16 * nx * ny * nz};
+    const cuuint32_t box[4] = {8 * nn::kBX, (cuuint32_t)nn::kBY, 1, (cuuint32_t)(CI / 8)};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(X), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -803,14 +867,20 @@ cudaError_t launch_tma(const nn::Dims& d, const __nv_bfloat16* X, const uint8_t*
                        const __nv_bfloat16* skip, __nv_bfloat16* Y, float* Yf, int* err, cudaStream_t st, int sms) {
     using Sm = nn::TmaSmem<CI, CO < 16 ? 16 : CO>;
     CUtensorMap map;
-    if (!make_act_map(&map, X, CI, d.padded())) return cudaErrorNotSupported;
+    if (!make_act_map(&map, X, CI, d)) return cudaErrorNotSupported;
     auto kfn = nn::conv_tma_kernel<CI, CO, RELU, OUTF32>;
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, Sm::TOTAL);
     if (e != cudaSuccess) return e;
-    const long long tiles = (long long)((d.nx + nn::kM - 1) / nn::kM) * d.ny * d.nz * d.B;
-    const int per_sm = Sm::TOTAL <= 110 * 1024 ? 2 : 1;
-    const int grid = int(tiles < (long long)per_sm * sms ? tiles : (long long)per_sm * sms);
-    { kfn<<<grid, 128, Sm::TOTAL, st>>>(map, d, W, b, skip, Y, Yf, err); ia::note_launch(); }
+    // output planes of an item: z cut evenly; shorter cuts where the patches alone would leave multiprocessors idle
+    const long long patches = (long long)((d.nx + nn::kPX - 1) / nn::kPX) * ((d.ny + nn::kPY - 1) / nn::kPY) * d.B;
+    long long cuts = (d.nz + Sm::ZP - 1) / Sm::ZP;
+    cuts = std::min<long long>(std::max<long long>(cuts, 2ll * sms / patches), std::max(1, d.nz / 4));
+    cuts = std::max<long long>(cuts, (d.nz + Sm::ZP - 1) / Sm::ZP);
+    const int zc = int((d.nz + cuts - 1) / cuts);
+    const long long items = patches * ((d.nz + zc - 1) / zc);
+    if (items > 0x7fffffffll) return cudaErrorInvalidValue;
+    const int grid = int(std::min<long long>(items, 2ll * sms));
+    { kfn<<<grid, nn::kConvThreads, Sm::TOTAL, st>>>(map, d, zc, W, b, skip, Y, Yf, err); ia::note_launch(); }
     return cudaGetLastError();
 }
 
@@ -841,8 +911,7 @@ int forward_tc(ia_handle* h, NNState* s, const nn::Dims& f, const __nv_bfloat16*
     auto tk = [&](long long n) { __nv_bfloat16* p = c; c += (n + 63) / 64 * 64; return p; };
     __nv_bfloat16 *a1 = tk(F * 16), *u1 = tk(F * 32), *a5 = tk(F * 16), *p1 = tk(H * 16), *a2 = tk(H * 32),
                   *u2 = tk(H * 32), *a4 = tk(H * 32), *p2 = tk(Q * 32), *a3 = tk(Q * 32);
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+    const int sms = s->sms;
     const float* b = s->bias_tc;
     cudaError_t e = cudaSuccess;
     e = e ? e : conv_layer(16, 16, true, false, f, x16, s->wtc[0], b + 0, nullptr, a1, nullptr);
@@ -856,6 +925,24 @@ int forward_tc(ia_handle* h, NNState* s, const nn::Dims& f, const __nv_bfloat16*
     e = e ? e : conv_layer(32, 16, true, false, f, u1, s->wtc[4], b + 128, a1, a5, nullptr);
     e = e ? e : conv_layer(16, 1, false, true, f, a5, s->wtc[5], b + 160, nullptr, nullptr, out);
     return e == cudaSuccess ? IA_OK : IA_ERR_CUDA;
+}
+
+// the BF16 input of the inference path (16 channels), its halo and the channels that no one writes zero
+int ensure_x16(NNState* s, const nn::Dims& f, cudaStream_t st) {
+    const size_t need = 2 * 16 * (size_t)f.padded();
+    if (need > s->x16_bytes) {
+        cudaFree(s->x16);
+        s->x16 = nullptr;
+        s->x16_bytes = 0;
+        s->x16_dims = nn::Dims{0, 0, 0, 0};
+        if (cudaMalloc(&s->x16, need) != cudaSuccess) return IA_ERR_CUDA;
+        s->x16_bytes = need;
+    }
+    if (!same_dims(f, s->x16_dims)) {
+        if (cudaMemsetAsync(s->x16, 0, need, st) != cudaSuccess) return IA_ERR_CUDA;
+        s->x16_dims = f;
+    }
+    return IA_OK;
 }
 
 int check_dims(int B, int nx, int ny, int nz) {
@@ -872,15 +959,7 @@ int nn_apply(ia_handle* h, const float* r, const float* L32, float* out, int nx,
     if (!s) return IA_ERR_CUDA;
     cudaStream_t st = h->stream;
     const nn::Dims f{1, nx, ny, nz};
-    const size_t need = 2 * 16 * (size_t)f.padded();
-    if (need > s->x16_bytes) {
-        cudaFree(s->x16);
-        s->x16 = nullptr;
-        s->x16_bytes = 0;
-        if (cudaMalloc(&s->x16, need) != cudaSuccess) return IA_ERR_CUDA;
-        s->x16_bytes = need;
-        if (cudaMemsetAsync(s->x16, 0, need, st) != cudaSuccess) return IA_ERR_CUDA;
-    }
+    if (ensure_x16(s, f, st) != IA_OK) return IA_ERR_CUDA;
     cudaMemsetAsync(s->dscale, 0, 4, st);
     const int nb = nblk(f.cells()) < 1216 ? nblk(f.cells()) : 1216;
     { nn::absmax_k<<<nb, 256, 0, st>>>(f, r, s->dscale); ia::note_launch(); }
@@ -955,16 +1034,14 @@ int ia_nn_forward(ia_handle* h, const float* x0, float* out, int32_t B, int32_t 
         cudaMemcpyAsync(out, G.out, sizeof(float) * f.padded(), cudaMemcpyDeviceToDevice, st);
         return cuda_fail(cudaStreamSynchronize(st));
     }
-    __nv_bfloat16* x16 = nullptr;
-    if (cudaMalloc(&x16, 2 * 16 * (size_t)f.padded()) != cudaSuccess) return IA_ERR_CUDA;
-    cudaMemsetAsync(x16, 0, 2 * 16 * (size_t)f.padded(), st);
-    { nn::in_to_bf16<<<nblk(f.cells()), 256, 0, st>>>(f, x0, x16); ia::note_launch(); }
+    if (ensure_x16(s, f, st) != IA_OK) return IA_ERR_CUDA;
+    { nn::in_to_bf16<<<nblk(f.cells()), 256, 0, st>>>(f, x0, s->x16); ia::note_launch(); }
     cudaMemsetAsync(s->derr, 0, 4, st);
-    int rc = forward_tc(h, s, f, x16, out);
-    cudaError_t e = cudaStreamSynchronize(st);
-    cudaFree(x16);
-    if (rc != IA_OK || e != cudaSuccess) return IA_ERR_CUDA;
-    return nn_error_flag(h) ? IA_ERR_CUDA : IA_OK;
+    if (forward_tc(h, s, f, s->x16, out) != IA_OK) return IA_ERR_CUDA;
+    int err = 0;
+    cudaError_t e = cudaMemcpyAsync(&err, s->derr, 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    return e != cudaSuccess || err ? IA_ERR_CUDA : IA_OK;
 }
 
 int ia_nn_loss_grad(ia_handle* h, const float* x0, const float* target, int32_t B, int32_t nx, int32_t ny,
