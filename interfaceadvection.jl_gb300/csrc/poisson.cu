@@ -81,6 +81,22 @@ __device__ __forceinline__ T off7(const Grid& g, const TL* __restrict__ L, const
     }
     return a;
 }
+// b - Σ_i L[I,i] v[I-δi] + L[I+δi,i] v[I+δi] as one chain of multiply-adds
+template <int D, class T>
+__device__ __forceinline__ T resid7(const Grid& g, const T* __restrict__ L, T b, const T* v, int I, const Nb& o) {
+    const int s1 = int(g.s[1]), s2 = int(g.s[2]);
+    const T* L1 = L + g.N;
+    T a = fma(-L[I], v[I + o.xl], b);
+    a = fma(-L[I + 1], v[I + o.xh], a);
+    a = fma(-L1[I], v[I + o.yl], a);
+    a = fma(-L1[I + s1], v[I + o.yh], a);
+    if (D == 3) {
+        const T* L2 = L1 + g.N;
+        a = fma(-L2[I], v[I + o.zl], a);
+        a = fma(-L2[I + s2], v[I + o.zh], a);
+    }
+    return a;
+}
 // D_I = -Σ_i (L[I,i] + L[I+δi,i])
 template <int D, class TL>
 __device__ __forceinline__ auto diag7(const Grid& g, const TL* __restrict__ L, int I) -> decltype(cf(L[0])) {
@@ -122,12 +138,13 @@ inline dim3 cell_grid(const Grid& g) {
     const long long I = lin(g, x, y, z);
 
 template <class T>
-__global__ void set_diag_k(Grid g, const T* __restrict__ L, T* __restrict__ iD) {
+__global__ void set_diag_k(Grid g, const T* __restrict__ L, T* __restrict__ iD, T* __restrict__ diag) {
     INTERIOR_XYZ
     T dd = T(0);
     for (int i = 0; i < g.D; ++i) dd -= L[I + i * g.N] + L[I + g.s[i] + i * g.N];
     const T eps = sizeof(T) == 8 ? T(2.220446049250313e-16) : T(1.1920929e-7);
     iD[I] = (dd * dd < T(2) * eps) ? T(0) : T(1) / dd;
+    if (diag) diag[I] = dd;
 }
 
 // Coarsening along a dimension e of n cells: the first pr[e] coarse cells cover two fine cells each, the
@@ -202,8 +219,10 @@ __global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, const d
 
 // Red-black Gauss-Seidel half-sweep, one thread per cell of the colour: thread tx takes the pair of
 // interior cells (1 + 2tx, 2 + 2tx) of its row and updates the one of this colour, so no
-// lane idles; the diagonal comes from the face coefficients the update reads anyway
-// (same value and zero-diagonal rule as set_diag_k).
+// lane idles; in FP32 the diagonal comes from the face coefficients the update reads anyway
+// (same value and zero-diagonal rule as set_diag_k).  In FP64 the inverse diagonal is read (set_diag_k) and the
+// update is a chain of 8 multiply-adds: with the diagonal's sums and the division it was about 30 FP64
+// instructions a cell, at 16 cycles a warp each the whole cost (100x200x100, mean over the levels: 18.2 -> 8.0 us).
 // With PROL (over-relaxed first red half-sweep of a post-smoothing whose prolongation is fused
 // into the sweeps) the cell's previous value is x + the injected coarse correction.
 // In 3D a thread takes its pair in RB_ZT consecutive z planes and reads every plane's operands before
@@ -221,8 +240,8 @@ inline dim3 pair_tile_grid(const Grid& g) {
 }
 template <class T, int D, bool PROL = false, class TL = T, bool REG = true>
 __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, const T* __restrict__ b,
-                            T* __restrict__ xv, int color, T omega, int conflicts, int cls, Grid gc = Grid(),
-                            const T* __restrict__ xc = nullptr) {
+                            const T* __restrict__ iD, T* __restrict__ xv, int color, T omega, int conflicts, int cls,
+                            Grid gc = Grid(), const T* __restrict__ xc = nullptr) {
     const int y = y0 + int(blockIdx.y * blockDim.y + threadIdx.y);   // rows [y0, y1) of the interior
     if (y >= y1) return;
     const int xp = 1 + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -240,15 +259,25 @@ __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, co
     auto load = [&](int x, int z, int& I, T& off, T& dd, T& bv, T& xo) {
         I = x + y * int(g.s[1]) + z * int(g.s[2]);
         const Nb o = nb_of<D>(g, x, y, z);
-        off = off7<D>(g, L, xv, I, o);
-        dd = diag7<D>(g, L, I);
-        bv = b[I];
+        if constexpr (sizeof(T) == 8) {
+            off = T(0);
+            dd = iD[I];
+            bv = resid7<D>(g, L, b[I], xv, I, o);
+        } else {
+            off = off7<D>(g, L, xv, I, o);
+            dd = diag7<D>(g, L, I);
+            bv = b[I];
+        }
         if (omega != T(1)) {
             xo = xv[I];
             if (PROL) xo += xc[mg_parent_cell<REG>(gc, x, y, z)];
         }
     };
     auto store = [&](int I, T off, T dd, T bv, T xo) {
+        if constexpr (sizeof(T) == 8) {
+            xv[I] = omega == T(1) ? bv * dd : fma(omega, fma(bv, dd, -xo), xo);
+            return;
+        }
         const T iD = (dd * dd < T(2) * eps) ? T(0) : T(1) / dd;
         const T gs = (bv - off) * iD;
         if (omega == T(1)) xv[I] = gs;
@@ -297,6 +326,7 @@ __device__ __forceinline__ T first_nb(const Grid& g, const Grid& gc, const T* __
     const bool in = cx >= 1 && cx <= g.n[0] - 2 && cy >= 1 && cy <= g.n[1] - 2 &&
                     (g.D == 2 || (cz >= 1 && cz <= g.n[2] - 2));
     if (!in) return xv[J];
+    if (!PROL && sizeof(T) == 8) return b[J] * iD[J];   // the caller's sum takes the factor omega
     if (PROL) return xv[J] + xc[mg_parent_cell<REG>(gc, cx, cy, cz)];
     return omega == T(1) ? b[J] * iD[J] : omega * (b[J] * iD[J]);
 }
@@ -350,7 +380,8 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
             for (int q = 0; q < 2 * D; ++q) v[q] = xv[J[q]] + xc[Pn[q]];
         } else {
 #pragma unroll
-            for (int q = 0; q < 2 * D; ++q) v[q] = omega == T(1) ? b[J[q]] * iD[J[q]] : omega * (b[J[q]] * iD[J[q]]);
+            for (int q = 0; q < 2 * D; ++q)
+                v[q] = omega == T(1) || sizeof(T) == 8 ? b[J[q]] * iD[J[q]] : omega * (b[J[q]] * iD[J[q]]);
         }
     } else {
         const Nb o = nb_of<D>(g, x, y, z);
@@ -365,6 +396,23 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
             v[4] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.zl, x, y, zl, omega);
             v[5] = first_nb<T, PROL, REG>(g, gc, b, iD, xc, xv, I + o.zh, x, y, zh, omega);
         }
+    }
+    if constexpr (sizeof(T) == 8) {
+        T a = fma(L[I], v[0], L[I + 1] * v[1]);
+        a = fma(L1[I], v[2], a);
+        a = fma(L1[I + s1], v[3], a);
+        if (D == 3) {
+            a = fma(L2[I], v[4], a);
+            a = fma(L2[I + s2], v[5], a);
+        }
+        if (PROL) {
+            const T gs = (b[I] - a) * iD[I];
+            const T xo = omega == T(1) ? T(0) : xv[I] + xc[mg_parent_cell<REG>(gc, x, y, z)];
+            xv[I] = omega == T(1) ? gs : fma(omega, gs - xo, xo);
+        } else {
+            xv[I] = omega * (fma(-omega, a, b[I]) * iD[I]);
+        }
+        return;
     }
     T a = cf(L[I]) * v[0] + cf(L[I + 1]) * v[1];
     a += cf(L1[I]) * v[2] + cf(L1[I + s1]) * v[3];
@@ -583,10 +631,11 @@ __global__ void residual_k(Grid g, const T* __restrict__ L, const T* __restrict_
 }
 
 // residual of the (at most 2^D) fine children of each coarse cell, summed straight into the coarse
-// right-hand side (residual_k + restrict_k without the fine residual array; same sums, same order)
+// right-hand side (no fine residual array); diag: the level's diagonal, read in FP64 only (7 multiply-adds a cell
+// instead of 17 FP64 operations)
 template <class T, int D, class TL = T, bool REG = true>
 __global__ void resid_restrict_k(Grid gc, int yc0, int yc1, Grid gf, const TL* __restrict__ L,
-                                 const T* __restrict__ b, const T* __restrict__ xv, T* __restrict__ bc) {
+                                 const T* __restrict__ diag, const T* __restrict__ b, const T* __restrict__ xv, T* __restrict__ bc) {
     const int xc = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int yc = yc0 + int(blockIdx.y * blockDim.y + threadIdx.y);   // coarse rows [yc0, yc1)
     const int zc = D == 3 ? 1 + int(blockIdx.z) : 0;
@@ -603,7 +652,8 @@ __global__ void resid_restrict_k(Grid gc, int yc0, int yc1, Grid gf, const TL* _
                 const int x = fx + i, y = fy + j, z = fz + k;
                 const int I = x + y * s1 + z * s2;
                 const Nb o = nb_of<D>(gf, x, y, z);
-                sum += b[I] - (off7<D>(gf, L, xv, I, o) + diag7<D>(gf, L, I) * xv[I]);
+                if constexpr (sizeof(T) == 8) sum += resid7<D>(gf, L, fma(-diag[I], xv[I], b[I]), xv, I, o);
+                else sum += b[I] - (off7<D>(gf, L, xv, I, o) + diag7<D>(gf, L, I) * xv[I]);
             }
     bc[xc + yc * int(gc.s[1]) + zc * int(gc.s[2])] = sum;
 }
@@ -629,6 +679,7 @@ struct TailArgs {
     Grid g[TAIL_MAX];
     const T* L[TAIL_MAX];
     const T* iD[TAIL_MAX];
+    const T* diag[TAIL_MAX];                         // FP64 only
     int off[TAIL_MAX];                               // x of the level in shared memory; b follows it
     int nu1[TAIL_MAX], nu2[TAIL_MAX];
     int nuc, total;                                  // total: shared values in all
@@ -694,11 +745,16 @@ __global__ void __launch_bounds__(TAIL_THREADS) mg_tail_k(const __grid_constant_
                     if (!px[k] || x > nx || (conflicts && wrap_class(g, conflicts, x, y, z) != cls)) continue;
                     const int I = x + y * s1 + z * s2;
                     const Nb o = nb_of<D>(g, x, y, z);
-                    T off = __ldg(L + I) * xv[I + o.xl] + __ldg(L + I + 1) * xv[I + o.xh];
-                    off += __ldg(L + N + I) * xv[I + o.yl] + __ldg(L + N + I + s1) * xv[I + o.yh];
-                    if (D == 3) off += __ldg(L + 2 * N + I) * xv[I + o.zl] + __ldg(L + 2 * N + I + s2) * xv[I + o.zh];
-                    const T gs = (b[I] - off) * __ldg(iD + I);
-                    xv[I] = om == T(1) ? gs : xv[I] + om * (gs - xv[I]);
+                    T r = fma(-__ldg(L + I), xv[I + o.xl], b[I]);
+                    r = fma(-__ldg(L + I + 1), xv[I + o.xh], r);
+                    r = fma(-__ldg(L + N + I), xv[I + o.yl], r);
+                    r = fma(-__ldg(L + N + I + s1), xv[I + o.yh], r);
+                    if (D == 3) {
+                        r = fma(-__ldg(L + 2 * N + I), xv[I + o.zl], r);
+                        r = fma(-__ldg(L + 2 * N + I + s2), xv[I + o.zh], r);
+                    }
+                    const T d = __ldg(iD + I);
+                    xv[I] = om == T(1) ? r * d : fma(om, fma(r, d, -xv[I]), xv[I]);
                 }
                 __syncthreads();
             }
@@ -723,7 +779,9 @@ __global__ void __launch_bounds__(TAIL_THREADS) mg_tail_k(const __grid_constant_
                 for (int j = 0; j < my; ++j)
                     for (int i = 0; i < mx; ++i) {
                         const int x = fx + i, y = fy + j, z = fz + k, I = x + y * int(g.s[1]) + z * int(g.s[2]);
-                        sum += b[I] - (off7<D>(g, a.L[l], xv, I, nb_of<D>(g, x, y, z)) + diag7<D>(g, a.L[l], I) * xv[I]);
+                        const Nb o = nb_of<D>(g, x, y, z);
+                        if constexpr (sizeof(T) == 8) sum += resid7<D>(g, a.L[l], fma(-a.diag[l][I], xv[I], b[I]), xv, I, o);
+                        else sum += b[I] - (off7<D>(g, a.L[l], xv, I, o) + diag7<D>(g, a.L[l], I) * xv[I]);
                     }
             bc[Ic] = sum;
         });
@@ -755,20 +813,6 @@ __global__ void __launch_bounds__(TAIL_THREADS) mg_tail_k(const __grid_constant_
 // cells).  FP64: 256, since a multiprocessor issues FP64 at 1/64 of the FP32 rate and a half-sweep on more cells is
 // faster spread over the device.
 template <class T> constexpr long long tail_pairs() { return sizeof(T) == 4 ? TAIL_PAIRS * TAIL_THREADS : 256; }
-
-template <class T>
-__global__ void zero_k(long long n, T* a) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        a[q] = T(0);
-}
-__global__ void to_f32_k(long long n, const double* __restrict__ a, float* __restrict__ b) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        b[q] = f32_rn(a[q]);
-}
-__global__ void to_f64_k(long long n, const float* __restrict__ a, double* __restrict__ b) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        b[q] = double(a[q]);
-}
 
 // ------------------------------------------------------------------ Krylov kernels
 // Row loops: a block takes whole x-rows of interior cells (rows dealt round-robin over a
@@ -1034,36 +1078,6 @@ __global__ void finalize_max_k(const unsigned long long* __restrict__ pmax, long
     if (threadIdx.x == 0) *out = m;
 }
 
-// q = A p and partial dot p·q
-template <int D>
-__global__ void matvec_dot_k(Grid g, const double* __restrict__ L, const double* __restrict__ diag,
-                             const double* __restrict__ pv, double* __restrict__ q, double* __restrict__ partial) {
-    double acc = 0.0, unused = 0.0;
-    ROWS_BEGIN_D(g)
-    const Nb o = nb_of<D>(g, x, y, z);
-    const double v = off7<D>(g, L, pv, I, o) + diag[I] * pv[I];
-    q[I] = v;
-    acc += pv[I] * v;
-    ROWS_END
-    block_sum2(acc, unused);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-}
-
-// partial dots s·q and s·r
-__global__ void dot2_k(Grid g, const double* __restrict__ sv, const double* __restrict__ q,
-                       const double* __restrict__ r, double* __restrict__ partial) {
-    double a1 = 0.0, a2 = 0.0;
-    ROWS_BEGIN(g)
-    a1 += sv[I] * q[I];
-    a2 += sv[I] * r[I];
-    ROWS_END
-    block_sum2(a1, a2);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = a1;
-        partial[gridDim.x + blockIdx.x] = a2;
-    }
-}
-
 // fixed-order sum of `n` partials for `k` quantities → out[0..k)
 // Σ partial[qd·n + i] over i in a fixed order, valid in thread 0 (a block of 1024 threads)
 __device__ double finalize_sum(const double* __restrict__ partial, long long n, int qd) {
@@ -1144,31 +1158,94 @@ __device__ void fcg_alpha(FcgDev* S, double pq) {
     S->alpha32 = float(alpha);
     S->stop = stop ? 1 : 0;
     S->rin = 0u;
+    S->rin64 = 0ull;
     if (!stop) {
         S->rho_prev = sr;
         S->alpha_prev = alpha;
     }
 }
 
-__global__ void xpby_k(Grid g, const double* __restrict__ sv, double beta, double* __restrict__ pv) {
-    ROWS_BEGIN(g)
-    pv[I] = (beta == 0.0) ? sv[I] : sv[I] + beta * pv[I];
-    ROWS_END
+// ---- FP64 Krylov kernels (IA_POISSON_FP64).  As the FP32 ones below, with the scalars on the device; the vectors
+// are the library's, whose ghost entries stay zero, so they are streamed whole.
+// q = A p and partial sums of p·q on the tiles of matvec32_tile_k, one chain of multiply-adds a cell
+template <int D, int ZT>
+__global__ void __launch_bounds__(256) matvec64_tile_k(Grid g, const double* __restrict__ L, const double* __restrict__ diag,
+                                                       const double* __restrict__ pv, double* __restrict__ q,
+                                                       double* __restrict__ partial, FcgDev* S) {
+    const int x = 1 + int(blockIdx.x) * 32 + int(threadIdx.x & 31), y = 1 + int(blockIdx.y) * 8 + int(threadIdx.x >> 5);
+    const int z0 = D == 3 ? 1 + ZT * int(blockIdx.z) : 0;
+    double acc = 0.0, unused = 0.0;
+    if (x <= g.n[0] - 2 && y <= g.n[1] - 2) {
+#pragma unroll
+        for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
+            const int z = z0 + k;
+            if (D == 3 && z > g.n[2] - 2) break;
+            const int I = x + y * int(g.s[1]) + z * int(g.s[2]);
+            const double v = -resid7<D>(g, L, -diag[I] * pv[I], pv, I, nb_of<D>(g, x, y, z));
+            q[I] = v;
+            acc = fma(pv[I], v, acc);
+        }
+    }
+    acc = warp_sum(acc);
+    __shared__ double ws[8];
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) acc += ws[w];
+        partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = acc;
+    }
+    if (!last_block(&S->done_mv, nb)) return;
+    double pq = 0.0;
+    sum2_by256(partial, nullptr, nb, pq, unused);
+    if (threadIdx.x == 0) fcg_alpha(S, pq);
 }
-
-// x += α p ; r -= α q ; L∞(r)
-__global__ void update_k(Grid g, double alpha, const double* __restrict__ pv, const double* __restrict__ q,
-                         double* __restrict__ xv, double* __restrict__ r, unsigned long long* linf) {
+__global__ void __launch_bounds__(256) dot2_64_k(long long n, const double* __restrict__ sv, const double* __restrict__ q,
+                                                 const double* __restrict__ r, double* __restrict__ partial, FcgDev* S, int first) {
+    double a1 = 0.0, a2 = 0.0;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+        const double s = sv[i];
+        a1 = fma(s, q[i], a1);
+        a2 = fma(s, r[i], a2);
+    }
+    block_sum2(a1, a2);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = a1;
+        partial[gridDim.x + blockIdx.x] = a2;
+    }
+    if (!last_block(&S->done_dot, gridDim.x)) return;
+    double sq = 0.0, sr = 0.0;
+    sum2_by256(partial, partial + gridDim.x, gridDim.x, sq, sr);
+    if (threadIdx.x == 0) fcg_beta(S, sq, sr, first);
+}
+__global__ void __launch_bounds__(256) xpby64_k(long long n, const double* __restrict__ sv, const FcgDev* __restrict__ S,
+                                                double* __restrict__ pv) {
+    const double beta = S->beta;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
+        pv[i] = beta == 0.0 ? sv[i] : fma(beta, pv[i], sv[i]);
+}
+// x += α p (x's ghost entries, the caller's, take the direction's zeros) ; r -= α q ; L∞(r) bits into S->rin64
+// (nothing after a breakdown)
+__global__ void __launch_bounds__(256) update64_k(long long n, FcgDev* __restrict__ S, const double* __restrict__ pv,
+                                                  const double* __restrict__ q, double* __restrict__ xv, double* __restrict__ r) {
+    if (S->stop) return;
+    const double alpha = S->alpha_prev;
     unsigned long long m = 0ull;
-    ROWS_BEGIN(g)
-    xv[I] += alpha * pv[I];
-    const double v = r[I] - alpha * q[I];
-    r[I] = v;
-    const unsigned long long b = abs_bits(v);
-    m = b > m ? b : m;
-    ROWS_END
+    const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
+        xv[i] = fma(alpha, pv[i], xv[i]);
+        const double v = fma(-alpha, q[i], r[i]);
+        r[i] = v;
+        const unsigned long long b = abs_bits(v);
+        m = b > m ? b : m;
+    }
     m = block_max(m);
-    if (threadIdx.x == 0) atomicMax(linf, m);
+    if (threadIdx.x == 0) atomicMax(&S->rin64, m);
 }
 
 // ---- FP32 inner Krylov kernels (mixed / learned): FP32 products, per-thread sums in FP32
@@ -1464,6 +1541,8 @@ static TailArgs<T> tail_args(PoissonMG* mg, int l0, int nu1, int nu2, int nuc) {
         a.g[k] = L.g;
         a.L[k] = L.template L_<T>();
         a.iD[k] = L.template iD_<T>();
+        a.diag[k] = nullptr;
+        if constexpr (sizeof(T) == 8) a.diag[k] = L.r;
         a.off[k] = a.total;
         a.total += 2 * int(L.g.N);
         a.nu1[k] = (l0 + k == 0 && mg->nu1f > 0) ? mg->nu1f : nu1;
@@ -1510,7 +1589,7 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
             int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
             tb_launch(mg, ta, 2 * nu1, st);
             timing_end(h, tk);
-            { resid_restrict_k<T, 3><<<cell_grid(C.g), blk(), 0, st>>>(C.g, 1, C.g.n[1] - 1, L.g, Lc, b, L.r32, C.template b_<T>()); ia::note_launch(); }
+            { resid_restrict_k<T, 3><<<cell_grid(C.g), blk(), 0, st>>>(C.g, 1, C.g.n[1] - 1, L.g, Lc, (const T*)nullptr, b, L.r32, C.template b_<T>()); ia::note_launch(); }
             cudaError_t e = vcycle<T>(h, mg, l + 1, st, nu1, nu2, nuc);
             if (e != cudaSuccess) return e;
             ta.xin = L.r32;
@@ -1547,8 +1626,8 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
             if (cls & ~conf) continue;
             auto go = [&](const auto* coef) {
                 using TL = std::decay_t<decltype(*coef)>;
-                if (L.g.D == 3) rbgs_pair_k<T, 3, false, TL><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, color, om, conf, cls);
-                else rbgs_pair_k<T, 2, false, TL><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, color, om, conf, cls);
+                if (L.g.D == 3) rbgs_pair_k<T, 3, false, TL><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, iD, x, color, om, conf, cls);
+                else rbgs_pair_k<T, 2, false, TL><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, iD, x, color, om, conf, cls);
             };
             if constexpr (sizeof(T) == 4) {
                 if (L16) go(L16);
@@ -1567,8 +1646,8 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
         auto go = [&](auto REG, const auto* coef) {
             using TL = std::decay_t<decltype(*coef)>;
             constexpr bool R = decltype(REG)::value;
-            if (L.g.D == 3) rbgs_pair_k<T, 3, true, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, 0, om, 0, 0, C.g, xc);
-            else rbgs_pair_k<T, 2, true, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, x, 0, om, 0, 0, C.g, xc);
+            if (L.g.D == 3) rbgs_pair_k<T, 3, true, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, iD, x, 0, om, 0, 0, C.g, xc);
+            else rbgs_pair_k<T, 2, true, TL, R><<<gr, blk(), 0, st>>>(L.g, y0, y1, coef, b, iD, x, 0, om, 0, 0, C.g, xc);
         };
         if constexpr (sizeof(T) == 4) {
             if (L16) reg ? go(std::true_type{}, L16) : go(std::false_type{}, L16);
@@ -1610,11 +1689,13 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto restrict_rows = [&](int yc0, int yc1) {
         const dim3 gr = rows(cell_grid(C.g), yc0, yc1);
         T* bc = C.template b_<T>();
+        const T* dg = nullptr;   // FP64: the diagonal is kept in the level's scratch vector
+        if constexpr (sizeof(T) == 8) dg = L.r;
         auto go = [&](auto REG, const auto* coef) {
             using TL = std::decay_t<decltype(*coef)>;
             constexpr bool R = decltype(REG)::value;
-            if (L.g.D == 3) resid_restrict_k<T, 3, TL, R><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, coef, b, x, bc);
-            else resid_restrict_k<T, 2, TL, R><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, coef, b, x, bc);
+            if (L.g.D == 3) resid_restrict_k<T, 3, TL, R><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, coef, dg, b, x, bc);
+            else resid_restrict_k<T, 2, TL, R><<<gr, blk(), 0, st>>>(C.g, yc0, yc1, L.g, coef, dg, b, x, bc);
         };
         if constexpr (sizeof(T) == 4) {
             if (L16) reg ? go(std::true_type{}, L16) : go(std::false_type{}, L16);
@@ -1838,8 +1919,9 @@ int mg_create(ia_handle* h) {
         return IA_ERR_CUDA;
     const size_t N = (size_t)g0.N;
     cudaError_t e = cudaSuccess;
-    e = e ? e : cudaMalloc(&mg->r, 8 * N);
-    e = e ? e : cudaMalloc(&mg->s, 8 * N);
+    // FP64: the finest level's right-hand side is the Krylov residual; mixed: the FP64 true residual
+    if (!mixed) mg->r = mg->lev[0].b;
+    else e = e ? e : cudaMalloc(&mg->r, 8 * N);
     e = e ? e : cudaMalloc(&mg->p, 8 * N);
     e = e ? e : cudaMalloc(&mg->q, 8 * N);
     mg->kb = kblocks(g0);
@@ -1881,7 +1963,6 @@ int mg_create(ia_handle* h) {
     e = e ? e : cudaMallocHost(&mg->hsc, 8 * 16);
     if (e != cudaSuccess) return IA_ERR_CUDA;
     cudaMemset(mg->r, 0, 8 * N);
-    cudaMemset(mg->s, 0, 8 * N);
     cudaMemset(mg->p, 0, 8 * N);
     cudaMemset(mg->q, 0, 8 * N);
     mg->nu1 = 2;
@@ -1902,7 +1983,8 @@ void mg_destroy(ia_handle* h) {
         cudaFree(L.x32); cudaFree(L.b32); cudaFree(L.r32); cudaFree(L.L32); cudaFree(L.iD32); cudaFree(L.L16);
         cudaFree(L.ratio);
     }
-    cudaFree(mg->r); cudaFree(mg->s); cudaFree(mg->p); cudaFree(mg->q);
+    if (mg->r != mg->lev[0].b) cudaFree(mg->r);
+    cudaFree(mg->p); cudaFree(mg->q);
     cudaFree(mg->p32); cudaFree(mg->q32); cudaFree(mg->e32);
     cudaFree(mg->rl32); cudaFree(mg->nl32); cudaFree(mg->t32);
     cudaFree(mg->partial); cudaFree(mg->dsc); cudaFree(mg->fcg); cudaFree(mg->diag64);
@@ -1924,11 +2006,11 @@ static cudaError_t mg_setup(ia_handle* h, const double* L0) {
     if (!mixed) { set_diag64_k<<<mg->kb, KTHREADS, 0, st>>>(F.g, L0, mg->diag64); ia::note_launch(); }
     if (!mixed) {
         cudaMemcpyAsync(F.L, L0, 8 * nv, cudaMemcpyDeviceToDevice, st);
-        { set_diag_k<double><<<grd(F.g), blk(), 0, st>>>(F.g, F.L, F.iD); ia::note_launch(); }
+        { set_diag_k<double><<<grd(F.g), blk(), 0, st>>>(F.g, F.L, F.iD, F.r); ia::note_launch(); }
         for (int l = 1; l < mg->nlev; ++l) {
             { restrict_L_k<double><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l - 1].g,
                                                                        mg->lev[l - 1].L, mg->lev[l].ratio, mg->lev[l].L); ia::note_launch(); }
-            { set_diag_k<double><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l].L, mg->lev[l].iD); ia::note_launch(); }
+            { set_diag_k<double><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l].L, mg->lev[l].iD, mg->lev[l].r); ia::note_launch(); }
         }
     } else {
         // FP64 diagonal, FP32 (and FP16) coefficient copies and the FP32 inverse diagonal in one pass
@@ -1938,35 +2020,8 @@ static cudaError_t mg_setup(ia_handle* h, const double* L0) {
         for (int l = 1; l < mg->nlev; ++l) {
             { restrict_L_k<float><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l - 1].g,
                                                                       mg->lev[l - 1].L32, mg->lev[l].ratio, mg->lev[l].L32); ia::note_launch(); }
-            { set_diag_k<float><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l].L32, mg->lev[l].iD32); ia::note_launch(); }
+            { set_diag_k<float><<<grd(mg->lev[l].g), blk(), 0, st>>>(mg->lev[l].g, mg->lev[l].L32, mg->lev[l].iD32, nullptr); ia::note_launch(); }
         }
-    }
-    return cudaGetLastError();
-}
-
-// s = M r (one V-cycle)
-static cudaError_t mg_precondition(ia_handle* h) {
-    PoissonMG* mg = h->mg;
-    cudaStream_t st = h->stream;
-    MGLevel& F = mg->lev[0];
-    const long long N = F.g.N;
-    cudaError_t e;
-    if (h->cfg.poisson_mode != IA_POISSON_FP64) {
-        int tk = timing_begin(h, TK_MG_TRANSFER);
-        { to_f32_k<<<1216, 256, 0, st>>>(N, mg->r, F.b32); ia::note_launch(); }
-        timing_end(h, tk);
-        tk = timing_begin(h, TK_MG_SMOOTH);
-        e = vcycle_run<float>(h, mg, st);
-        timing_end(h, tk);
-        if (e != cudaSuccess) return e;
-        { to_f64_k<<<1216, 256, 0, st>>>(N, F.x32, mg->s); ia::note_launch(); }
-    } else {
-        cudaMemcpyAsync(F.b, mg->r, 8 * N, cudaMemcpyDeviceToDevice, st);
-        int tk = timing_begin(h, TK_MG_SMOOTH);
-        e = vcycle_run<double>(h, mg, st);
-        timing_end(h, tk);
-        if (e != cudaSuccess) return e;
-        cudaMemcpyAsync(mg->s, F.x, 8 * N, cudaMemcpyDeviceToDevice, st);
     }
     return cudaGetLastError();
 }
@@ -2000,7 +2055,6 @@ static int poisson_solve_mixed(ia_handle* h, double* xv, const double* zz, const
     PoissonMG* mg = h->mg;
     cudaStream_t st = h->stream;
     const Grid& g = h->g;
-    const dim3 gb = grd(g);
     MGLevel& F = mg->lev[0];
     const long long N = g.N;
     unsigned long long* dlinf = reinterpret_cast<unsigned long long*>(mg->dsc + 8);
@@ -2133,45 +2187,36 @@ int poisson_solve(ia_handle* h, double* xv, const double* zz, const double* L, d
     }
     cudaStream_t st = h->stream;
     const Grid& g = h->g;
-    const dim3 gb = grd(g);
     if (mg_setup(h, L) != cudaSuccess) return IA_ERR_CUDA;
     unsigned long long* dlinf = reinterpret_cast<unsigned long long*>(mg->dsc + 8);
-    double* dots = mg->dsc;
+    MGLevel& F = mg->lev[0];
+    // the residual is the V-cycle's right-hand side and the preconditioned residual its result, in place
+    double* r = mg->r;
     int tk = timing_begin(h, TK_KRYLOV);
     true_residual(mg, g, L, zz, xv, dlinf, st);
     timing_end(h, tk);
     double res = read_linf(h, dlinf);
+    FcgDev* S = mg->fcg;
+    cudaMemsetAsync(&S->done_dot, 0, 2 * sizeof(unsigned int), st);   // as in poisson_solve_mixed
     int it = 0;
-    double rho_prev = 0.0, alpha_prev = 0.0;
     while (!(res <= tol) && it < itmx) {
-        if (mg_precondition(h) != cudaSuccess) return IA_ERR_CUDA;
-        tk = timing_begin(h, TK_KRYLOV);
-        { dot2_k<<<mg->kb, KTHREADS, 0, st>>>(g, mg->s, mg->q, mg->r, mg->partial); ia::note_launch(); }
-        { finalize_k<<<1, 1024, 0, st>>>(mg->partial, mg->kb, 2, dots); ia::note_launch(); }
+        tk = timing_begin(h, TK_MG_SMOOTH);
+        const cudaError_t e = vcycle_run<double>(h, mg, st);
         timing_end(h, tk);
-        cudaMemcpyAsync(mg->hsc + 2, dots, 16, cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) return IA_ERR_CUDA;
-        const double sq = mg->hsc[2], sr = mg->hsc[3];
+        if (e != cudaSuccess) return IA_ERR_CUDA;
         // flexible CG: β = s_k·(r_k - r_{k-1}) / (s_{k-1}·r_{k-1}) with r_k - r_{k-1} = -α q_{k-1}
-        const double beta = (it == 0) ? 0.0 : (-alpha_prev * sq) / rho_prev;
-        const double rho = sr;
         tk = timing_begin(h, TK_KRYLOV);
-        { xpby_k<<<mg->kb, KTHREADS, 0, st>>>(g, mg->s, beta, mg->p); ia::note_launch(); }
-        LAUNCH_D(g, matvec_dot_k, mg->kb, KTHREADS, g, L, mg->diag64, mg->p, mg->q, mg->partial);
-        { finalize_k<<<1, 1024, 0, st>>>(mg->partial, mg->kb, 1, dots); ia::note_launch(); }
+        { dot2_64_k<<<mg->vb, KTHREADS, 0, st>>>(g.N, F.x, mg->q, r, mg->partial, S, it == 0 ? 1 : 0); ia::note_launch(); }
+        { xpby64_k<<<mg->vb, KTHREADS, 0, st>>>(g.N, F.x, S, mg->p); ia::note_launch(); }
+        LAUNCH_TILE(g, matvec64_tile_k, g, L, mg->diag64, mg->p, mg->q, mg->partial, S);
+        { update64_k<<<mg->vb, KTHREADS, 0, st>>>(g.N, S, mg->p, mg->q, xv, r); ia::note_launch(); }
         timing_end(h, tk);
-        cudaMemcpyAsync(mg->hsc + 2, dots, 8, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(mg->hsc + 2, &S->rin64, 16, cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) return IA_ERR_CUDA;
-        const double pq = mg->hsc[2];
-        if (!(pq != 0.0) || !std::isfinite(pq)) break;
-        const double alpha = rho / pq;
-        cudaMemsetAsync(dlinf, 0, 8, st);
-        tk = timing_begin(h, TK_KRYLOV);
-        { update_k<<<mg->kb, KTHREADS, 0, st>>>(g, alpha, mg->p, mg->q, xv, mg->r, dlinf); ia::note_launch(); }
-        timing_end(h, tk);
-        res = read_linf(h, dlinf);
-        rho_prev = rho;
-        alpha_prev = alpha;
+        int stop = 0;
+        std::memcpy(&stop, reinterpret_cast<const char*>(mg->hsc + 3) + offsetof(FcgDev, stop) - offsetof(FcgDev, rin), 4);
+        if (stop) break;
+        std::memcpy(&res, mg->hsc + 2, 8);
         ++it;
     }
     { perbc_k<<<unsigned((bc_plane_cells(g) + 255) / 256), 256, 0, st>>>(g, xv); ia::note_launch(); }

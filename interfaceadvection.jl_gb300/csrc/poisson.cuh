@@ -17,6 +17,7 @@ constexpr int MG_MAX_LEVELS = 32;   // a dimension has less than 2^31 cells
 struct FcgDev {
     double alpha_prev, rho_prev, sr, beta;
     float beta32, alpha32;
+    unsigned long long rin64;   // L∞ of the FP64 solver's residual (bits), read back with the next two
     unsigned int rin;   // read back together with stop (8 bytes)
     int stop;
     unsigned int done_dot, done_mv;   // blocks finished in the current reduction kernel (0 between launches)
@@ -54,7 +55,7 @@ template <> inline float* MGLevel::iD_<float>() { return iD32; }
 struct PoissonMG {
     int nlev = 0;
     ia::MGLevel lev[ia::MG_MAX_LEVELS];
-    double *r = nullptr, *s = nullptr, *p = nullptr, *q = nullptr;   // fine-level Krylov vectors (FP64)
+    double *r = nullptr, *p = nullptr, *q = nullptr;                  // fine-level Krylov vectors (FP64)
     float *p32 = nullptr, *q32 = nullptr, *e32 = nullptr;             // inner FP32 Krylov vectors (mixed)
     float *rl32 = nullptr, *nl32 = nullptr, *t32 = nullptr;           // learned: residual, net output, A·net
     int precond = 0;                                                  // IA_PRECOND_* of the learned mode
