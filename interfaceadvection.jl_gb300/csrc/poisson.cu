@@ -666,153 +666,348 @@ __global__ void prolong_k(Grid gf, Grid gc, const T* __restrict__ xc, T* __restr
 }
 
 // The small levels of the V-cycle in one launch: a single block runs the whole cycle below (and on) the first
-// level of at most tail_pairs<T>() pairs of cells, with x and b of every such level in shared memory and a block barrier
-// between the stages.  The stages are those of the levels above (first red half-sweep from zero, relaxed red-black
-// half-sweeps, residual restriction, prolongation); the coarsest level is solved by nuc symmetric sweeps on its
-// mean-free right-hand side (a colour swept twice in a row keeps its values, so those sweeps are skipped).
-// What bounds it: the chain of barriers and shared-memory latencies, about 0.3 us a stage, where a launch of its
-// own takes 2 to 3 us whatever the size.
-constexpr int TAIL_MAX = 16, TAIL_THREADS = 1024, TAIL_PAIRS = 2;
+// level of at most tail_pairs<T>() pairs of cells, with a block barrier between the stages.  The stages are those of
+// the levels above (relaxed red-black half-sweeps from zero, residual restriction, prolongation); the coarsest level
+// is solved by nuc symmetric sweeps on its mean-free right-hand side (a colour swept twice in a row keeps its
+// values, so those sweeps are skipped).
+// Shared memory holds, for each level, x on the ghost-padded grid, and by pairs of x-neighbours (thread t of the
+// level has pair t, its red and its black cell) the right-hand side, the 2D face coefficients and the inverse
+// diagonal, and the cells' indices.  Ghosts across a periodic wrap are kept as copies by the thread that writes their
+// cell, so that a cell's neighbours lie at the same distances everywhere.
+// What bounds it: latency, a chain of about 40 stages of 0.4 us, where a launch of its own takes 2 to 3 us.
+// A level's sizes are kept in registers (keep): read from the kernel's parameters, which the compiler otherwise does
+// again in every stage, they cost more than the stage's arithmetic (1000 cycles a stage, of which 130 the update).
+constexpr int TAIL_MAX = 16, TAIL_THREADS = 1024, TAIL_PAIRS = 2, TAIL_WORDS = 4;
+// v, as a value that the compiler can only keep
+__device__ __forceinline__ int keep(int v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+template <class T>
+__device__ __forceinline__ T* keep(T* v) {
+    asm volatile("" : "+l"(v));
+    return v;
+}
 template <class T>
 struct TailArgs {
     int nl;                                          // levels; 0 is the largest
     Grid g[TAIL_MAX];
     const T* L[TAIL_MAX];
     const T* iD[TAIL_MAX];
-    const T* diag[TAIL_MAX];                         // FP64 only
-    int off[TAIL_MAX];                               // x of the level in shared memory; b follows it
+    int np[TAIL_MAX];                                // pairs
+    int xo[TAIL_MAX], bo[TAIL_MAX], co[TAIL_MAX];    // x, right-hand side, coefficients (offsets in values)
+    int io[TAIL_MAX];                                // TAIL_WORDS a pair (offset in words behind the values)
+    int ro, values, words;                           // residual scratch; sizes in all
     int nu1[TAIL_MAX], nu2[TAIL_MAX];
-    int nuc, total;                                  // total: shared values in all
+    int nuc;
     T omega;
     const T* b;                                      // right-hand side and result of level 0
     T* x;
+    size_t bytes() const { return sizeof(T) * (size_t)values + 4 * (size_t)words; }
 };
-
+// flags of a cell: copies to keep at x + n, x - n, y + n, ... (bits 0-5); its wrap_class (bits 6-8); two children
+// along x, y, z (bits 9-11)
+template <int D>
+__device__ __forceinline__ unsigned tail_flags(const Grid& g, int conflicts, int x, int y, int z) {
+    const int c[3] = {x, y, z};
+    unsigned f = unsigned(wrap_class(g, conflicts, x, y, z)) << 6;
+#pragma unroll
+    for (int e = 0; e < D; ++e) {
+        if (g.isper(e)) f |= (c[e] == 1 ? 1u << 2 * e : 0u) | (c[e] == g.n[e] - 2 ? 2u << 2 * e : 0u);
+        if (c[e] <= g.pr[e]) f |= 512u << e;
+    }
+    return f;
+}
+// distances to the copies across the wraps
+struct Wraps {
+    int w0, w1, w2;
+    __device__ Wraps(const Grid& g) : w0(keep(g.n[0] - 2)), w1(keep((g.n[1] - 2) * int(g.s[1]))), w2(keep((g.n[2] - 2) * int(g.s[2]))) {}
+};
 template <class T, int D>
-__global__ void __launch_bounds__(TAIL_THREADS) mg_tail_k(const __grid_constant__ TailArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char tail_raw[];
-    T* sm = reinterpret_cast<T*>(tail_raw);
-    __shared__ T mean_s;
-    const int tid = threadIdx.x;
-    // every interior cell of a level, as f(x, y, z, index)
-    auto cells = [&](const Grid& g, auto&& f) {
-        const int nx = g.n[0] - 2, ny = g.n[1] - 2, nz = D == 3 ? g.n[2] - 2 : 1, n = nx * ny * nz;
-        for (int t = tid; t < n; t += TAIL_THREADS) {
-            const int r = t / nx, x = 1 + t - r * nx, rz = r / ny, y = 1 + r - rz * ny, z = D == 3 ? 1 + rz : 0;
-            f(x, y, z, x + y * int(g.s[1]) + z * int(g.s[2]));
+__device__ __forceinline__ void tail_store(const Wraps& w, T* x, int I, unsigned f, T v) {
+    x[I] = v;
+    if (f & 63u) {
+        if (f & 1u) x[I + w.w0] = v;
+        if (f & 2u) x[I - w.w0] = v;
+        if (f & 4u) x[I + w.w1] = v;
+        if (f & 8u) x[I - w.w1] = v;
+        if (D == 3) {
+            if (f & 16u) x[I + w.w2] = v;
+            if (f & 32u) x[I - w.w2] = v;
         }
-    };
-    // nh half-sweeps x += omega (x_GS - x) of alternating colours from color0 on, after x += P(x of level l + 1)
-    // when prol.  A thread keeps its (at most TAIL_PAIRS) pairs of cells in x, decoded once: the divisions would
-    // otherwise be most of a stage's instructions.
-    auto sweeps = [&](int l, int nh, int color0, T om, bool prol) {
+    }
+}
+template <int D>
+__device__ __forceinline__ void tail_pair(const Grid& g, int t, int& x, int& y, int& z) {
+    const int hx = (g.n[0] - 1) / 2, ny = g.n[1] - 2, r = t / hx, rz = r / ny;
+    x = 1 + 2 * (t - r * hx);
+    y = 1 + r - rz * ny;
+    z = D == 3 ? 1 + rz : 0;
+}
+// Pair t of level g in TAIL_WORDS words at w (with a stride): its first cell with bit 30 when that is the red one and
+// bit 31 when there is a second; the flags of both (16 bits each); their parents on gc; the first child of the first
+// cell on gf (that of the second lies 2 on, or 1 behind a single child).  gc, gf: null where there is no such level.
+template <int D>
+__device__ __forceinline__ void tail_words(const Grid& g, const Grid* gc, const Grid* gf, int t, unsigned* w, int step) {
+    int x, y, z;
+    tail_pair<D>(g, t, x, y, z);
+    const int conflicts = wrap_conflicts(g);
+    const bool two = x < g.n[0] - 2;
+    w[0] = unsigned(x + y * int(g.s[1]) + z * int(g.s[2])) | (((x + y + z) & 1) ? 0u : 1u << 30) | (two ? 1u << 31 : 0u);
+    w[step] = tail_flags<D>(g, conflicts, x, y, z) | (two ? tail_flags<D>(g, conflicts, x + 1, y, z) << 16 : 0u);
+    w[2 * step] = gc ? unsigned(mg_parent_cell<false>(*gc, x, y, z)) | (two ? unsigned(mg_parent_cell<false>(*gc, x + 1, y, z)) << 16 : 0u) : 0u;
+    w[3 * step] = gf ? unsigned(lin(*gf, mg_child(g, 0, x), mg_child(g, 1, y), D == 3 ? mg_child(g, 2, z) : 0)) : 0u;
+}
+// the words by colour: cells (0: none), flags, parents (red in the low half words)
+struct PairCells {
+    unsigned red = 0, black = 0, fl = 0;
+    bool swap = false;   // the first cell is black
+    __device__ PairCells() {}
+    __device__ PairCells(unsigned w0, unsigned w1) {
+        const unsigned I = w0 & 0x3FFFFFFFu, J = w0 >> 31 ? I + 1 : 0u;
+        swap = !(w0 >> 30 & 1u);
+        red = swap ? J : I;
+        black = swap ? I : J;
+        fl = order(w1);
+    }
+    __device__ unsigned order(unsigned v) const { return swap ? v >> 16 | v << 16 : v; }
+};
+// Σ of the children of a coarse cell with flags f, the first at r
+template <class T, int D>
+__device__ __forceinline__ T tail_children(const T* r, unsigned f, int s1, int s2) {
+    const bool bx = f & 512u, by = f & 1024u, bz = D == 3 && (f & 2048u);
+    T v[8];
+#pragma unroll
+    for (int q = 0; q < (D == 3 ? 8 : 4); ++q) {
+        const bool in = (!(q & 1) || bx) && (!(q & 2) || by) && (!(q & 4) || bz);
+        v[q] = in ? r[(q & 1 ? 1 : 0) + (q & 2 ? s1 : 0) + (q & 4 ? s2 : 0)] : T(0);
+    }
+    T sum = v[0];
+#pragma unroll
+    for (int q = 1; q < (D == 3 ? 8 : 4); ++q) sum += v[q];
+    return sum;
+}
+
+// coefficients and cell words of every level into shared memory
+template <class T, int D>
+__device__ void tail_setup(const TailArgs<T>& a, T* sm) {
+    const int tid = threadIdx.x;
+    unsigned* w = reinterpret_cast<unsigned*>(sm + a.values);
+    for (int k = 0; k < a.nl; ++k) {
+        const Grid& g = a.g[k];
+        const int np = keep(a.np[k]), N = keep(int(g.N)), s1 = keep(int(g.s[1])), s2 = keep(int(g.s[2])), co = keep(a.co[k]), io = keep(a.io[k]);
+        const T* __restrict__ L0 = keep(a.L[k]);
+        const T* __restrict__ iD = keep(a.iD[k]);
+        for (int t = tid; t < np; t += TAIL_THREADS) {
+            tail_words<D>(g, k + 1 < a.nl ? &a.g[k + 1] : nullptr, k > 0 ? &a.g[k - 1] : nullptr, t, w + io + t, np);
+            const PairCells pc(w[io + t], 0u);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int I = c ? pc.black : pc.red;
+                const T* L = L0 + I;
+                T v[7] = {};
+                if (I) {
+                    v[0] = __ldg(L);
+                    v[1] = __ldg(L + 1);
+                    v[2] = __ldg(L + N);
+                    v[3] = __ldg(L + N + s1);
+                    v[4] = __ldg(iD + I);
+                    if (D == 3) {
+                        v[5] = __ldg(L + 2 * N);
+                        v[6] = __ldg(L + 2 * N + s2);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 2 * D + 1; ++q) sm[co + (2 * q + c) * np + t] = v[q];
+            }
+        }
+    }
+}
+
+// one V-cycle on the levels (after tail_setup); mean_s: shared
+template <class T, int D>
+__device__ __forceinline__ void tail_cycle(const TailArgs<T>& a, T* sm, T& mean_s) {
+    const int tid = threadIdx.x, last = keep(a.nl) - 1;
+    const unsigned* w = reinterpret_cast<const unsigned*>(sm + keep(a.values));
+    T* scratch = sm + keep(a.ro);
+    // A visit of a level: nh half-sweeps x += om (x_GS - x) of alternating colours from color0 on.
+    //  mode 0: from x = 0 (nh >= 1), then the restriction of the residual into the next level's right-hand side
+    //  mode 1: after x += P(x of the next level)
+    //  mode 2: the coarsest level, from x = 0
+    auto visit = [&](int l, int nh, int color0, T om, int mode) {
         const Grid& g = a.g[l];
-        T* xv = sm + a.off[l];
-        const T* b = xv + g.N;
-        const T* __restrict__ L = a.L[l];
-        const T* __restrict__ iD = a.iD[l];
-        const int N = int(g.N), s1 = int(g.s[1]), s2 = int(g.s[2]);
-        const int nx = g.n[0] - 2, ny = g.n[1] - 2, nz = D == 3 ? g.n[2] - 2 : 1;
-        const int hx = (nx + 1) / 2, n = hx * ny * nz, conflicts = wrap_conflicts(g);
-        int px[TAIL_PAIRS], py[TAIL_PAIRS], pz[TAIL_PAIRS];   // px = 0: no pair
+        const int np = keep(a.np[l]), s1 = keep(int(g.s[1])), s2 = keep(int(g.s[2])), conflicts = keep(wrap_conflicts(g));
+        const int bo = keep(a.bo[l]), co = keep(a.co[l]), step = 2 * np;
+        const Wraps wr(g);
+        T* x = sm + keep(a.xo[l]);
+        const unsigned* id = w + keep(a.io[l]);
+        PairCells pc[TAIL_PAIRS];
 #pragma unroll
         for (int k = 0; k < TAIL_PAIRS; ++k) {
-            const int t = tid + k * TAIL_THREADS, r = t / hx, rz = r / ny;
-            px[k] = t < n ? 1 + 2 * (t - r * hx) : 0;
-            py[k] = 1 + r - rz * ny;
-            pz[k] = D == 3 ? 1 + rz : 0;
+            const int t = tid + k * TAIL_THREADS;
+            if (t < np) pc[k] = PairCells(id[t], id[np + t]);
         }
-        if (prol) {
-            const Grid& gc = a.g[l + 1];
-            const T* xc = sm + a.off[l + 1];
+        // b - Σ c x_nb of cell I, coefficients at c; Σ c when asked for
+        auto gather = [&](int c, int I, T r, T* dd) {
+            const T c0 = sm[c], c1 = sm[c + step], c2 = sm[c + 2 * step], c3 = sm[c + 3 * step];
+            const T x0 = x[I - 1], x1 = x[I + 1], x2 = x[I - s1], x3 = x[I + s1];
+            T c4 = T(0), c5 = T(0), x4 = T(0), x5 = T(0);
+            if (D == 3) {
+                c4 = sm[c + 5 * step];
+                c5 = sm[c + 6 * step];
+                x4 = x[I - s2];
+                x5 = x[I + s2];
+            }
+            if (dd) *dd = (c0 + c1) + (c2 + c3) + (c4 + c5);
+            r = fma(-c0, x0, r);
+            r = fma(-c1, x1, r);
+            r = fma(-c2, x2, r);
+            r = fma(-c3, x3, r);
+            if (D == 3) {
+                r = fma(-c4, x4, r);
+                r = fma(-c5, x5, r);
+            }
+            return r;
+        };
+        if (mode == 1) {
+            const T* xc = sm + keep(a.xo[l + 1]);
 #pragma unroll
             for (int k = 0; k < TAIL_PAIRS; ++k) {
-                if (!px[k]) continue;
-                const int row = py[k] * s1 + pz[k] * s2;
-                const int up = mg_parent(gc, 1, py[k]) * int(gc.s[1]) + (D == 3 ? mg_parent(gc, 2, pz[k]) * int(gc.s[2]) : 0);
-                xv[row + px[k]] += xc[up + mg_parent(gc, 0, px[k])];
-                if (px[k] < nx) xv[row + px[k] + 1] += xc[up + mg_parent(gc, 0, px[k] + 1)];
+                const int t = tid + k * TAIL_THREADS;
+                if (t >= np) continue;
+                const unsigned par = pc[k].order(id[2 * np + t]);
+                const int r = pc[k].red, b = pc[k].black;
+                const T vr = r ? x[r] + xc[par & 0xFFFFu] : T(0), vb = b ? x[b] + xc[par >> 16] : T(0);
+                if (r) tail_store<T, D>(wr, x, r, pc[k].fl & 0xFFFFu, vr);
+                if (b) tail_store<T, D>(wr, x, b, pc[k].fl >> 16, vb);
             }
             __syncthreads();
         }
         for (int s = 0; s < nh; ++s) {
-            const int color = (color0 + s) & 1;
+            const int color = (color0 + s) & 1, sh = 16 * color;
             for (int cls = 0; cls <= conflicts; ++cls) {
                 if (cls & ~conflicts) continue;
+                // the operands of every pair are read before the first store
+                T nv[TAIL_PAIRS];
 #pragma unroll
                 for (int k = 0; k < TAIL_PAIRS; ++k) {
-                    const int x = px[k] + (((px[k] + py[k] + pz[k]) & 1) != color), y = py[k], z = pz[k];
-                    if (!px[k] || x > nx || (conflicts && wrap_class(g, conflicts, x, y, z) != cls)) continue;
-                    const int I = x + y * s1 + z * s2;
-                    const Nb o = nb_of<D>(g, x, y, z);
-                    T r = fma(-__ldg(L + I), xv[I + o.xl], b[I]);
-                    r = fma(-__ldg(L + I + 1), xv[I + o.xh], r);
-                    r = fma(-__ldg(L + N + I), xv[I + o.yl], r);
-                    r = fma(-__ldg(L + N + I + s1), xv[I + o.yh], r);
-                    if (D == 3) {
-                        r = fma(-__ldg(L + 2 * N + I), xv[I + o.zl], r);
-                        r = fma(-__ldg(L + 2 * N + I + s2), xv[I + o.zh], r);
-                    }
-                    const T d = __ldg(iD + I);
-                    xv[I] = om == T(1) ? r * d : fma(om, fma(r, d, -xv[I]), xv[I]);
+                    const int t = tid + k * TAIL_THREADS, I = color ? pc[k].black : pc[k].red;
+                    if (!I) continue;
+                    const int c = co + color * np + t;
+                    const T xo = x[I], d = sm[c + 4 * step], r = gather(c, I, sm[bo + color * np + t], nullptr);
+                    nv[k] = om == T(1) ? r * d : fma(om, fma(r, d, -xo), xo);
+                }
+#pragma unroll
+                for (int k = 0; k < TAIL_PAIRS; ++k) {
+                    const int I = color ? pc[k].black : pc[k].red;
+                    const unsigned f = pc[k].fl >> sh & 0xFFFFu;
+                    if (I && int(f >> 6 & 7u) == cls) tail_store<T, D>(wr, x, I, f, nv[k]);
                 }
                 __syncthreads();
             }
         }
-    };
-    // level 0's right-hand side (its ghost entries are zero); everything else from zero
-    const int N0 = int(a.g[0].N);
-    for (int q = tid; q < a.total; q += TAIL_THREADS) sm[q] = q >= N0 && q < 2 * N0 ? a.b[q - N0] : T(0);
-    __syncthreads();
-    const int last = a.nl - 1;
-    for (int l = 0; l < last; ++l) {
-        const Grid &g = a.g[l], &gc = a.g[l + 1];
-        T* xv = sm + a.off[l];
-        const T* b = xv + g.N;
-        sweeps(l, 2 * a.nu1[l], 0, a.omega, false);
-        T* bc = sm + a.off[l + 1] + gc.N;
-        cells(gc, [&](int X, int Y, int Z, int Ic) {
-            const int fx = mg_child(gc, 0, X), fy = mg_child(gc, 1, Y), fz = D == 3 ? mg_child(gc, 2, Z) : 0;
-            const int mx = mg_children(gc, 0, X), my = mg_children(gc, 1, Y), mz = D == 3 ? mg_children(gc, 2, Z) : 1;
-            T sum = T(0);
-            for (int k = 0; k < mz; ++k)
-                for (int j = 0; j < my; ++j)
-                    for (int i = 0; i < mx; ++i) {
-                        const int x = fx + i, y = fy + j, z = fz + k, I = x + y * int(g.s[1]) + z * int(g.s[2]);
-                        const Nb o = nb_of<D>(g, x, y, z);
-                        if constexpr (sizeof(T) == 8) sum += resid7<D>(g, a.L[l], fma(-a.diag[l][I], xv[I], b[I]), xv, I, o);
-                        else sum += b[I] - (off7<D>(g, a.L[l], xv, I, o) + diag7<D>(g, a.L[l], I) * xv[I]);
-                    }
-            bc[Ic] = sum;
-        });
+        if (mode != 0) return;
+#pragma unroll
+        for (int k = 0; k < TAIL_PAIRS; ++k)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int t = tid + k * TAIL_THREADS, I = c ? pc[k].black : pc[k].red;
+                if (!I) continue;
+                T dd;
+                const T r = gather(co + c * np + t, I, sm[bo + c * np + t], &dd);
+                scratch[I] = fma(dd, x[I], r);
+            }
         __syncthreads();
+        const int npc = keep(a.np[l + 1]), bc = keep(a.bo[l + 1]), ic = keep(a.io[l + 1]);
+        for (int t = tid; t < npc; t += TAIL_THREADS) {
+            const unsigned w0 = w[ic + t], f = w[ic + npc + t];
+            const T* r = scratch + w[ic + 3 * npc + t];
+            const int first = bc + (w0 >> 30 & 1u ? 0 : npc) + t, second = bc + (w0 >> 30 & 1u ? npc : 0) + t;   // slots
+            sm[first] = tail_children<T, D>(r, f & 0xFFFFu, s1, s2);
+            if (w0 >> 31) sm[second] = tail_children<T, D>(r + (f & 512u ? 2 : 1), f >> 16, s1, s2);
+        }
+        __syncthreads();
+    };
+    // level 0's right-hand side; x = 0 everywhere, and the right-hand sides of no cell
+    {
+        const int np = keep(a.np[0]), bo = keep(a.bo[0]);
+        const unsigned* id = w + keep(a.io[0]);
+        const T* b = keep(a.b);
+        for (int t = tid; t < np; t += TAIL_THREADS) {
+            const PairCells pc(id[t], 0u);
+            const T r = pc.red ? b[pc.red] : T(0), k = pc.black ? b[pc.black] : T(0);
+            sm[bo + t] = r;
+            sm[bo + np + t] = k;
+        }
+    }
+    for (int k = 0; k <= last; ++k) {
+        const int n = keep(int(a.g[k].N)), xo = keep(a.xo[k]);
+        for (int q = tid; q < n; q += TAIL_THREADS) sm[xo + q] = T(0);
     }
     {
+        const int np = keep(a.np[last]), bo = keep(a.bo[last]);
+        if (last > 0)
+            for (int t = tid; t < 2 * np; t += TAIL_THREADS) sm[bo + t] = T(0);
+    }
+    __syncthreads();
+    for (int l = 0; l < last; ++l) visit(l, 2 * keep(a.nu1[l]), 0, a.omega, 0);
+    {
         const Grid& g = a.g[last];
-        T* b = sm + a.off[last] + g.N;
-        // FP64 sum by one warp (ghost entries are zero): an FP64 instruction occupies the pipe for 16 cycles
+        const int np = keep(a.np[last]), bo = keep(a.bo[last]);
+        const unsigned* id = w + keep(a.io[last]);
+        // FP64 sum by one warp (the slots of no cell are zero): an FP64 instruction occupies the pipe for 16 cycles
         // a warp, whatever its lanes do
         if (tid < 32) {
             double acc = 0.0;
-            for (int q = tid; q < int(g.N); q += 32) acc += double(b[q]);
+            for (int q = tid; q < 2 * np; q += 32) acc += double(sm[bo + q]);
             for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             if (tid == 0) mean_s = T(acc / double((g.n[0] - 2) * (g.n[1] - 2) * (D == 3 ? g.n[2] - 2 : 1)));
         }
         __syncthreads();
         const T mean = mean_s;
-        cells(g, [&](int, int, int, int I) { b[I] -= mean; });
+        for (int t = tid; t < np; t += TAIL_THREADS) {
+            const PairCells pc(id[t], 0u);
+            if (pc.red) sm[bo + t] -= mean;
+            if (pc.black) sm[bo + np + t] -= mean;
+        }
         __syncthreads();
         // R B, B R, R B, ...: a colour following itself changes nothing
-        sweeps(last, a.nuc + 1, 0, T(1), false);
+        visit(last, keep(a.nuc) + 1, 0, T(1), 2);
     }
-    for (int l = last - 1; l >= 0; --l) sweeps(l, 2 * a.nu2[l], 1, a.omega, true);
-    for (int q = tid; q < N0; q += TAIL_THREADS) a.x[q] = sm[q];   // the ghost entries stay zero
+    for (int l = last - 1; l >= 0; --l) visit(l, 2 * keep(a.nu2[l]), 1, a.omega, 1);
+    // the result (its ghost entries stay zero)
+    {
+        const int np = keep(a.np[0]), xo = keep(a.xo[0]);
+        const unsigned* id = w + keep(a.io[0]);
+        T* x = keep(a.x);
+        for (int t = tid; t < np; t += TAIL_THREADS) {
+            const int I = id[t] & 0x3FFFFFFFu;
+            x[I] = sm[xo + I];
+            if (id[t] >> 31) x[I + 1] = sm[xo + I + 1];
+        }
+    }
+}
+template <class T, int D>
+__global__ void __launch_bounds__(TAIL_THREADS) mg_tail_k(const __grid_constant__ TailArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char tail_raw[];
+    __shared__ T mean_s;
+    T* sm = reinterpret_cast<T*>(tail_raw);
+    tail_setup<T, D>(a, sm);
+    __syncthreads();
+    tail_cycle<T, D>(a, sm, mean_s);
 }
 
 // Pairs of cells in the largest level that the one-block kernel takes.  FP32: TAIL_PAIRS for each thread (16^3
 // cells).  FP64: 256, since a multiprocessor issues FP64 at 1/64 of the FP32 rate and a half-sweep on more cells is
 // faster spread over the device.
 template <class T> constexpr long long tail_pairs() { return sizeof(T) == 4 ? TAIL_PAIRS * TAIL_THREADS : 256; }
+
+// ---- the one-launch solver of small grids (poisson_cluster.cuh)
+// Interior cells up to which it is used, and pairs of cells of its tail's largest level.  Measured on GB300, a step
+// with the multi-launch solver and on this path: FP32 (mixed) 41x35x30 4.3 and 2.8 ms, 32x64x32 4.9 and 4.2 ms; FP64
+// 128x64 2.4 and 2.6 ms (16 multiprocessors have a tenth of the device's FP64 pipes), 64x64 the same.
+template <class T> constexpr long long cluster_cells() { return sizeof(T) == 4 ? 65536 : 4096; }
+template <class T> constexpr long long cluster_tail_pairs() { return sizeof(T) == 4 ? 512 : 128; }
 
 // ------------------------------------------------------------------ Krylov kernels
 // Row loops: a block takes whole x-rows of interior cells (rows dealt round-robin over a
@@ -1456,10 +1651,11 @@ __global__ void __launch_bounds__(256) add_correction_k(Grid g, const float* __r
     }
 }
 
-// periodic ghosts of a scalar (WaterLily perBC!), one thread per cell of the boundary planes
-__global__ void perbc_k(Grid g, double* a) {
+// periodic ghost of a scalar (WaterLily perBC!) at number t of the boundary planes' cells; reads only positions that
+// no thread writes: the mapped position has no periodic ghost coordinate left
+__device__ __forceinline__ void perbc_cell(const Grid& g, double* a, long long t) {
     int c[3];
-    if (!bc_plane_cell(g, blockIdx.x * (long long)blockDim.x + threadIdx.x, c)) return;
+    if (!bc_plane_cell(g, t, c)) return;
     const int x = c[0], y = c[1], z = c[2];
     bool any = false;
     for (int e = 0; e < g.D; ++e)
@@ -1467,13 +1663,15 @@ __global__ void perbc_k(Grid g, double* a) {
             c[e] = bc_src(g, e, c[e]);
             any = true;
         }
-    if (!any) return;
-    // only read positions that no thread writes: the mapped position must have
-    // no periodic ghost coordinate left (it has none after mapping)
-    a[lin(g, x, y, z)] = a[lin3(g, c)];
+    if (any) a[lin(g, x, y, z)] = a[lin3(g, c)];
 }
+// one thread per cell of the boundary planes
+__global__ void perbc_k(Grid g, double* a) { perbc_cell(g, a, blockIdx.x * (long long)blockDim.x + threadIdx.x); }
 
 }  // namespace
+}  // namespace ia
+#include "poisson_cluster.cuh"
+namespace ia {
 
 // ------------------------------------------------------------------ host side
 
@@ -1512,39 +1710,49 @@ static void tb_launch(const PoissonMG* mg, const TbArgs& a, int S, cudaStream_t 
     ia::note_launch();
 }
 
-// shared values of the one-block V-cycle from level l on: x and b of each level
-static long long tail_values(const PoissonMG* mg, int l) {
-    long long n = 0;
-    for (; l < mg->nlev; ++l) n += 2 * mg->lev[l].g.N;
-    return n;
+constexpr int TAIL_BYTES = 200 * 1024;   // shared memory of the one-block V-cycle
+// shared-memory layout of the one-block V-cycle from level l0 on
+template <class T>
+static TailArgs<T> tail_layout(const PoissonMG* mg, int l0) {
+    TailArgs<T> a;
+    a.nl = mg->nlev - l0;
+    int v = 0, w = 0;
+    for (int k = 0; k < a.nl && k < TAIL_MAX; ++k) {
+        const Grid& g = mg->lev[l0 + k].g;
+        const int np = (g.n[0] - 1) / 2 * (g.n[1] - 2) * (g.D == 3 ? g.n[2] - 2 : 1);
+        a.g[k] = g;
+        a.np[k] = np;
+        a.xo[k] = v;
+        a.bo[k] = v += int(g.N);
+        a.co[k] = v += 2 * np;
+        v += (2 * g.D + 1) * 2 * np;
+        a.io[k] = w;
+        w += TAIL_WORDS * np;
+    }
+    a.ro = v;
+    a.values = v + int(a.g[0].N);
+    a.words = w;
+    return a;
 }
-constexpr long long TAIL_BYTES = 160 * 1024;   // the rest of the 228 KB caches the coefficients in L1
 // first level of the one-block V-cycle; the coarsest level (at most 512 cells) always fits
 template <class T>
-static int tail_level(const PoissonMG* mg) {
+static int tail_level(const PoissonMG* mg, long long most = tail_pairs<T>()) {
     int l = mg->nlev - 1;
     while (l > 0 && mg->nlev - l < TAIL_MAX) {
         const Grid& g = mg->lev[l - 1].g;
         const long long pairs = (long long)((g.n[0] - 1) / 2) * (g.n[1] - 2) * (g.D == 3 ? g.n[2] - 2 : 1);
-        if (pairs > tail_pairs<T>() || tail_values(mg, l - 1) * (long long)sizeof(T) > TAIL_BYTES) break;
+        if (pairs > most || mg->lev[l].g.N > 0xFFFF || tail_layout<T>(mg, l - 1).bytes() > (size_t)TAIL_BYTES) break;
         --l;
     }
     return l;
 }
 template <class T>
 static TailArgs<T> tail_args(PoissonMG* mg, int l0, int nu1, int nu2, int nuc) {
-    TailArgs<T> a;
-    a.nl = mg->nlev - l0;
-    a.total = 0;
+    TailArgs<T> a = tail_layout<T>(mg, l0);
     for (int k = 0; k < a.nl; ++k) {
         MGLevel& L = mg->lev[l0 + k];
-        a.g[k] = L.g;
         a.L[k] = L.template L_<T>();
         a.iD[k] = L.template iD_<T>();
-        a.diag[k] = nullptr;
-        if constexpr (sizeof(T) == 8) a.diag[k] = L.r;
-        a.off[k] = a.total;
-        a.total += 2 * int(L.g.N);
         a.nu1[k] = (l0 + k == 0 && mg->nu1f > 0) ? mg->nu1f : nu1;
         a.nu2[k] = (l0 + k == 0 && mg->nu2f > 0) ? mg->nu2f : nu2;
     }
@@ -1564,7 +1772,7 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     const T* iD = L.template iD_<T>();
     if (l >= tail_level<T>(mg)) {
         const TailArgs<T> a = tail_args<T>(mg, l, nu1, nu2, nuc);
-        const size_t bytes = sizeof(T) * (size_t)a.total;
+        const size_t bytes = a.bytes();
         if (L.g.D == 3) mg_tail_k<T, 3><<<1, TAIL_THREADS, bytes, st>>>(a);
         else mg_tail_k<T, 2><<<1, TAIL_THREADS, bytes, st>>>(a);
         ia::note_launch();
@@ -1849,6 +2057,7 @@ int mg_create(ia_handle* h) {
             e = e ? e : cudaMalloc(&L.r, 8 * n);
             e = e ? e : cudaMalloc(&L.L, 8 * n * g0.D);
             e = e ? e : cudaMalloc(&L.iD, 8 * n);
+            if ((long long)mg->lev[0].g.N <= 2 * cluster_cells<float>()) e = e ? e : cudaMalloc(&L.t, 8 * n);
             if (!e) {
                 cudaMemset(L.x, 0, 8 * n);
                 cudaMemset(L.b, 0, 8 * n);
@@ -1912,10 +2121,10 @@ int mg_create(ia_handle* h) {
         if (!coarser) break;
     }
     mg->nlev = nl;
-    if (cudaFuncSetAttribute(mg_tail_k<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess ||
-        cudaFuncSetAttribute(mg_tail_k<float, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess ||
-        cudaFuncSetAttribute(mg_tail_k<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess ||
-        cudaFuncSetAttribute(mg_tail_k<double, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_BYTES)) != cudaSuccess)
+    if (cudaFuncSetAttribute(mg_tail_k<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES) != cudaSuccess ||
+        cudaFuncSetAttribute(mg_tail_k<float, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES) != cudaSuccess ||
+        cudaFuncSetAttribute(mg_tail_k<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES) != cudaSuccess ||
+        cudaFuncSetAttribute(mg_tail_k<double, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES) != cudaSuccess)
         return IA_ERR_CUDA;
     const size_t N = (size_t)g0.N;
     cudaError_t e = cudaSuccess;
@@ -1979,7 +2188,7 @@ void mg_destroy(ia_handle* h) {
     if (!mg) return;
     for (int l = 0; l < MG_MAX_LEVELS; ++l) {
         MGLevel& L = mg->lev[l];
-        cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.L); cudaFree(L.iD);
+        cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.L); cudaFree(L.iD); cudaFree(L.t);
         cudaFree(L.x32); cudaFree(L.b32); cudaFree(L.r32); cudaFree(L.L32); cudaFree(L.iD32); cudaFree(L.L16);
         cudaFree(L.ratio);
     }
@@ -2163,6 +2372,135 @@ static int poisson_solve_mixed(ia_handle* h, double* xv, const double* zz, const
     return (res <= tol) ? IA_OK : IA_WARN_NOT_CONVERGED;
 }
 
+// ---- the one-launch solver of small grids (poisson_cluster.cuh)
+// Two-dimensional grids with an odd extent and a long side are solved on one level, by the coarsest level's sweeps, as
+// they always were: these stop at the same residual as the multigrid with 10 to 20 times its error, on 161 x 97 cells
+// up to 5e-9 of the pressure, and results are to stay within 1e-9 of what they were.  (On sides of up to 96 cells, and
+// on the even and the three-dimensional grids that fit this path, the two are below 5e-10 apart, and the multigrid
+// runs.)  161 x 97, mixed, a step: 249 ms with one block sweeping, 13.5 ms here, 1.9 ms with the multigrid.
+static bool one_level(const Grid& g) {
+    return ((g.n[0] & 1) || (g.n[1] & 1)) && std::max(g.n[0], g.n[1]) - 2 > 96;
+}
+
+template <class T, int D>
+static int cluster_blocks(PoissonMG* mg, long long pairs) {
+    int& most = mg->cluster;   // the largest cluster that the device can place; -1: not asked yet
+    if (most < 0) {
+        int got = 0;
+        const auto k = solve_cluster_k<T, D>;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES) == cudaSuccess &&
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+            for (int c = CL_MAX; c >= 1 && !got; c /= 2) {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute at = {};
+                at.id = cudaLaunchAttributeClusterDimension;
+                at.val.clusterDim.x = c;
+                at.val.clusterDim.y = at.val.clusterDim.z = 1;
+                cfg.gridDim = dim3(c);
+                cfg.blockDim = dim3(TAIL_THREADS);
+                cfg.dynamicSmemBytes = TAIL_BYTES;
+                cfg.attrs = &at;
+                cfg.numAttrs = 1;
+                int n = 0;
+                if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= 1) got = c;
+            }
+        cudaGetLastError();
+        most = got;
+    }
+    return most >= 1 && pairs <= (long long)CL_PAIRS * most * TAIL_THREADS ? most : 0;
+}
+
+// Solves on the cluster path when it applies: *done says whether it did.
+template <class T, int D>
+static cudaError_t cluster_solve(ia_handle* h, double* xv, const double* zz, const double* L, double tol, int itmx,
+                                 int* iters, double* resid, bool* done) {
+    PoissonMG* mg = h->mg;
+    const Grid& g = h->g;
+    *done = false;
+    const long long cells = (long long)(g.n[0] - 2) * (g.n[1] - 2) * (D == 3 ? g.n[2] - 2 : 1);
+    // (relaxation factor 1, at which the half-sweeps and the blocked smoother do the same arithmetic, stays on the
+    // kernels that share it)
+    if (h->timing.on || mg->smoother != IA_SMOOTHER_HALFSWEEP || mg->omega == 1.0 ||
+        cells > (D == 2 && one_level(g) ? cluster_cells<float>() : cluster_cells<T>()) ||
+        (sizeof(T) == 8 && !mg->lev[0].t))
+        return cudaSuccess;
+    const bool flat = D == 2 && one_level(g);
+    const int lt = flat ? 0 : tail_level<T>(mg, cluster_tail_pairs<T>());
+    const long long pairs = (long long)((g.n[0] - 1) / 2) * (g.n[1] - 2) * (D == 3 ? g.n[2] - 2 : 1);
+    const int C = cluster_blocks<T, D>(mg, pairs);
+    // (on one level the tail, which then has the coarsest level alone, is not used)
+    const int l0 = flat ? mg->nlev - 1 : lt;
+    if (!C || lt > CL_LEVELS || (mg->nlev > 1 && mg->lev[1].g.N > 0xFFFF) ||
+        tail_layout<T>(mg, l0).bytes() + cl_words_bytes(lt) > (size_t)TAIL_BYTES)
+        return cudaSuccess;
+    *done = true;
+    SolveArgs<T> a;
+    a.tail = tail_args<T>(mg, l0, mg->nu1, mg->nu2, mg->nuc);
+    a.nd = lt;
+    a.flat = flat ? 1 : 0;
+    for (int l = 0; l <= lt; ++l) {
+        MGLevel& V = mg->lev[l];
+        a.g[l] = V.g;
+        a.x[l] = V.template x_<T>();
+        a.b[l] = V.template b_<T>();
+        a.L[l] = V.template L_<T>();
+        a.iD[l] = V.template iD_<T>();
+        if (l == lt) break;
+        if constexpr (sizeof(T) == 8) a.r[l] = V.t;
+        else a.r[l] = V.r32;
+        a.nu1[l] = (l == 0 && mg->nu1f > 0) ? mg->nu1f : mg->nu1;
+        a.nu2[l] = (l == 0 && mg->nu2f > 0) ? mg->nu2f : mg->nu2;
+    }
+    a.omega = T(mg->omega);
+    if constexpr (sizeof(T) == 4) {
+        a.p = mg->p32;
+        a.q = mg->q32;
+        a.e = mg->e32;
+        a.L0 = mg->lev[0].L32;
+    } else {
+        a.p = mg->p;
+        a.q = mg->q;
+        a.e = nullptr;
+        a.L0 = L;
+    }
+    a.xs = xv;
+    a.z = zz;
+    a.L64 = L;
+    a.diag64 = mg->diag64;
+    a.tol = tol;
+    a.inner_rtol = mg->inner_rtol;
+    a.itmx = itmx;
+    a.inner_max = mg->inner_max;
+    a.partial = mg->partial;
+    a.out = reinterpret_cast<SolveOut*>(mg->dsc);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(TAIL_THREADS);
+    cfg.dynamicSmemBytes = a.tail.bytes() + cl_words_bytes(lt);
+    cfg.stream = h->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, solve_cluster_k<T, D>, a);
+    ia::note_launch();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(mg->hsc, a.out, sizeof(SolveOut), cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return e;
+    SolveOut o;
+    std::memcpy(&o, mg->hsc, sizeof(o));
+    mg->stats[1] += o.vcycles;
+    if (sizeof(T) == 4) {
+        mg->stats[3] += o.total;
+        mg->stats[4] += o.outer;
+    }
+    *iters = o.total;
+    *resid = o.res;
+    return cudaSuccess;
+}
+
 // r = z - A x over interior cells; L∞(r) to the host
 int poisson_residual(ia_handle* h, double* r, const double* x, const double* z, const double* L, double* linf) {
     cudaStream_t st = h->stream;
@@ -2181,13 +2519,25 @@ int poisson_solve(ia_handle* h, double* xv, const double* zz, const double* L, d
                   double* resid) {
     PoissonMG* mg = h->mg;
     if (!mg) return IA_ERR_INVALID;
-    if (h->cfg.poisson_mode != IA_POISSON_FP64) {
+    if (h->cfg.poisson_mode != IA_POISSON_LEARNED) {
         if (mg_setup(h, L) != cudaSuccess) return IA_ERR_CUDA;
+        bool done = false;
+        cudaError_t e;
+        if (h->cfg.poisson_mode == IA_POISSON_FP64)
+            e = h->g.D == 3 ? cluster_solve<double, 3>(h, xv, zz, L, tol, itmx, iters, resid, &done)
+                            : cluster_solve<double, 2>(h, xv, zz, L, tol, itmx, iters, resid, &done);
+        else
+            e = h->g.D == 3 ? cluster_solve<float, 3>(h, xv, zz, L, tol, itmx, iters, resid, &done)
+                            : cluster_solve<float, 2>(h, xv, zz, L, tol, itmx, iters, resid, &done);
+        if (e != cudaSuccess) return IA_ERR_CUDA;
+        if (done) return (*resid <= tol) ? IA_OK : IA_WARN_NOT_CONVERGED;
+    }
+    if (h->cfg.poisson_mode != IA_POISSON_FP64) {
+        if (h->cfg.poisson_mode == IA_POISSON_LEARNED && mg_setup(h, L) != cudaSuccess) return IA_ERR_CUDA;
         return poisson_solve_mixed(h, xv, zz, L, tol, itmx, iters, resid);
     }
     cudaStream_t st = h->stream;
     const Grid& g = h->g;
-    if (mg_setup(h, L) != cudaSuccess) return IA_ERR_CUDA;
     unsigned long long* dlinf = reinterpret_cast<unsigned long long*>(mg->dsc + 8);
     MGLevel& F = mg->lev[0];
     // the residual is the V-cycle's right-hand side and the preconditioned residual its result, in place

@@ -26,7 +26,8 @@ struct FcgDev {
 struct MGLevel {
     Grid g;
     // FP64 operator and vectors (IA_POISSON_FP64)
-    double *x = nullptr, *b = nullptr, *r = nullptr, *L = nullptr, *iD = nullptr;
+    double *x = nullptr, *b = nullptr, *r = nullptr, *L = nullptr, *iD = nullptr;   // r: the diagonal
+    double* t = nullptr;   // residual scratch of the one-launch solver
     // FP32 operator and vectors (IA_POISSON_MIXED)
     float *x32 = nullptr, *b32 = nullptr, *r32 = nullptr, *L32 = nullptr, *iD32 = nullptr;
     // finest level of the mixed V-cycle: FP16 copy of L32 for the smoother and the residual restriction
@@ -78,6 +79,7 @@ struct PoissonMG {
     int coef16 = 0;                                                   // finest-level smoother on L16 (mixed)
     int slab_rows = 0;                                                // finest-level wavefront slab (rows; 0 off)
     int nsm = 0;                                                      // multiprocessors of the device
+    int cluster = -1;                                                 // blocks of the one-launch solver's cluster
     // each precision's finest-level V-cycle is captured once into a CUDA graph (its launch
     // sequence and arguments are fixed for the handle) and replayed; recaptured when the
     // smoothing parameters change
