@@ -11,6 +11,22 @@
 namespace ia {
 
 // ------------------------------------------------------------------ PLIC
+//
+// These routines run on the few interface cells, FP64 throughout, and are bound by their FP64 instructions (16 cycles
+// of the pipe for a warp) and, on small grids, by the length of their chains.  A division costs about 20 of them, so
+// quotients with a common or constant divisor are formed from its reciprocal and one correction step, and the two
+// cubics of the plane constant are one.  Faces of a sphere in 256^3 cells, one sweep: 56 us with every division and two
+// cubics, 44 us so.
+
+// x / y from r = 1/y (correctly rounded): Markstein's final step, the quotient that the division gives; the division
+// itself where r is near the ends of the range (a velocity or a difference of fractions below 1e-290)
+__device__ __forceinline__ double quot(double x, double y, double r) {
+    const int e = __double2hiint(r) & 0x7FF00000;
+    if (e < (64 << 20) || e > ((2047 - 64) << 20)) return x / y;
+    const double q = x * r;
+    return fma(fma(-y, q, x), r, q);
+}
+__device__ __forceinline__ double third(double x) { return quot(x, 3.0, 1.0 / 3.0); }
 
 // Sorted, |n|-normalised magnitudes m1 <= m2 (<= m3) of a normal.
 __device__ __forceinline__ void plic_sort(double& a, double& b) {
@@ -42,18 +58,19 @@ __device__ inline double plic_volume(double m1, double m2, double m3, double a) 
     return (2.0 * a - m12) / (2.0 * m3);
 }
 
-// Real root of c3 x^3 + c2 x^2 + c1 x + c0 selected by the trigonometric
-// form used in src/PLIC.jl:165-176.
+// Real root of c3 x^3 + c2 x^2 + c1 x + c0, c3 = -1 or -2, selected by the
+// trigonometric form used in src/PLIC.jl:165-176.
 __device__ inline double plic_cubic_root(double c0, double c1, double c2, double c3) {
-    const double a0 = c0 / c3, a1 = c1 / c3, a2 = c2 / c3;
-    const double p0 = a1 / 3.0 - a2 * a2 / 9.0;
-    const double q0 = (a1 * a2 - 3.0 * a0) / 6.0 - a2 * a2 * a2 / 27.0;
+    const double ic3 = c3 == -1.0 ? -1.0 : -0.5;   // c3 is -1 or -2: exact
+    const double a0 = c0 * ic3, a1 = c1 * ic3, a2 = c2 * ic3;
+    const double p0 = third(a1) - quot(a2 * a2, 9.0, 1.0 / 9.0);
+    const double q0 = quot(a1 * a2 - 3.0 * a0, 6.0, 1.0 / 6.0) - quot(a2 * a2 * a2, 27.0, 1.0 / 27.0);
     double a = q0 / sqrt(-p0 * p0 * p0);
     a = (a * a <= 1.0) ? a : 0.0;
-    const double t = acos(a) / 3.0;
+    const double t = third(acos(a));
     double st, ct;
     sincos(t, &st, &ct);
-    return sqrt(-p0) * (sqrt(3.0) * st - ct) - a2 / 3.0;
+    return sqrt(-p0) * (1.7320508075688772 * st - ct) - third(a2);
 }
 
 // Plane constant for volume v <= 1/2 (src/PLIC.jl:117-149).
@@ -63,19 +80,20 @@ __device__ __forceinline__ double plic_intercept(double m1, double m2, double v)
 __device__ inline double plic_intercept(double m1, double m2, double m3, double v) {
     const double m12 = m1 + m2;
     const double p = 6.0 * m1 * m2 * m3;
-    const double v1 = ((m2 == 0.0) ? 1.0 : m1 / m2) * m1 / (6.0 * m3);
-    const double v2 = v1 + (m2 - m1) / (2.0 * m3);
-    const double v3 = (m3 < m12)
-                          ? (m3 * m3 * (3.0 * m12 - m3) + m1 * m1 * (m1 - 3.0 * m3) + m2 * m2 * (m2 - 3.0 * m3)) / p
-                          : m12 / (2.0 * m3);
+    const double r3 = 1.0 / m3;
+    const double v1 = quot(((m2 == 0.0) ? 1.0 : m1 / m2) * m1, 6.0 * m3, (1.0 / 6.0) * r3);
+    const double v2 = v1 + quot(m2 - m1, 2.0 * m3, 0.5 * r3);
+    const double s2 = m1 * m1 + m2 * m2, s3 = m1 * m1 * m1 + m2 * m2 * m2;
+    const bool low = m3 < m12;
+    const double v3 = low ? (m3 * m3 * (3.0 * m12 - m3) + m1 * m1 * (m1 - 3.0 * m3) + m2 * m2 * (m2 - 3.0 * m3)) / p
+                          : quot(m12, 2.0 * m3, 0.5 * r3);
     if (v < v1) return cbrt(p * v);
     if (v < v2) return 0.5 * (m1 + sqrt(m1 * m1 + 8.0 * m2 * m3 * (v - v1)));
-    if (v < v3)
-        return plic_cubic_root(m1 * m1 * m1 + m2 * m2 * m2 - p * v, -3.0 * (m1 * m1 + m2 * m2), 3.0 * m12, -1.0);
-    if (m3 < m12)
-        return plic_cubic_root(m1 * m1 * m1 + m2 * m2 * m2 + m3 * m3 * m3 - p * v,
-                               -3.0 * (m1 * m1 + m2 * m2 + m3 * m3), 3.0, -2.0);
-    return m3 * v + 0.5 * m12;
+    const bool mid = v < v3;
+    if (!mid && !low) return m3 * v + 0.5 * m12;
+    // one evaluation for both cubics: lanes of a warp meet either
+    const double c0 = (mid ? s3 : s3 + m3 * m3 * m3) - p * v, c1 = -3.0 * (mid ? s2 : s2 + m3 * m3);
+    return plic_cubic_root(c0, c1, mid ? 3.0 * m12 : 3.0, mid ? -1.0 : -2.0);
 }
 
 // getIntercept (src/PLIC.jl:20-39): α of the cell with normal n and fraction g.
@@ -86,12 +104,13 @@ __device__ double get_intercept(const double n[3], double g) {
     double a = 0.5;
     const double v = g < 0.5 ? g : 1.0 - g;
     if (g != 0.5) {
-        double m1 = fabs(n[0]) / t, m2 = fabs(n[1]) / t;
+        const double r = 1.0 / t;
+        double m1 = quot(fabs(n[0]), t, r), m2 = quot(fabs(n[1]), t, r);
         if (D == 2) {
             plic_sort(m1, m2);
             a = plic_intercept(m1, m2, v);
         } else {
-            double m3 = fabs(n[2]) / t;
+            double m3 = quot(fabs(n[2]), t, r);
             plic_sort(m1, m2, m3);
             a = plic_intercept(m1, m2, m3, v);
         }
@@ -113,16 +132,17 @@ __device__ double get_volume_fraction(const double n[3], double b) {
     // (b - min(n1,0) - min(n2,0) - ...) evaluated left to right
     double a = b - fmin(n[0], 0.0) - fmin(n[1], 0.0);
     if (D == 3) a -= fmin(n[2], 0.0);
-    a /= t;
+    const double r = 1.0 / t;
+    a = quot(a, t, r);
     (void)shift;
     if (a <= 0.0 || a == 0.5 || a >= 1.0) return fmin(fmax(a, 0.0), 1.0);
     const double w = a < 0.5 ? a : 1.0 - a;
-    double m1 = fabs(n[0]) / t, m2 = fabs(n[1]) / t, v;
+    double m1 = quot(fabs(n[0]), t, r), m2 = quot(fabs(n[1]), t, r), v;
     if (D == 2) {
         plic_sort(m1, m2);
         v = plic_volume(m1, m2, w);
     } else {
-        double m3 = fabs(n[2]) / t;
+        double m3 = quot(fabs(n[2]), t, r);
         plic_sort(m1, m2, m3);
         v = plic_volume(m1, m2, m3, w);
     }
@@ -196,8 +216,9 @@ __device__ void normal_wh(const Stencil& S, double n[3]) {
     const long long dstep = signbit(n[ad]) ? -S.s[ad] : S.s[ad];
     double an = fabs(n[ad]);
     an = (an == 0.0) ? 1.0 : an;
+    const double ran = 1.0 / an;
 #pragma unroll
-    for (int d = 0; d < D; ++d) n[d] /= an;
+    for (int d = 0; d < D; ++d) n[d] = quot(n[d], an, ran);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
         if (d == ad) continue;
