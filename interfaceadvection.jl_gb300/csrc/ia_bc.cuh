@@ -109,7 +109,7 @@ __device__ __forceinline__ long long okey(double v) {
 __device__ __forceinline__ double dmin(double a, double b) { return okey(b) < okey(a) ? b : a; }
 __device__ __forceinline__ double dmax(double a, double b) { return okey(a) < okey(b) ? b : a; }
 __device__ __forceinline__ bool dlt(double a, double b) { return okey(a) < okey(b); }
-__device__ __forceinline__ double dabs(double v) { return __longlong_as_double(__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFll); }
+__device__ __forceinline__ double dabs(double v) { return __longlong_as_double((long long)abs_bits(v)); }
 
 // Density at the lower d-face from two cell fractions: λρ + (1-λρ)(fa+fb)/2
 // (getρ(d,I,f,λρ), src/VOFutil.jl:176).  Full/empty pairs skip the FP64 work.

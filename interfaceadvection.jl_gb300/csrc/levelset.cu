@@ -25,12 +25,11 @@ namespace {
 
 inline dim3 blk() { return dim3(32, 8, 1); }
 
-constexpr long long kInfBits = 0x7FF0000000000000ll;
-__device__ __forceinline__ long long abs_bits(double v) { return __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFll; }
+constexpr unsigned long long kInfBits = 0x7FF0000000000000ull;
 
 // |a| <= |b| ? a : b (b when either is NaN)
 __device__ __forceinline__ double minmod(double a, double b) {
-    const long long ka = abs_bits(a), kb = abs_bits(b);
+    const unsigned long long ka = abs_bits(a), kb = abs_bits(b);
     return ka <= kb && kb <= kInfBits ? a : b;
 }
 
@@ -45,7 +44,7 @@ __device__ __forceinline__ double upwind(double a, double b, double c, double d,
     const double dR = fma(-0.5, minmod(m3, m2), d - c), dL = fma(0.5, minmod(m2, m1), c - b);
     const double wR = __longlong_as_double(__double_as_longlong(dR) ^ flip);
     const double wL = __longlong_as_double(__double_as_longlong(dL) ^ flip);
-    const long long kR = okey(wR), kN = okey(__longlong_as_double(__double_as_longlong(wL) ^ (1ll << 63)));
+    const long long kR = okey(wR), kN = ~okey(wL);   // ~: the key of -wL
     const bool num = abs_bits(dR) <= kInfBits && abs_bits(dL) <= kInfBits;
     const bool r_neg = __double_as_longlong(wR) < 0 && abs_bits(dR) != 0, l_pos = __double_as_longlong(wL) > 0;
     return num && r_neg && kR < kN ? dR : (num && l_pos && kR > kN ? dL : 0.0);
@@ -56,7 +55,7 @@ template <int D>
 __device__ __forceinline__ double rhs_cell(const Grid& g, const double* __restrict__ phi, double ini, int I, const int c[3]) {
     const double cc = phi[I];
     const long long kc = __double_as_longlong(cc), ki = __double_as_longlong(ini);
-    if ((ki & 0x7FFFFFFFFFFFFFFFll) == 0 || abs_bits(ini) > kInfBits) {   // sign 0 (or NaN): no gradient
+    if (abs_bits(ini) == 0 || abs_bits(ini) > kInfBits) {   // sign 0 (or NaN): no gradient
         return ini * 1.0;
     }
     const long long flip = ki & (1ll << 63);
@@ -68,7 +67,7 @@ __device__ __forceinline__ double rhs_cell(const Grid& g, const double* __restri
         const int oa = ci != 1 ? -2 : (g.isper(i) ? n - 3 - ci : -1), oe = ci != n - 2 ? 2 : (g.isper(i) ? 2 - ci : 1);
         const double a = phi[I + oa * si], b = phi[I - si], d = phi[I + si], e = phi[I + oe * si];
         const bool flat = __double_as_longlong(a) == kc && __double_as_longlong(b) == kc && __double_as_longlong(d) == kc &&
-                          __double_as_longlong(e) == kc && (kc & 0x7FFFFFFFFFFFFFFFll) < kInfBits;
+                          __double_as_longlong(e) == kc && abs_bits(cc) < kInfBits;
         if (!flat) {
             const double u = upwind(a, b, cc, d, e, flip);
             acc = fma(u, u, acc);

@@ -1094,10 +1094,6 @@ __device__ __forceinline__ unsigned long long block_max(unsigned long long m) {
     return m;
 }
 
-__device__ __forceinline__ unsigned long long abs_bits(double v) {
-    return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
-}
-
 // diagonal D_I = -Σ_i (L[I,i] + L[I+δi,i]) of the FP64 operator
 __device__ __forceinline__ double diag_of(const Grid& g, const double* L, long long I) {
     double dd = 0.0;
