@@ -97,7 +97,7 @@ int translate_fill_status(const Grid& g, const DevStatus& s, const double* u1, c
 
 // One advect! (src/advection.jl:17-78) or one advectVOF1d! sweep sequence.
 int vof_sweep(ia_handle* h, const double* fin, double* fout, const double* u1, const double* u2, double dt, int d,
-              bool first, int8_t* cbar, double* rhouf, double tol_rep, int counter, float2* dila) {
+              bool first, int8_t* cbar, double* rhouf, double tol_rep, int counter, float2* dila, bool scanned) {
     const Grid& g = h->g;
     {
         const int k = 0, counter_base = counter;
@@ -128,6 +128,12 @@ int vof_sweep(ia_handle* h, const double* fin, double* fout, const double* u1, c
         a.flux = h->flux;
         a.vals = h->tmp1;
         a.st = h->dst;
+        if (scanned) {
+            a.tiles = h->tiles;
+            a.tile_count = &h->dst->list_count[30];
+            a.above = &h->dst->list_count[31];
+            a.tile_blocks = h->list_blocks;
+        }
         if (dila) {
             const ff rql = ff_split(0.25 * h->cfg.lrho), rq1 = ff_split(0.25 * (h->cfg.lrho + (1.0 - h->cfg.lrho)));
             a.dila = dila;
@@ -156,9 +162,31 @@ int vof_sweep(ia_handle* h, const double* fin, double* fout, const double* u1, c
 int advect_sweeps(ia_handle* h, double* f, const double* u1, const double* u2, double dt, const int* dirs,
                   int nsweeps, int8_t* cbar, double* rhouf, double tol_rep, bool first_writes_cbar,
                   int counter_base) {
+    // large 3D grids: one pass over the tiles of one fluid instead of one in every sweep (each dimension is swept once)
+    const bool scan = h->tiles && first_writes_cbar && nsweeps == 3 && dt > 0.0 && std::isfinite(dt);
+    if (scan) {
+        ScanArgs a;
+        a.g = h->g;
+        a.f = f;
+        a.u1 = u1;
+        a.u2 = u2;
+        a.cbar = cbar;
+        a.rhouf = rhouf;
+        a.h = dt / 2.0;
+        a.hl = (dt / 2.0) * h->cfg.lrho;
+        const double lim = 0.5 / dt;
+        std::memcpy(&a.ulim, &lim, 8);
+        a.tiles = h->tiles;
+        a.count = &h->dst->list_count[30];
+        a.above = &h->dst->list_count[31];
+        const int tk = timing_begin(h, TK_VOF_BULK);
+        const cudaError_t e = vof_scan_call(a, h->stream);
+        timing_end(h, tk);
+        if (e != cudaSuccess) return IA_ERR_CUDA;
+    }
     for (int k = 0; k < nsweeps; ++k) {
         const int rc = vof_sweep(h, f, f, u1, u2, dt, dirs[k], first_writes_cbar && k == 0, cbar, rhouf, tol_rep,
-                                 counter_base + k);
+                                 counter_base + k, nullptr, scan);
         if (rc != IA_OK) return rc;
     }
     return IA_OK;
@@ -271,6 +299,7 @@ int ia_create(const ia_config* cfg, ia_handle** out) {
     e = e ? e : cudaMalloc(&h->list, sizeof(unsigned int) * (size_t)h->g.N);
     e = e ? e : cudaMalloc(&h->flist, sizeof(unsigned int) * (size_t)h->g.N);
     e = e ? e : cudaMalloc(&h->flux, nb);
+    if (h->g.D == 3 && h->g.N >= VOF_SCAN_CELLS) e = e ? e : cudaMalloc(&h->tiles, sizeof(unsigned int) * (size_t)vof_tiles(h->g));
     e = e ? e : cudaMalloc(&h->dst, sizeof(DevStatus));
     e = e ? e : cudaMalloc(&h->partial, sizeof(double) * 4096);
     e = e ? e : cudaMalloc(&h->dscalar, sizeof(double) * 64);
@@ -298,6 +327,7 @@ int ia_destroy(ia_handle* h) {
     cudaFree(h->list);
     cudaFree(h->flist);
     cudaFree(h->flux);
+    cudaFree(h->tiles);
     cudaFree(h->dst);
     cudaFree(h->partial);
     cudaFree(h->dscalar);

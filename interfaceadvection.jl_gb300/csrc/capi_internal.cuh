@@ -38,6 +38,7 @@ struct ia_handle {
     unsigned int* list = nullptr;      // compacted cells needing the full update
     unsigned int* flist = nullptr;     // compacted faces needing reconstruction
     double* flux = nullptr;            // cached fluxes of listed faces
+    unsigned int* tiles = nullptr;     // tiles of the grid that the sweeps of a call go through (large 3D grids)
     ia::DevStatus* dst = nullptr;      // device status
     ia::DevStatus* hst = nullptr;      // pinned host mirror
     double* partial = nullptr;         // reduction partials
@@ -60,9 +61,10 @@ int status_collect(ia_handle* h, const double* u1, const double* u2, ia_status* 
 // code (src/advection.jl:145-189).  Shared by every entry point that reports a fill status.
 int translate_fill_status(const Grid& g, const DevStatus& s, const double* u1, const double* u2, ia_status& st);
 // one VOF sweep along d, fin -> fout (fin == fout: in place); dila (coupled momentum step, float-float
-// arithmetic): receives the momentum update's dilation term of every cell as FP32 pairs
+// arithmetic): receives the momentum update's dilation term of every cell as FP32 pairs; scanned: after the call's
+// vof_scan_call, whose tiles (h->tiles) the bulk pass goes through
 int vof_sweep(ia_handle* h, const double* fin, double* fout, const double* u1, const double* u2, double dt, int d,
-              bool first, int8_t* cbar, double* rhouf, double tol_rep, int counter, float2* dila = nullptr);
+              bool first, int8_t* cbar, double* rhouf, double tol_rep, int counter, float2* dila = nullptr, bool scanned = false);
 int advect_sweeps(ia_handle* h, double* f, const double* u1, const double* u2, double dt, const int* dirs,
                   int nsweeps, int8_t* cbar, double* rhouf, double tol_rep, bool first_writes_cbar,
                   int counter_base);

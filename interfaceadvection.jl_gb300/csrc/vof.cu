@@ -38,12 +38,15 @@ namespace ia {
 namespace {
 
 constexpr unsigned long long ONE_BITS = 0x3FF0000000000000ull;   // 1.0
-constexpr unsigned long long ABS_MASK = 0x7FFFFFFFFFFFFFFFull;
 
 __device__ __forceinline__ unsigned long long bits(double v) { return (unsigned long long)__double_as_longlong(v); }
 // |v| <= limit, decided on the bit pattern (false for inf / NaN)
-__device__ __forceinline__ bool abs_le(unsigned long long b, unsigned long long lim_bits) {
-    return (b & ABS_MASK) <= lim_bits;
+__device__ __forceinline__ bool abs_le(double v, unsigned long long lim_bits) { return abs_bits(v) <= lim_bits; }
+__device__ __forceinline__ bool is_zero(double v) { return abs_bits(v) == 0ull; }
+// v < 1/2 (false for NaN)
+__device__ __forceinline__ bool below_half(double v) {
+    const unsigned long long b = bits(v);
+    return abs_bits(v) <= 0x7FF0000000000000ull && ((b >> 63) || b < 0x3FE0000000000000ull);
 }
 // f ∈ {+0, 1} exactly
 __device__ __forceinline__ bool is_bulk(unsigned long long b) { return b == 0ull || b == ONE_BITS; }
@@ -89,7 +92,7 @@ __device__ __forceinline__ bool face_simple(const SweepArgs& a, long long K, int
     const long long sd = a.g.s[a.d];
     dl = a.h * (a.u1[K] + a.u2[K]);
     const unsigned long long db = bits(dl);
-    if ((db & ABS_MASK) == 0ull) {   // δl == 0: no flux, ρuf untouched
+    if (is_zero(dl)) {   // δl == 0: no flux, ρuf untouched
         F = 0.0;
         return true;
     }
@@ -119,7 +122,7 @@ __device__ __forceinline__ bool face_mass_simple(const SweepArgs& a, long long K
     // s = u1[K] + u2[K]
     const long long sd = a.g.s[a.d];
     const unsigned long long sb = bits(s);
-    if ((sb & ABS_MASK) == 0ull) {   // δl == 0: ρuf stays 0
+    if (is_zero(s)) {   // δl == 0: ρuf stays 0
         m = 0.0;
         return true;
     }
@@ -172,17 +175,10 @@ __device__ __forceinline__ void warp_append(unsigned int* list, unsigned int* co
     if (pred) list[base + __popc(mask & ((1u << lane) - 1u))] = val;
 }
 
+// One lane's cell of a bulk pass (a lane without one comes along for the list appends, which are warp-collective)
 template <int D, bool FIRST, bool DILA>
-__global__ void __launch_bounds__(256) vof_bulk(SweepArgs a) {
-    // x in [1, n-2] one cell per lane, so that a row of 32k interior cells fills k warps; the
-    // last block column's first warp takes the ghost cells x = 0 and n-1 of the block's 8 rows.
-    // Lanes without a cell stay in the warp (the list appends are warp-collective).
+__device__ __forceinline__ void bulk_cell(const SweepArgs& a, int x, int y, int z, bool valid) {
     const Grid& g = a.g;
-    const bool gcol = blockIdx.x + 1 == gridDim.x;
-    const int x = gcol ? ((threadIdx.x & 1) ? g.n[0] - 1 : 0) : 1 + int(blockIdx.x) * 32 + int(threadIdx.x);
-    const int y = gcol ? int(blockIdx.y) * 8 + int(threadIdx.x >> 1) : int(blockIdx.y) * 8 + int(threadIdx.y);
-    const int z = blockIdx.z;
-    const bool valid = (gcol ? (threadIdx.y == 0 && threadIdx.x < 16) : x <= g.n[0] - 2) && y < g.n[1];
     bool need_cell = false, need_face = false;
     long long O = 0;
     if (valid) {
@@ -194,24 +190,21 @@ __global__ void __launch_bounds__(256) vof_bulk(SweepArgs a) {
         int cb;
         if (FIRST) {
             // c̄ = f < 0.5 ? 0 : 1 over every cell (src/advection.jl:40), on the bit pattern
-            const unsigned long long bo = bits(a.fin[O]);
-            const bool lt_half = ((bo & ABS_MASK) <= 0x7FF0000000000000ull) &&            // not NaN
-                                 ((bo >> 63) || bo < 0x3FE0000000000000ull);             // negative or < 0.5
-            a.cbar[O] = lt_half ? 0 : 1;
+            a.cbar[O] = below_half(a.fin[O]) ? 0 : 1;
             cb = (bc == ONE_BITS) ? 1 : 0;          // only consulted when bc is bulk
         } else {
             cb = a.cbar[S];
         }
         const bool bulk = (bm == bc) && (bc == bp) && is_bulk(bc) && (cb == (bc == ONE_BITS ? 1 : 0)) &&
-                          abs_le(bits(a.u1[S]), a.ulim) && abs_le(bits(a.u1[S + sd]), a.ulim) &&
-                          abs_le(bits(a.u2[S]), a.ulim) && abs_le(bits(a.u2[S + sd]), a.ulim);
+                          abs_le(a.u1[S], a.ulim) && abs_le(a.u1[S + sd], a.ulim) &&
+                          abs_le(a.u2[S], a.ulim) && abs_le(a.u2[S + sd], a.ulim);
         need_cell = !bulk;
         double sS = 0.0;   // u1[S] + u2[S]: the dilation difference's and an interior face's mass flux sum
         if (DILA) {
             // the momentum update's dilation term of this (ghost-mapped) cell, on FP32 pairs: c̄ of the
             // source cell (in the first sweep from its fraction, as the c̄ pass above computes it)
             int cs;
-            if (FIRST) cs = (((bc & ABS_MASK) <= 0x7FF0000000000000ull) && ((bc >> 63) || bc < 0x3FE0000000000000ull)) ? 0 : 1;
+            if (FIRST) cs = below_half(__longlong_as_double((long long)bc)) ? 0 : 1;
             else cs = cb;
             // the velocity difference in FP64 as (u1 + u2)(S + δd) − (u1 + u2)(S): the second sum is the face
             // mass flux's for an interior cell, so the cell issues two FP64 additions for both instead of
@@ -242,8 +235,150 @@ __global__ void __launch_bounds__(256) vof_bulk(SweepArgs a) {
     warp_append(a.flist, a.flist_count, valid && need_face, (unsigned int)O);
 }
 
+template <int D, bool FIRST, bool DILA>
+__global__ void __launch_bounds__(256) vof_bulk(SweepArgs a) {
+    // x in [1, n-2] one cell per lane, so that a row of 32k interior cells fills k warps; the
+    // last block column's first warp takes the ghost cells x = 0 and n-1 of the block's 8 rows.
+    const Grid& g = a.g;
+    const bool gcol = blockIdx.x + 1 == gridDim.x;
+    const int x = gcol ? ((threadIdx.x & 1) ? g.n[0] - 1 : 0) : 1 + int(blockIdx.x) * 32 + int(threadIdx.x);
+    const int y = gcol ? int(blockIdx.y) * 8 + int(threadIdx.x >> 1) : int(blockIdx.y) * 8 + int(threadIdx.y);
+    const bool valid = (gcol ? (threadIdx.y == 0 && threadIdx.x < 16) : x <= g.n[0] - 2) && y < g.n[1];
+    bulk_cell<D, FIRST, DILA>(a, x, y, blockIdx.z, valid);
+}
+
+// ---- whole-call scan (3D advection alone): the full cells of a call in one pass
+// Most tiles of a grid hold one fluid, and then nothing in them changes in any sweep: a cell changes in a sweep along d
+// only if its two neighbours along d differ from it, every dimension is swept once a call, so by induction only if some
+// cell of the 3 x 3 x 3 box around it (of the box around its source cell, for a ghost) differs from it in the field
+// that the call starts from.  vof_scan writes what all sweeps would write into such a tile (ρuf along every direction,
+// c̄) and lists the others; the sweeps' bulk passes then go through the listed tiles (vof_bulk_tiles).  A velocity above
+// the bulk test's bound anywhere sends every tile to the sweeps.
+// What bounds it: HBM and the FP64 pipe alike (81 B and 6 FP64 operations a cell for the three directions, 0.2 ms each
+// at 256^3), and before them latency: a block's loads of f end at a barrier, so that eight blocks of 32 registers a
+// thread beat four that load two planes of velocities at once (a call 527 us against 559).  A sphere in 256^3 cells:
+// 856 us a call with a pass over the whole grid in each of the three sweeps, 527 us with the scan.
+constexpr int VT_X = 32, VT_Y = 8, VT_Z = 8;
+inline __host__ __device__ int tiles_of(int n, int t) { return (n + t - 1) / t; }
+__device__ __forceinline__ void tile_origin(const Grid& g, int t, int& x0, int& y0, int& z0) {
+    const int tx = tiles_of(g.n[0], VT_X), ty = tiles_of(g.n[1], VT_Y);
+    x0 = t % tx * VT_X;
+    t /= tx;
+    y0 = t % ty * VT_Y;
+    z0 = t / ty * VT_Z;
+}
+
+// The coordinates outside a tile [lo, hi] of dimension e whose cells its own can depend on: the one on either side; with
+// the upper ghost in the tile the two below it (its source's neighbour; the ghost can have a tile to itself); with a
+// periodic ghost in the tile or beside it the three around that ghost's source.  The k-th of them (at most 8).
+__device__ __forceinline__ int tile_low(const Grid& g, int e, int lo, int hi) {
+    return max(0, hi == g.n[e] - 1 ? min(lo - 1, g.n[e] - 3) : lo - 1);
+}
+__device__ __forceinline__ bool beside(const Grid& g, int e, int lo, int hi, int k, int& c) {
+    const int low = tile_low(g, e, lo, hi);
+    if (k < lo - low) { c = low + k; return true; }
+    k -= lo - low;
+    if (hi < g.n[e] - 1) {
+        if (k == 0) { c = hi + 1; return true; }
+        --k;
+    }
+    if (!g.isper(e)) return false;
+    if (lo == 0) {
+        if (k < 3) { c = g.n[e] - 3 + k; return true; }
+        k -= 3;
+    }
+    if (hi >= g.n[e] - 2 && k < 3) { c = k; return true; }
+    return false;
+}
+
+__global__ void __launch_bounds__(256, 8) vof_scan(ScanArgs a) {
+    const Grid& g = a.g;
+    int x0, y0, z0;
+    tile_origin(g, blockIdx.x, x0, y0, z0);
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5, x = x0 + tx, y = y0 + ty;
+    const int x1 = min(x0 + VT_X, g.n[0]) - 1, y1 = min(y0 + VT_Y, g.n[1]) - 1, z1 = min(z0 + VT_Z, g.n[2]) - 1;
+    const long long s1 = g.s[1], s2 = g.s[2];
+    const unsigned long long ref = bits(a.f[x0 + y0 * s1 + z0 * s2]);
+    const int zl = tile_low(g, 2, z0, z1), zh = min(z1 + 1, g.n[2] - 1);
+    bool same = is_bulk(ref);
+    auto column = [&](int cx, int cy) {   // (cx, cy) at the tile's depths and those beside it
+        const double* f = a.f + cx + cy * s1;
+#pragma unroll 5
+        for (int z = zl; z <= zh; ++z) same = same & (bits(f[z * s2]) == ref);
+        if (g.isper(2)) {
+            if (z0 == 0)
+                for (int z = max(0, g.n[2] - 3); z < g.n[2]; ++z) same = same & (bits(f[z * s2]) == ref);
+            if (z1 >= g.n[2] - 2)
+                for (int z = 0; z < 3; ++z) same = same & (bits(f[z * s2]) == ref);
+        }
+    };
+    if (x <= x1 && y <= y1) column(x, y);
+    int cx, cy;
+    if (ty < 2) {   // two warps: the tile's x in the rows beside it
+        for (int k = ty; beside(g, 1, y0, y1, k, cy); k += 2)
+            if (x <= x1) column(x, cy);
+    } else if (ty < 6) {   // 128 threads: row q % 16 of column q / 16 beside it (rows 8-15: those beside the tile)
+        const int q = tid - 64;
+        for (int k = q >> 4; beside(g, 0, x0, x1, k, cx); k += 8) {
+            if ((q & 15) < 8) {
+                if (y0 + (q & 15) <= y1) column(cx, y0 + (q & 15));
+            } else if (beside(g, 1, y0, y1, (q & 15) - 8, cy)) {
+                column(cx, cy);
+            }
+        }
+    }
+    const bool uniform = __syncthreads_and(same);
+    if (!uniform && tid == 0) a.tiles[atomicAdd(a.count, 1u)] = blockIdx.x;
+    const bool one = ref == ONE_BITS;
+    const double c = one ? a.h : a.hl;
+    bool fast = true;
+    if (x <= x1 && y <= y1) {
+        const bool in_x = x >= 1 && x <= g.n[0] - 2, in_y = y >= 1 && y <= g.n[1] - 2;
+        const bool lo_x = x >= 1, lo_y = y >= 1;
+#pragma unroll 1
+        for (int z = z0; z <= z1; ++z) {
+            const long long I = x + y * s1 + z * s2;
+            const bool in_z = z >= 1 && z <= g.n[2] - 2, lo_z = z >= 1;
+            double p[3], q[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                p[d] = a.u1[I + d * g.N];
+                q[d] = a.u2[I + d * g.N];
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) fast = fast & abs_le(p[d], a.ulim) & abs_le(q[d], a.ulim);
+            if (!uniform) continue;
+            a.cbar[I] = one ? 1 : 0;
+            if (!a.rhouf) continue;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const bool face = (d == 0 ? lo_x : in_x) && (d == 1 ? lo_y : in_y) && (d == 2 ? lo_z : in_z);
+                const double s = p[d] + q[d];
+                a.rhouf[I + d * g.N] = face && !is_zero(s) ? c * s : 0.0;
+            }
+        }
+    }
+    if (!__syncthreads_and(fast) && tid == 0) atomicOr(a.above, 1u);
+}
+
+// the bulk pass of a sweep over the listed tiles (every tile when a velocity was above the bound), a plane at a time
+template <bool FIRST>
+__global__ void __launch_bounds__(256) vof_bulk_tiles(SweepArgs a) {
+    const Grid& g = a.g;
+    const bool every = *a.above != 0u;
+    const long long n = every ? (long long)tiles_of(g.n[0], VT_X) * tiles_of(g.n[1], VT_Y) * tiles_of(g.n[2], VT_Z)
+                              : (long long)*a.tile_count;
+    for (long long k = blockIdx.x; k < n * VT_Z; k += gridDim.x) {
+        int x0, y0, z0;
+        tile_origin(g, every ? int(k / VT_Z) : int(a.tiles[k / VT_Z]), x0, y0, z0);
+        const int x = x0 + int(threadIdx.x), y = y0 + int(threadIdx.y), z = z0 + int(k % VT_Z);
+        if (z < g.n[2]) bulk_cell<3, FIRST, false>(a, x, y, z, x < g.n[0] && y < g.n[1]);
+    }
+}
+
 template <int D>
-__global__ void __launch_bounds__(128) vof_faces(SweepArgs a) {
+// one warp a block: few warps have work, and this spreads them over the SMs (a sphere at 256^3: 540 us a call, 559 with four)
+__global__ void __launch_bounds__(32) vof_faces(SweepArgs a) {
     const unsigned int count = *a.flist_count;
     for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const long long K = a.flist[k];
@@ -308,6 +443,10 @@ template <int D, bool FIRST>
 void launch_bulk(const SweepArgs& a, cudaStream_t st) {
     dim3 blk(32, 8, 1);
     dim3 grd((a.g.n[0] - 2 + 31) / 32 + 1, (a.g.n[1] + 7) / 8, a.g.n[2]);
+    if (a.tiles) {
+        if constexpr (D == 3) { vof_bulk_tiles<FIRST><<<a.tile_blocks, blk, 0, st>>>(a); ia::note_launch(); }
+        return;
+    }
     if (a.dila) { vof_bulk<D, FIRST, true><<<grd, blk, 0, st>>>(a); ia::note_launch(); }
     else { vof_bulk<D, FIRST, false><<<grd, blk, 0, st>>>(a); ia::note_launch(); }
 }
@@ -320,9 +459,17 @@ cudaError_t vof_sweep_bulk(const SweepArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+long long vof_tiles(const Grid& g) {
+    return (long long)tiles_of(g.n[0], VT_X) * tiles_of(g.n[1], VT_Y) * tiles_of(g.n[2], VT_Z);
+}
+cudaError_t vof_scan_call(const ScanArgs& a, cudaStream_t st) {
+    { vof_scan<<<unsigned(vof_tiles(a.g)), 256, 0, st>>>(a); ia::note_launch(); }
+    return cudaGetLastError();
+}
+
 cudaError_t vof_sweep_faces(const SweepArgs& a, cudaStream_t st, int list_blocks) {
-    if (a.g.D == 2) { vof_faces<2><<<list_blocks, 128, 0, st>>>(a); ia::note_launch(); }
-    else { vof_faces<3><<<list_blocks, 128, 0, st>>>(a); ia::note_launch(); }
+    if (a.g.D == 2) { vof_faces<2><<<list_blocks * 4, 32, 0, st>>>(a); ia::note_launch(); }
+    else { vof_faces<3><<<list_blocks * 4, 32, 0, st>>>(a); ia::note_launch(); }
     return cudaGetLastError();
 }
 

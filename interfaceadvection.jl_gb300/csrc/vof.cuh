@@ -38,7 +38,32 @@ struct SweepArgs {
     // momentum update reads (src/flow.jl:216, 229); rq = λρ/4 and (λρ + (1-λρ))/4 as pairs
     float2* dila = nullptr;
     float rq_l_hi = 0.f, rq_l_lo = 0.f, rq_1_hi = 0.f, rq_1_lo = 0.f;
+    // after vof_scan_call: the bulk pass goes through these tiles alone (every tile when *above is set)
+    const unsigned int* tiles = nullptr;
+    const unsigned int* tile_count = nullptr;
+    const unsigned int* above = nullptr;
+    int tile_blocks = 0;
 };
+
+// the scan of a whole call (3D): ρuf (all components, or nullptr) and c̄ of the tiles of one fluid, a list of the others
+struct ScanArgs {
+    Grid g;
+    const double* f;
+    const double* u1;
+    const double* u2;
+    int8_t* cbar;
+    double* rhouf;
+    double h, hl;                     // δt/2, δt/2 · λρ
+    unsigned long long ulim;
+    unsigned int* tiles;
+    unsigned int* count;
+    unsigned int* above;
+};
+// cells from which a call scans first: below, the extra launch costs what the sweeps' passes over the grid do (a sphere,
+// without and with the scan: 32^3 159 and 172 us, 96^3 197 and 198, 128^3 240 and 229, 256^3 855 and 527)
+constexpr long long VOF_SCAN_CELLS = 1500000;
+long long vof_tiles(const Grid& g);
+cudaError_t vof_scan_call(const ScanArgs& a, cudaStream_t st);
 
 cudaError_t vof_sweep_bulk(const SweepArgs& a, cudaStream_t st);
 cudaError_t vof_sweep_faces(const SweepArgs& a, cudaStream_t st, int list_blocks);

@@ -40,3 +40,23 @@ def test_quotients_near_the_ends_of_the_range(cuda, D, speed):
     u = fzeros(tuple(intf.Ng) + (D,), torch.float64, "cuda")
     u[..., 0] = speed
     against_oracle(intf, u, u, 1.0, 2, rel=1e5 * speed)
+
+
+@pytest.mark.parametrize("n,per,centre", [((190, 94, 86), (), (0.5, 0.5, 0.5)), ((191, 95, 87), (0, 1, 2), (0.02, 0.98, 0.0)),
+                                          ((254, 89, 65), (0, 2), (0.99, 0.5, 0.99)), ((97, 160, 95), (1,), (0.0, 0.0, 1.0))])
+@pytest.mark.parametrize("cfl", [0.45, 0.9])
+def test_tiles_of_one_fluid(cuda, n, per, centre, cfl):
+    """From 1.5 million cells on the tiles of one fluid are done in one pass: sizes with whole, ragged and ghost-only last
+    tiles, interfaces at and across the boundaries, and velocities below and above the bound of that pass."""
+    r = 0.2 * min(n)
+    intf = ia.cVOF(n, perdir=per, InterfaceSDF=lambda x: torch.sqrt(
+        sum((x[d] - centre[d] * n[d] - 0.137 * (d + 1)) ** 2 for d in range(3))) - r)
+    g = torch.Generator().manual_seed(len(per))
+    u1, u2 = (fzeros(tuple(intf.Ng) + (3,), torch.float64, "cuda") for _ in range(2))
+    x = torch.meshgrid(*[torch.arange(m, dtype=torch.float64) for m in intf.Ng], indexing="ij")
+    for u in (u1, u2):
+        for d in range(3):
+            k, ph = torch.randint(1, 4, (3,), generator=g), torch.rand(3, generator=g)
+            u[..., d] = (cfl * torch.stack([torch.sin(6.283185307179586 * (k[e] * x[e] / intf.Ng[e] + ph[e]))
+                                            for e in range(3)]).prod(0)).to("cuda")
+    against_oracle(intf, u1, u2, 1.0, 3, per)
