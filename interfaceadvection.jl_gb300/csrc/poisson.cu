@@ -431,6 +431,8 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
     }
 }
 
+#include "poisson_regular.cuh"
+
 // ---- temporally blocked red-black Gauss-Seidel (3D, FP32): S half-sweeps in one launch.
 // A block owns a TB_X x TB_Y column of interior cells and a range of z-planes and marches up
 // z as a wavefront: at step t half-sweep s works on plane t - s over the column widened by
@@ -1045,11 +1047,13 @@ constexpr int KBLOCKS = 1216;   // 8 blocks on each of 152 SMs
             for (int x = 1 + threadIdx.x; x <= nxi_; x += blockDim.x) {                    \
                 const int I = row_ + x;
 
-// Blocks of the whole-array FP32 vector kernels: two float4 a thread on small grids (every further block only adds
-// a partial to the last block's sum), the row loops' grid on large ones.
-inline int vblocks(const Grid& g) {
+// Blocks of the whole-array vector kernels: two float4 a thread on small grids (every further block only adds a partial
+// to the last block's sum), on large ones as many as are resident at once (update32_k and dot2_32_k at 128x192x160:
+// 12.1 and 14.3 us with 4 an SM, 12.8 and 20.0 with 8, of which 6 and 4 were resident; 8 of 32 registers 17.3 and 19.7).
+constexpr int VB_RESIDENT = 4;
+inline int vblocks(const Grid& g, int nsm) {
     const long long b = (g.N / 4 + 2 * KTHREADS - 1) / (2 * KTHREADS);
-    return int(std::max<long long>(1, std::min<long long>(b, KBLOCKS)));
+    return int(std::max<long long>(1, std::min<long long>(b, std::min(VB_RESIDENT * std::max(nsm, 1), KBLOCKS))));
 }
 inline int kblocks(const Grid& g) {
     const long long rows = (long long)(g.n[1] - 2) * (g.D == 3 ? g.n[2] - 2 : 1);
@@ -1441,56 +1445,90 @@ __global__ void __launch_bounds__(256) update64_k(long long n, FcgDev* __restric
 
 // ---- FP32 inner Krylov kernels (mixed / learned): FP32 products, per-thread sums in FP32
 // over its cells, FP64 block and cross-block sums.
-// q = A p and per-block partial sums of p·q on x-y tiles: a block of 256 threads takes 32 x 8 cells of
-// MV_ZT consecutive z planes (one plane in 2D), so that the stencil's x and y neighbours come from L1 and
-// every load of a cell issues at once (a row loop, one row per block and step, waits for each row's
-// loads and fetches the y neighbours from other SMs' rows through L2).  The partials, one per block,
-// are summed in a fixed order.  Four blocks per SM (64 registers) let a thread keep more of its planes'
-// loads in flight: 0.180 against 0.194 ms per launch at 256x512x256 with the default 32 registers.
+// The x-y tiles of a matrix product: 32 x 8 cells of zt consecutive planes, x fastest
+struct MvTiles {
+    int nx, ny, n, zt;
+    __host__ __device__ MvTiles(const Grid& g, int planes) : zt(planes) {
+        nx = (g.n[0] - 2 + 31) / 32;
+        ny = (g.n[1] - 2 + 7) / 8;
+        n = nx * ny * (g.D == 3 ? (g.n[2] - 2 + zt - 1) / zt : 1);
+    }
+    __device__ __forceinline__ void origin(int t, int& x, int& y, int& z) const {
+        const int r = t / nx;
+        x = 1 + (t - r * nx) * 32;
+        z = r / ny;
+        y = 1 + (r - z * ny) * 8;
+        z = 1 + z * zt;
+    }
+};
+constexpr int MV_RESIDENT = 5;   // blocks on a multiprocessor
+inline unsigned mv_blocks(const Grid& g, int zt, int nsm) {
+    return unsigned(std::min(MvTiles(g, zt).n, MV_RESIDENT * std::max(nsm, 1)));
+}
 
-template <int D, int ZT>
-__global__ void __launch_bounds__(256, 4) matvec32_tile_k(Grid g, const float* __restrict__ L,
-                                                       const float* __restrict__ pv, float* __restrict__ q,
-                                                       double* __restrict__ partial, FcgDev* S) {
-    const int x = 1 + int(blockIdx.x) * 32 + int(threadIdx.x & 31), y = 1 + int(blockIdx.y) * 8 + int(threadIdx.x >> 5);
-    const int z0 = D == 3 ? 1 + ZT * int(blockIdx.z) : 0;
-    float acc = 0.f;
-    auto cell = [&](int z) {
-        const int I = x + y * int(g.s[1]) + z * int(g.s[2]);
-        const Nb o = nb_of<D>(g, x, y, z);
-        const float v = off7<D>(g, L, pv, I, o) + diag7<D>(g, L, I) * pv[I];
-        q[I] = v;
-        acc += pv[I] * v;
-    };
-    if (x <= g.n[0] - 2 && y <= g.n[1] - 2) {
-        if (D == 3 && z0 + ZT - 1 <= g.n[2] - 2) {
-            // a full tile: no bound test between the planes, so that their loads can be issued early
-            // and a plane's values reused as the next plane's z neighbours
+// q = A p and per-block partial sums of p·q on x-y tiles: a block of 256 threads takes 32 x 8 cells of MV_ZT consecutive
+// z planes (one plane in 2D) at a time, so that the stencil's x and y neighbours come from L1 and every load of a cell
+// issues at once (a row loop, one row per block and step, waits for each row's loads and fetches the y neighbours from
+// other SMs' rows through L2).  As many blocks as the device holds go through all tiles: a block of its own for each
+// tile ended in a fence and a count, and the last one summed 16384 partials (256x512x256: 183 us so, 166 with 32-bit
+// byte offsets, 141 with 5 resident blocks an SM, 146 with 4, 150 with 6).  The partials are summed in a fixed order.
+// IX: unsigned below RB_CELLS cells, else size_t.
+template <int D, int ZT, class IX>
+__global__ void __launch_bounds__(256, MV_RESIDENT) matvec32_tile_k(Grid g, Ends ends, const float* __restrict__ L,
+                                                                 const float* __restrict__ pv, float* __restrict__ q,
+                                                                 double* __restrict__ partial, FcgDev* S) {
+    const int s1 = int(g.s[1]), s2 = D == 3 ? int(g.s[2]) : 0;
+    const MvTiles tiles(g, ZT);
+    double sum = 0.0;
+    for (int t = blockIdx.x; t < tiles.n; t += gridDim.x) {
+        int x, y, z0;
+        tiles.origin(t, x, y, z0);
+        x += int(threadIdx.x & 31);
+        y += int(threadIdx.x >> 5);
+        if (D == 2) z0 = 0;
+        const int xl = x == 1 ? ends.lo[0] : -1, xh = x == g.n[0] - 2 ? ends.hi[0] : 1;
+        const int yl = y == 1 ? ends.lo[1] : -s1, yh = y == g.n[1] - 2 ? ends.hi[1] : s1;
+        float acc = 0.f;
+        auto cell = [&](int z) {
+            const IX I = x + y * s1 + z * s2;
+            const int zl = z == 1 ? ends.lo[2] : -s2, zh = z == g.n[2] - 2 ? ends.hi[2] : s2;
+            const float c = at(pv, I);
+            const Star s = star7<D>(L, g.N, I, s1, s2, at(pv, I + xl), at(pv, I + xh), at(pv, I + yl), at(pv, I + yh),
+                                    D == 3 ? at(pv, I + zl) : 0.f, D == 3 ? at(pv, I + zh) : 0.f);
+            const float v = s.off + s.dd * c;
+            *(float*)((char*)q + I * (IX)4) = v;
+            acc += c * v;
+        };
+        if (x <= g.n[0] - 2 && y <= g.n[1] - 2) {
+            if (D == 3 && z0 + ZT - 1 <= g.n[2] - 2) {
+                // a full tile: no bound test between the planes, so that their loads can be issued early
+                // and a plane's values reused as the next plane's z neighbours
 #pragma unroll
-            for (int k = 0; k < ZT; ++k) cell(z0 + k);
-        } else {
-            for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
-                if (D == 3 && z0 + k > g.n[2] - 2) break;
-                cell(z0 + k);
+                for (int k = 0; k < ZT; ++k) cell(z0 + k);
+            } else {
+                for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
+                    if (D == 3 && z0 + k > g.n[2] - 2) break;
+                    cell(z0 + k);
+                }
             }
         }
+        // a warp's sum over a tile in FP32 (a fixed shuffle tree), over its tiles in FP64 by one lane: a per-thread
+        // FP64 reduction costs more FP64-pipe time than the stencil itself
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        if ((threadIdx.x & 31) == 0) sum += double(acc);
     }
-    // the warp's sum in FP32 (a fixed shuffle tree), the block's eight warp sums in FP64 by one thread:
-    // a per-thread FP64 reduction costs more FP64-pipe time than the stencil itself
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     __shared__ double ws[8];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = double(acc);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
     __syncthreads();
-    const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
     if (threadIdx.x == 0) {
         double a = 0.0;
         for (int w = 0; w < 8; ++w) a += ws[w];
-        partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = a;
+        partial[blockIdx.x] = a;
     }
     // the last block: p·q in a fixed order, then α
-    if (!last_block(&S->done_mv, nb)) return;
+    if (!last_block(&S->done_mv, gridDim.x)) return;
     double pq = 0.0, unused = 0.0;
-    sum2_by256(partial, nullptr, nb, pq, unused);
+    sum2_by256(partial, nullptr, gridDim.x, pq, unused);
     if (threadIdx.x == 0) fcg_alpha(S, pq);
 }
 
@@ -1498,25 +1536,43 @@ __global__ void __launch_bounds__(256, 4) matvec32_tile_k(Grid g, const float* _
 // ever written, so their ghost entries stay zero and sums and updates over all N entries equal
 // those over the interior; the arrays are streamed as 16-byte vectors (cudaMalloc alignment),
 // the N mod 4 tail by the first threads.
-__global__ void dot2_32_k(long long n, const float* __restrict__ sv, const float* __restrict__ q,
+__global__ void __launch_bounds__(256, VB_RESIDENT) dot2_32_k(long long n, const float* __restrict__ sv, const float* __restrict__ q,
                           const float* __restrict__ r, double* __restrict__ partial, FcgDev* S, int first) {
-    float a1 = 0.f, a2 = 0.f;
+    double b1 = 0.0, b2 = 0.0;
     const long long n4 = n / 4, stride = (long long)gridDim.x * blockDim.x;
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const float4* s4 = reinterpret_cast<const float4*>(sv);
     const float4* q4 = reinterpret_cast<const float4*>(q);
     const float4* r4 = reinterpret_cast<const float4*>(r);
-    for (long long i = t0; i < n4; i += stride) {
-        const float4 a = s4[i], bq = q4[i], br = r4[i];
+    auto add = [&](const float4& a, const float4& bq, const float4& br, float& a1, float& a2) {
         a1 += a.x * bq.x + a.y * bq.y + a.z * bq.z + a.w * bq.w;
         a2 += a.x * br.x + a.y * br.y + a.z * br.z + a.w * br.w;
+    };
+    // four vectors of each array in flight; their products are summed in FP32, a thread's sums in FP64
+    long long i = t0;
+    for (; i + 3 * stride < n4; i += 4 * stride) {
+        float4 a[4], bq[4], br[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            a[k] = s4[i + k * stride];
+            bq[k] = q4[i + k * stride];
+            br[k] = r4[i + k * stride];
+        }
+        float a1 = 0.f, a2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) add(a[k], bq[k], br[k], a1, a2);
+        b1 += double(a1);
+        b2 += double(a2);
     }
+    float a1 = 0.f, a2 = 0.f;
+    for (; i < n4; i += stride) add(s4[i], q4[i], r4[i], a1, a2);
     if (t0 < n - 4 * n4) {
-        const long long i = 4 * n4 + t0;
-        a1 += sv[i] * q[i];
-        a2 += sv[i] * r[i];
+        const long long k = 4 * n4 + t0;
+        a1 += sv[k] * q[k];
+        a2 += sv[k] * r[k];
     }
-    double b1 = a1, b2 = a2;
+    b1 += double(a1);
+    b2 += double(a2);
     block_sum2(b1, b2);
     if (threadIdx.x == 0) {
         partial[blockIdx.x] = b1;
@@ -1531,7 +1587,7 @@ __global__ void dot2_32_k(long long n, const float* __restrict__ sv, const float
 
 // p = s + β p; β = 0 restarts from s without reading the old direction (which a rejected
 // preconditioner output may have left non-finite)
-__global__ void xpby32_k(long long n, const float* __restrict__ sv, const FcgDev* __restrict__ S,
+__global__ void __launch_bounds__(256, VB_RESIDENT) xpby32_k(long long n, const float* __restrict__ sv, const FcgDev* __restrict__ S,
                          float* __restrict__ pv) {
     const float beta = S->beta32;
     const long long n4 = n / 4, stride = (long long)gridDim.x * blockDim.x;
@@ -1539,6 +1595,7 @@ __global__ void xpby32_k(long long n, const float* __restrict__ sv, const FcgDev
     const float4* s4 = reinterpret_cast<const float4*>(sv);
     float4* p4 = reinterpret_cast<float4*>(pv);
     const bool restart = beta == 0.f;
+#pragma unroll 4
     for (long long i = t0; i < n4; i += stride) {
         const float4 a = s4[i];
         if (restart) {
@@ -1555,7 +1612,7 @@ __global__ void xpby32_k(long long n, const float* __restrict__ sv, const FcgDev
 }
 
 // e += α p ; r -= α q ; L∞(r) as float bits into S->rin (nothing after a breakdown)
-__global__ void update32_k(long long n, FcgDev* __restrict__ S, const float* __restrict__ pv,
+__global__ void __launch_bounds__(256, VB_RESIDENT) update32_k(long long n, FcgDev* __restrict__ S, const float* __restrict__ pv,
                            const float* __restrict__ q, float* __restrict__ e, float* __restrict__ r) {
     if (S->stop) return;
     const float alpha = S->alpha32;
@@ -1571,6 +1628,7 @@ __global__ void update32_k(long long n, FcgDev* __restrict__ S, const float* __r
         const unsigned long long b = __float_as_uint(v) & 0x7FFFFFFFu;
         m = b > m ? b : m;
     };
+#pragma unroll 4
     for (long long i = t0; i < n4; i += stride) {
         const float4 p = p4[i], qq = q4[i];
         float4 ee = e4[i], rr = r4[i];
@@ -1816,6 +1874,16 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto& C = mg->lev[l + 1];
     const T om = T(mg->omega);
     const bool reg = mg_regular(L.g, C.g);
+    // 3D levels in FP32 that halve evenly: the kernels of poisson_regular.cuh
+    const bool even = sizeof(T) == 4 && L.g.D == 3 && reg && L.g.N < RB_CELLS;
+    auto with_even = [&](auto&& launch) {
+        if constexpr (sizeof(T) == 4) {
+            const float* xc = C.x32;
+            if (L16) launch(rb_args(L.g, C.g, L16, b, iD, x, xc, om));
+            else launch(rb_args(L.g, C.g, Lc, b, iD, x, xc, om));
+        }
+        ia::note_launch();
+    };
     // each launch takes the interior rows [y0, y1)
     auto rows = [](dim3 gr, int y0, int y1) {
         gr.y = unsigned((y1 - y0 + 7) / 8);
@@ -1826,6 +1894,16 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto half = [&](int color, int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
         const dim3 gr = rows(pair_tile_grid(L.g), y0, y1);
+        if (even) {
+            with_even([&](auto a) {
+                a.y0 = y0;
+                a.y1 = y1;
+                a.color = color;
+                rb_half_k<std::decay_t<decltype(*a.L)>, false><<<gr, blk(), 0, st>>>(a);
+            });
+            timing_end(h, tk);
+            return;
+        }
         for (int cls = 0; cls <= conf; ++cls) {
             if (cls & ~conf) continue;
             auto go = [&](const auto* coef) {
@@ -1846,6 +1924,15 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto half_prol = [&](int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
         const dim3 gr = rows(pair_tile_grid(L.g), y0, y1);
+        if (even) {
+            with_even([&](auto a) {
+                a.y0 = y0;
+                a.y1 = y1;
+                rb_half_k<std::decay_t<decltype(*a.L)>, true><<<gr, blk(), 0, st>>>(a);
+            });
+            timing_end(h, tk);
+            return;
+        }
         const T* xc = C.template x_<T>();
         auto go = [&](auto REG, const auto* coef) {
             using TL = std::decay_t<decltype(*coef)>;
@@ -1869,8 +1956,20 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto first = [&](bool prol, int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FIRST) : -1;
         const dim3 gr = rows(pair_grid(L.g), y0, y1);
-        const T* xc = C.template x_<T>();
         const int wr = prol ? 0 : write_red;
+        if (even) {
+            with_even([&](auto a) {
+                using TL = std::decay_t<decltype(*a.L)>;
+                a.y0 = y0;
+                a.y1 = y1;
+                a.write_red = wr;
+                if (prol) rb_first_k<TL, true><<<gr, blk(), 0, st>>>(a);
+                else rb_first_k<TL, false><<<gr, blk(), 0, st>>>(a);
+            });
+            timing_end(h, tk);
+            return;
+        }
+        const T* xc = C.template x_<T>();
         auto go = [&](auto PROL, auto REG, const auto* coef) {
             using TL = std::decay_t<decltype(*coef)>;
             constexpr bool P = decltype(PROL)::value, R = decltype(REG)::value;
@@ -1893,6 +1992,14 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     auto restrict_rows = [&](int yc0, int yc1) {
         const dim3 gr = rows(cell_grid(C.g), yc0, yc1);
         T* bc = C.template b_<T>();
+        if (even) {
+            with_even([&](auto a) {
+                a.y0 = yc0;
+                a.y1 = yc1;
+                if constexpr (sizeof(T) == 4) rb_restrict_k<<<gr, blk(), 0, st>>>(a, bc);
+            });
+            return;
+        }
         const T* dg = nullptr;   // FP64: the diagonal is kept in the level's scratch vector
         if constexpr (sizeof(T) == 8) dg = L.r;
         auto go = [&](auto REG, const auto* coef) {
@@ -2130,11 +2237,11 @@ int mg_create(ia_handle* h) {
     e = e ? e : cudaMalloc(&mg->p, 8 * N);
     e = e ? e : cudaMalloc(&mg->q, 8 * N);
     mg->kb = kblocks(g0);
-    mg->vb = vblocks(g0);
     {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&mg->nsm, cudaDevAttrMultiProcessorCount, dev);
+        mg->vb = vblocks(g0, mg->nsm);
         mg->zt = mv_planes(g0, mg->nsm);
         const dim3 mv = mv_tile_grid(g0, mg->zt);
         mg->mvb = (long long)mv.x * mv.y * mv.z;
@@ -2331,7 +2438,17 @@ static int poisson_solve_mixed(ia_handle* h, double* xv, const double* zz, const
             tk = timing_begin(h, TK_KRYLOV);
             { dot2_32_k<<<mg->vb, KTHREADS, 0, st>>>(N, sv, mg->q32, rr, mg->partial, S, it == 0 ? 1 : 0); ia::note_launch(); }
             { xpby32_k<<<mg->vb, KTHREADS, 0, st>>>(N, sv, S, mg->p32); ia::note_launch(); }
-            LAUNCH_TILE(g, matvec32_tile_k, g, F.L32, mg->p32, mg->q32, mg->partial, S);
+            auto matvec = [&](auto IX) {
+                using I = decltype(IX);
+                const unsigned gr = mv_blocks(g, mg->zt, mg->nsm);
+                const Ends e = ends_of(g);
+                if (g.D == 2) matvec32_tile_k<2, MV_ZT, I><<<gr, KTHREADS, 0, st>>>(g, e, F.L32, mg->p32, mg->q32, mg->partial, S);
+                else if (mg->zt == 1) matvec32_tile_k<3, 1, I><<<gr, KTHREADS, 0, st>>>(g, e, F.L32, mg->p32, mg->q32, mg->partial, S);
+                else matvec32_tile_k<3, MV_ZT, I><<<gr, KTHREADS, 0, st>>>(g, e, F.L32, mg->p32, mg->q32, mg->partial, S);
+                ia::note_launch();
+            };
+            if (g.N < RB_CELLS) matvec(0u);
+            else matvec(size_t(0));
             { update32_k<<<mg->vb, KTHREADS, 0, st>>>(N, S, mg->p32, mg->q32, mg->e32, rr); ia::note_launch(); }
             timing_end(h, tk);
             cudaMemcpyAsync(mg->hsc + 2, &S->rin, 8, cudaMemcpyDeviceToHost, st);
