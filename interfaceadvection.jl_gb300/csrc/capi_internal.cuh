@@ -34,7 +34,7 @@ struct ia_handle {
     cudaStream_t stream;
     ia_fields fld;
     // scratch owned by the library
-    double* tmp1 = nullptr;            // staged values of listed cells
+    double* tmp1 = nullptr;            // staged values of listed cells; the fractions between a pair of sweeps
     unsigned int* list = nullptr;      // compacted cells needing the full update
     unsigned int* flist = nullptr;     // compacted faces needing reconstruction
     double* flux = nullptr;            // cached fluxes of listed faces

@@ -429,7 +429,8 @@ __global__ void __launch_bounds__(128) vof_cells(SweepArgs a) {
         }
         // cleanWisp! (src/VOFutil.jl:127-136)
         v = (v < a.tol_clean) ? 0.0 : ((v > 1.0 - a.tol_clean) ? 1.0 : v);
-        a.vals[k] = v;
+        if (a.fin != a.fout) a.fout[O] = v;   // out of place nothing reads it in this sweep
+        else a.vals[k] = v;
     }
 }
 
