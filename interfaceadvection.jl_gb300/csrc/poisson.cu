@@ -97,6 +97,22 @@ __device__ __forceinline__ T resid7(const Grid& g, const T* __restrict__ L, T b,
     }
     return a;
 }
+// b + Σ_i L[I,i] v[I-δi] + L[I+δi,i] v[I+δi] likewise (a result's sign is an FP64 operation too)
+template <int D, class T>
+__device__ __forceinline__ T product7(const Grid& g, const T* __restrict__ L, T b, const T* v, int I, const Nb& o) {
+    const int s1 = int(g.s[1]), s2 = int(g.s[2]);
+    const T* L1 = L + g.N;
+    T a = fma(L[I], v[I + o.xl], b);
+    a = fma(L[I + 1], v[I + o.xh], a);
+    a = fma(L1[I], v[I + o.yl], a);
+    a = fma(L1[I + s1], v[I + o.yh], a);
+    if (D == 3) {
+        const T* L2 = L1 + g.N;
+        a = fma(L2[I], v[I + o.zl], a);
+        a = fma(L2[I + s2], v[I + o.zh], a);
+    }
+    return a;
+}
 // D_I = -Σ_i (L[I,i] + L[I+δi,i])
 template <int D, class TL>
 __device__ __forceinline__ auto diag7(const Grid& g, const TL* __restrict__ L, int I) -> decltype(cf(L[0])) {
@@ -119,6 +135,29 @@ __device__ __forceinline__ auto diag7(const Grid& g, const TL* __restrict__ L, i
     const int z = D == 3 ? 1 + int(blockIdx.z) : 0;                       \
     if (x > (g).n[0] - 2 || y > (g).n[1] - 2) return;                     \
     const int I = x + y * int((g).s[1]) + z * int((g).s[2]);
+// v == 1; in FP64 on the bit pattern, as a comparison takes the FP64 pipe as long as a sum
+__device__ __forceinline__ bool is_one(float v) { return v == 1.f; }
+__device__ __forceinline__ bool is_one(double v) { return __double_as_longlong(v) == 0x3FF0000000000000ll; }
+// The column and row of a thread of a smoother or restriction launch on a level of nx columns.  FP32: a warp takes 32
+// columns of a row.  FP64: rows follow one another through the lanes, as a warp's instruction takes as long with half of
+// its lanes idle (100x200x100, whose 50 pairs a row fill 78 % of two warps: a half-sweep, mean over the levels, 8.1 us with
+// rows of their own and 6.3 so).
+template <class T>
+__device__ __forceinline__ void plane_cell(int nx, int& col, int& row) {
+    if (sizeof(T) == 8) {
+        const int t = int(blockIdx.x) * 256 + int(threadIdx.y) * 32 + int(threadIdx.x);
+        row = t / nx;
+        col = t - row * nx;
+    } else {
+        col = int(blockIdx.x) * 32 + int(threadIdx.x);
+        row = int(blockIdx.y) * 8 + int(threadIdx.y);
+    }
+}
+template <class T>
+inline dim3 plane_grid(int nx, int rows, int planes) {
+    if (sizeof(T) == 8) return dim3(unsigned(((long long)nx * rows + 255) / 256), 1, planes);
+    return dim3((nx + 31) / 32, (rows + 7) / 8, planes);
+}
 inline dim3 cell_grid(const Grid& g) {
     return dim3((g.n[0] - 2 + 31) / 32, (g.n[1] - 2 + 7) / 8, g.D == 3 ? g.n[2] - 2 : 1);
 }
@@ -222,7 +261,7 @@ __global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, const d
 // lane idles; in FP32 the diagonal comes from the face coefficients the update reads anyway
 // (same value and zero-diagonal rule as set_diag_k).  In FP64 the inverse diagonal is read (set_diag_k) and the
 // update is a chain of 8 multiply-adds: with the diagonal's sums and the division it was about 30 FP64
-// instructions a cell, at 16 cycles a warp each the whole cost (100x200x100, mean over the levels: 18.2 -> 8.0 us).
+// instructions a cell, at 16 cycles a warp each the whole cost (100x200x100, mean over the levels: 18.2 -> 8.1 us).
 // With PROL (over-relaxed first red half-sweep of a post-smoothing whose prolongation is fused
 // into the sweeps) the cell's previous value is x + the injected coarse correction.
 // In 3D a thread takes its pair in RB_ZT consecutive z planes and reads every plane's operands before
@@ -230,21 +269,15 @@ __global__ void restrict_L_k(Grid gc, Grid gf, const T* __restrict__ Lf, const d
 // reads, and the loads of all planes are in flight at once (the z neighbours of one plane are the x
 // neighbours of the next, a repeated address).  The values are those of one plane per thread.
 constexpr int RB_ZT = 2;
-inline dim3 pair_grid(const Grid& g) {
-    const int pairs = (g.n[0] - 2 + 1) / 2;
-    return dim3((pairs + 31) / 32, (g.n[1] - 2 + 7) / 8, g.D == 3 ? g.n[2] - 2 : 1);
-}
-inline dim3 pair_tile_grid(const Grid& g) {
-    const int pairs = (g.n[0] - 2 + 1) / 2;
-    return dim3((pairs + 31) / 32, (g.n[1] - 2 + 7) / 8, g.D == 3 ? (g.n[2] - 2 + RB_ZT - 1) / RB_ZT : 1);
-}
 template <class T, int D, bool PROL = false, class TL = T, bool REG = true>
 __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, const T* __restrict__ b,
                             const T* __restrict__ iD, T* __restrict__ xv, int color, T omega, int conflicts, int cls,
                             Grid gc = Grid(), const T* __restrict__ xc = nullptr) {
-    const int y = y0 + int(blockIdx.y * blockDim.y + threadIdx.y);   // rows [y0, y1) of the interior
+    int pair, y;
+    plane_cell<T>((g.n[0] - 1) / 2, pair, y);
+    y += y0;   // rows [y0, y1) of the interior
     if (y >= y1) return;
-    const int xp = 1 + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int xp = 1 + 2 * pair;
     const int z0 = D == 3 ? 1 + RB_ZT * int(blockIdx.z) : 0;
     const T eps = sizeof(T) == 8 ? T(2.220446049250313e-16) : T(1.1920929e-7);
     // plane k's cell of this colour and its operands: the off-diagonal sum, the diagonal, b and
@@ -268,19 +301,19 @@ __global__ void rbgs_pair_k(Grid g, int y0, int y1, const TL* __restrict__ L, co
             dd = diag7<D>(g, L, I);
             bv = b[I];
         }
-        if (omega != T(1)) {
+        if (!is_one(omega)) {
             xo = xv[I];
             if (PROL) xo += xc[mg_parent_cell<REG>(gc, x, y, z)];
         }
     };
     auto store = [&](int I, T off, T dd, T bv, T xo) {
         if constexpr (sizeof(T) == 8) {
-            xv[I] = omega == T(1) ? bv * dd : fma(omega, fma(bv, dd, -xo), xo);
+            xv[I] = is_one(omega) ? bv * dd : fma(omega, fma(bv, dd, -xo), xo);
             return;
         }
         const T iD = (dd * dd < T(2) * eps) ? T(0) : T(1) / dd;
         const T gs = (bv - off) * iD;
-        if (omega == T(1)) xv[I] = gs;
+        if (is_one(omega)) xv[I] = gs;
         else xv[I] = xo + omega * (gs - xo);   // over-relaxation: x + ω (x_GS - x)
     };
     const int xmax = g.n[0] - 2;
@@ -328,23 +361,25 @@ __device__ __forceinline__ T first_nb(const Grid& g, const Grid& gc, const T* __
     if (!in) return xv[J];
     if (!PROL && sizeof(T) == 8) return b[J] * iD[J];   // the caller's sum takes the factor omega
     if (PROL) return xv[J] + xc[mg_parent_cell<REG>(gc, cx, cy, cz)];
-    return omega == T(1) ? b[J] * iD[J] : omega * (b[J] * iD[J]);
+    return is_one(omega) ? b[J] * iD[J] : omega * (b[J] * iD[J]);
 }
 
 template <class T, int D, bool PROL, class TL = T, bool REG = true>
 __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restrict__ L, const T* __restrict__ b,
                              const T* __restrict__ iD, const T* __restrict__ xc, T* __restrict__ xv, int write_red,
                              T omega) {
-    const int y = y0 + int(blockIdx.y * blockDim.y + threadIdx.y);   // rows [y0, y1) of the interior
+    int pair, y;
+    plane_cell<T>((g.n[0] - 1) / 2, pair, y);
+    y += y0;   // rows [y0, y1) of the interior
     const int z = D == 3 ? 1 + int(blockIdx.z) : 0;
     if (y >= y1) return;
-    const int x0 = 1 + 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int x0 = 1 + 2 * pair;
     const bool blk0 = ((x0 + y + z) & 1) == 1;
     const int x = blk0 ? x0 : x0 + 1, xr = blk0 ? x0 + 1 : x0;   // black and red cell of the pair
     const int s1 = int(g.s[1]), s2 = int(g.s[2]);
     if (!PROL && write_red && xr <= g.n[0] - 2) {
         const int Ir = xr + y * s1 + z * s2;
-        xv[Ir] = omega == T(1) ? b[Ir] * iD[Ir] : omega * (b[Ir] * iD[Ir]);
+        xv[Ir] = is_one(omega) ? b[Ir] * iD[Ir] : omega * (b[Ir] * iD[Ir]);
     }
     if (x > g.n[0] - 2) return;
     const int I = x + y * s1 + z * s2;
@@ -381,7 +416,7 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
         } else {
 #pragma unroll
             for (int q = 0; q < 2 * D; ++q)
-                v[q] = omega == T(1) || sizeof(T) == 8 ? b[J[q]] * iD[J[q]] : omega * (b[J[q]] * iD[J[q]]);
+                v[q] = is_one(omega) || sizeof(T) == 8 ? b[J[q]] * iD[J[q]] : omega * (b[J[q]] * iD[J[q]]);
         }
     } else {
         const Nb o = nb_of<D>(g, x, y, z);
@@ -407,8 +442,8 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
         }
         if (PROL) {
             const T gs = (b[I] - a) * iD[I];
-            const T xo = omega == T(1) ? T(0) : xv[I] + xc[mg_parent_cell<REG>(gc, x, y, z)];
-            xv[I] = omega == T(1) ? gs : fma(omega, gs - xo, xo);
+            const T xo = is_one(omega) ? T(0) : xv[I] + xc[mg_parent_cell<REG>(gc, x, y, z)];
+            xv[I] = is_one(omega) ? gs : fma(omega, gs - xo, xo);
         } else {
             xv[I] = omega * (fma(-omega, a, b[I]) * iD[I]);
         }
@@ -421,7 +456,7 @@ __global__ void rbgs_first_k(Grid g, int y0, int y1, Grid gc, const TL* __restri
     const T eps = sizeof(T) == 8 ? T(2.220446049250313e-16) : T(1.1920929e-7);
     const T iDI = (dd * dd < T(2) * eps) ? T(0) : T(1) / dd;
     const T gs = (b[I] - a) * iDI;
-    if (omega == T(1)) {
+    if (is_one(omega)) {
         xv[I] = gs;
     } else if (PROL) {   // over-relaxation from the prolongated value of this (black) cell
         const T xo = xv[I] + xc[mg_parent_cell<REG>(gc, x, y, z)];
@@ -638,8 +673,10 @@ __global__ void residual_k(Grid g, const T* __restrict__ L, const T* __restrict_
 template <class T, int D, class TL = T, bool REG = true>
 __global__ void resid_restrict_k(Grid gc, int yc0, int yc1, Grid gf, const TL* __restrict__ L,
                                  const T* __restrict__ diag, const T* __restrict__ b, const T* __restrict__ xv, T* __restrict__ bc) {
-    const int xc = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int yc = yc0 + int(blockIdx.y * blockDim.y + threadIdx.y);   // coarse rows [yc0, yc1)
+    int xc, yc;
+    plane_cell<T>(gc.n[0] - 2, xc, yc);
+    xc += 1;
+    yc += yc0;   // coarse rows [yc0, yc1)
     const int zc = D == 3 ? 1 + int(blockIdx.z) : 0;
     if (xc > gc.n[0] - 2 || yc >= yc1) return;
     const int s1 = int(gf.s[1]), s2 = int(gf.s[2]);
@@ -1376,7 +1413,7 @@ __global__ void __launch_bounds__(256) matvec64_tile_k(Grid g, const double* __r
             const int z = z0 + k;
             if (D == 3 && z > g.n[2] - 2) break;
             const int I = x + y * int(g.s[1]) + z * int(g.s[2]);
-            const double v = -resid7<D>(g, L, -diag[I] * pv[I], pv, I, nb_of<D>(g, x, y, z));
+            const double v = product7<D>(g, L, diag[I] * pv[I], pv, I, nb_of<D>(g, x, y, z));
             q[I] = v;
             acc = fma(pv[I], v, acc);
         }
@@ -1885,15 +1922,12 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
         ia::note_launch();
     };
     // each launch takes the interior rows [y0, y1)
-    auto rows = [](dim3 gr, int y0, int y1) {
-        gr.y = unsigned((y1 - y0 + 7) / 8);
-        return gr;
-    };
+    const int pairs = (L.g.n[0] - 1) / 2;
     // cells of one colour that touch across a wrap are updated in passes, one per class of such cells
     const int conf = wrap_conflicts(L.g);
     auto half = [&](int color, int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
-        const dim3 gr = rows(pair_tile_grid(L.g), y0, y1);
+        const dim3 gr = plane_grid<T>(pairs, y1 - y0, L.g.D == 3 ? (L.g.n[2] - 2 + RB_ZT - 1) / RB_ZT : 1);
         if (even) {
             with_even([&](auto a) {
                 a.y0 = y0;
@@ -1923,7 +1957,7 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     // coarse correction, which it adds to the value it reads
     auto half_prol = [&](int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FINE) : -1;
-        const dim3 gr = rows(pair_tile_grid(L.g), y0, y1);
+        const dim3 gr = plane_grid<T>(pairs, y1 - y0, L.g.D == 3 ? (L.g.n[2] - 2 + RB_ZT - 1) / RB_ZT : 1);
         if (even) {
             with_even([&](auto a) {
                 a.y0 = y0;
@@ -1955,7 +1989,7 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     // first black half-sweep: from x = 0 (pre) or from x + P(x_coarse) (post)
     auto first = [&](bool prol, int y0, int y1) {
         const int tk = (l == 0) ? timing_begin(h, TK_MG_FIRST) : -1;
-        const dim3 gr = rows(pair_grid(L.g), y0, y1);
+        const dim3 gr = plane_grid<T>(pairs, y1 - y0, L.g.D == 3 ? L.g.n[2] - 2 : 1);
         const int wr = prol ? 0 : write_red;
         if (even) {
             with_even([&](auto a) {
@@ -1990,7 +2024,7 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
     };
     // residual restriction of the coarse rows [yc0, yc1)
     auto restrict_rows = [&](int yc0, int yc1) {
-        const dim3 gr = rows(cell_grid(C.g), yc0, yc1);
+        const dim3 gr = plane_grid<T>(C.g.n[0] - 2, yc1 - yc0, C.g.D == 3 ? C.g.n[2] - 2 : 1);
         T* bc = C.template b_<T>();
         if (even) {
             with_even([&](auto a) {
