@@ -1399,15 +1399,16 @@ __device__ void fcg_alpha(FcgDev* S, double pq) {
 
 // ---- FP64 Krylov kernels (IA_POISSON_FP64).  As the FP32 ones below, with the scalars on the device; the vectors
 // are the library's, whose ghost entries stay zero, so they are streamed whole.
-// q = A p and partial sums of p·q on the tiles of matvec32_tile_k, one chain of multiply-adds a cell
+// q = A p and partial sums of p·q, ZT planes a thread, one chain of multiply-adds a cell; the rows follow one another
+// through the lanes
 template <int D, int ZT>
-__global__ void __launch_bounds__(256) matvec64_tile_k(Grid g, const double* __restrict__ L, const double* __restrict__ diag,
+__global__ void __launch_bounds__(256) matvec64_k(Grid g, const double* __restrict__ L, const double* __restrict__ diag,
                                                        const double* __restrict__ pv, double* __restrict__ q,
                                                        double* __restrict__ partial, FcgDev* S) {
-    const int x = 1 + int(blockIdx.x) * 32 + int(threadIdx.x & 31), y = 1 + int(blockIdx.y) * 8 + int(threadIdx.x >> 5);
+    const int nx = g.n[0] - 2, t = int(blockIdx.x) * 256 + int(threadIdx.x), x = 1 + t % nx, y = 1 + t / nx;   // (see plane_cell)
     const int z0 = D == 3 ? 1 + ZT * int(blockIdx.z) : 0;
     double acc = 0.0, unused = 0.0;
-    if (x <= g.n[0] - 2 && y <= g.n[1] - 2) {
+    if (y <= g.n[1] - 2) {
 #pragma unroll
         for (int k = 0; k < (D == 3 ? ZT : 1); ++k) {
             const int z = z0 + k;
@@ -1422,10 +1423,10 @@ __global__ void __launch_bounds__(256) matvec64_tile_k(Grid g, const double* __r
     __shared__ double ws[8];
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
     __syncthreads();
-    const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
+    const unsigned int nb = gridDim.x * gridDim.z;
     if (threadIdx.x == 0) {
         for (int w = 1; w < 8; ++w) acc += ws[w];
-        partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = acc;
+        partial[blockIdx.x + gridDim.x * blockIdx.z] = acc;
     }
     if (!last_block(&S->done_mv, nb)) return;
     double pq = 0.0;
@@ -2705,7 +2706,14 @@ int poisson_solve(ia_handle* h, double* xv, const double* zz, const double* L, d
         tk = timing_begin(h, TK_KRYLOV);
         { dot2_64_k<<<mg->vb, KTHREADS, 0, st>>>(g.N, F.x, mg->q, r, mg->partial, S, it == 0 ? 1 : 0); ia::note_launch(); }
         { xpby64_k<<<mg->vb, KTHREADS, 0, st>>>(g.N, F.x, S, mg->p); ia::note_launch(); }
-        LAUNCH_TILE(g, matvec64_tile_k, g, L, mg->diag64, mg->p, mg->q, mg->partial, S);
+        {
+            // (never more blocks than the 32 x 8 tiles that the partials are allocated for)
+            const dim3 gr(plane_grid<double>(g.n[0] - 2, g.n[1] - 2, mv_tile_grid(g, mg->zt).z));
+            if (g.D == 2) matvec64_k<2, MV_ZT><<<gr, KTHREADS, 0, st>>>(g, L, mg->diag64, mg->p, mg->q, mg->partial, S);
+            else if (mg->zt == 1) matvec64_k<3, 1><<<gr, KTHREADS, 0, st>>>(g, L, mg->diag64, mg->p, mg->q, mg->partial, S);
+            else matvec64_k<3, MV_ZT><<<gr, KTHREADS, 0, st>>>(g, L, mg->diag64, mg->p, mg->q, mg->partial, S);
+            ia::note_launch();
+        }
         { update64_k<<<mg->vb, KTHREADS, 0, st>>>(g.N, S, mg->p, mg->q, xv, r); ia::note_launch(); }
         timing_end(h, tk);
         cudaMemcpyAsync(mg->hsc + 2, &S->rin64, 16, cudaMemcpyDeviceToHost, st);
