@@ -1803,6 +1803,7 @@ static void tb_launch(const PoissonMG* mg, const TbArgs& a, int S, cudaStream_t 
 }
 
 constexpr int TAIL_BYTES = 200 * 1024;   // shared memory of the one-block V-cycle
+constexpr int CL_BYTES = 210 * 1024;     // and, with what is static, of a block of the one-launch solver
 // shared-memory layout of the one-block V-cycle from level l0 on
 template <class T>
 static TailArgs<T> tail_layout(const PoissonMG* mg, int l0) {
@@ -2536,7 +2537,7 @@ static int cluster_blocks(PoissonMG* mg, long long pairs) {
     if (most < 0) {
         int got = 0;
         const auto k = solve_cluster_k<T, D>;
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES) == cudaSuccess &&
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_BYTES) == cudaSuccess &&
             cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
             for (int c = CL_MAX; c >= 1 && !got; c /= 2) {
                 cudaLaunchConfig_t cfg = {};
@@ -2546,7 +2547,7 @@ static int cluster_blocks(PoissonMG* mg, long long pairs) {
                 at.val.clusterDim.y = at.val.clusterDim.z = 1;
                 cfg.gridDim = dim3(c);
                 cfg.blockDim = dim3(TAIL_THREADS);
-                cfg.dynamicSmemBytes = TAIL_BYTES;
+                cfg.dynamicSmemBytes = CL_BYTES;
                 cfg.attrs = &at;
                 cfg.numAttrs = 1;
                 int n = 0;
@@ -2556,6 +2557,22 @@ static int cluster_blocks(PoissonMG* mg, long long pairs) {
         most = got;
     }
     return most >= 1 && pairs <= (long long)CL_PAIRS * most * TAIL_THREADS ? most : 0;
+}
+
+// the words of the levels above the tail and of its first one: pairs a thread keeps of each, offsets; bytes in all
+template <int D>
+static size_t cl_layout(const PoissonMG* mg, int nd, int C, int* kp, int* wo) {
+    int off = 0;
+    for (int l = 0; l <= nd; ++l) {
+        const int share = (cl_pairs<D>(mg->lev[l].g) + C - 1) / C, k = (share + TAIL_THREADS - 1) / TAIL_THREADS;
+        if (kp) {
+            kp[l] = k;
+            wo[l] = off;
+        }
+        off += k * CL_WORDS * TAIL_THREADS;
+    }
+    if (wo) wo[nd + 1] = off;
+    return 4 * (size_t)off;
 }
 
 // Solves on the cluster path when it applies: *done says whether it did.
@@ -2579,10 +2596,11 @@ static cudaError_t cluster_solve(ia_handle* h, double* xv, const double* zz, con
     // (on one level the tail, which then has the coarsest level alone, is not used)
     const int l0 = flat ? mg->nlev - 1 : lt;
     if (!C || lt > CL_LEVELS || (mg->nlev > 1 && mg->lev[1].g.N > 0xFFFF) ||
-        tail_layout<T>(mg, l0).bytes() + cl_words_bytes(lt) > (size_t)TAIL_BYTES)
+        tail_layout<T>(mg, l0).bytes() + cl_layout<D>(mg, lt, C, nullptr, nullptr) > (size_t)CL_BYTES)
         return cudaSuccess;
     *done = true;
     SolveArgs<T> a;
+    const size_t words = cl_layout<D>(mg, lt, C, a.kp, a.wo);
     a.tail = tail_args<T>(mg, l0, mg->nu1, mg->nu2, mg->nuc);
     a.nd = lt;
     a.flat = flat ? 1 : 0;
@@ -2621,6 +2639,30 @@ static cudaError_t cluster_solve(ia_handle* h, double* xv, const double* zz, con
     a.inner_max = mg->inner_max;
     a.partial = mg->partial;
     a.out = reinterpret_cast<SolveOut*>(mg->dsc);
+    // each level's window, where they fit beside the rest
+    const int tops = lt + a.flat;
+    size_t bytes = a.tail.bytes() + words;
+    a.win[0] = -1;
+    a.win_values = 0;
+    if (D == 2 && bytes % sizeof(T) == 0) {
+        int off = 0;
+        for (int l = 0; l < tops && l < CL_LEVELS; ++l) {
+            a.win[l] = off;
+            int most = 0;
+            for (int r = 0; r < C; ++r) {
+                int lo, hi;
+                cl_window<D>(a.g[l], C, r, lo, hi);
+                most = std::max(most, hi - lo + 1);
+            }
+            off += most;
+        }
+        if (tops > 0 && bytes + sizeof(T) * (size_t)off <= (size_t)CL_BYTES) {
+            a.win_values = off;
+            bytes += sizeof(T) * (size_t)off;
+        } else {
+            a.win[0] = -1;
+        }
+    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeClusterDimension;
@@ -2628,7 +2670,7 @@ static cudaError_t cluster_solve(ia_handle* h, double* xv, const double* zz, con
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(TAIL_THREADS);
-    cfg.dynamicSmemBytes = a.tail.bytes() + cl_words_bytes(lt);
+    cfg.dynamicSmemBytes = bytes;
     cfg.stream = h->stream;
     cfg.attrs = &at;
     cfg.numAttrs = 1;

@@ -19,7 +19,35 @@ constexpr int CL_MAX = 16;        // blocks of a cluster
 constexpr int CL_PAIRS = 2;       // pairs of cells a thread keeps on a level
 enum { PRE, POST, FLAT };
 constexpr int CL_LEVELS = 4;      // levels above the tail
-constexpr size_t cl_words_bytes(int nd) { return size_t(nd + 1) * CL_PAIRS * TAIL_WORDS * TAIL_THREADS * 4; }
+constexpr int CL_WORDS = TAIL_WORDS + 1;   // a pair's words: tail_words', and the blocks whose windows hold its cells
+
+// Pairs of a level are dealt to the blocks in order, equally many each.  In 2D a block keeps x of a level above the tail
+// in shared memory, in a window that its neighbours write directly, so that a stage has no store that must reach L2
+// before the barrier and no load from there after it: a step of 161 x 97 cells on one level 14.1 -> 11.8 ms, in FP64
+// 12.2 -> 9.2.  In 3D a block's two planes are all in the neighbours' windows, and L2 is the faster way (a solve of
+// 32 x 64 x 32 cells 1404 us, with windows 1531).  A block's window
+// is x on the rows [lo, hi] that its own cells and their neighbours span (whole rows: a cell's copies across a wrap in x
+// lie in the windows that hold the cell).
+template <int D>
+__host__ __device__ inline int cl_pairs(const Grid& g) {
+    return (g.n[0] - 1) / 2 * (g.n[1] - 2) * (D == 3 ? g.n[2] - 2 : 1);
+}
+template <int D>
+__host__ __device__ inline int cl_cell(const Grid& g, int t) {   // first cell of pair t
+    const int hx = (g.n[0] - 1) / 2, ny = g.n[1] - 2, r = t / hx, z = r / ny;
+    return 1 + 2 * (t - r * hx) + (1 + r - z * ny) * int(g.s[1]) + (D == 3 ? (1 + z) * int(g.s[2]) : 0);
+}
+template <int D>
+__host__ __device__ inline void cl_window(const Grid& g, int C, int rank, int& lo, int& hi) {
+    const int n = cl_pairs<D>(g), share = (n + C - 1) / C, far = int(g.s[D - 1]);
+    const int t0 = rank * share, t1 = min((rank + 1) * share, n);
+    lo = 0;
+    hi = -1;   // a block without pairs
+    if (t0 >= t1) return;
+    const int s1 = int(g.s[1]);
+    lo = (cl_cell<D>(g, t0) - far) / s1 * s1;
+    hi = (cl_cell<D>(g, t1 - 1) + 1 + far) / s1 * s1 + s1 - 1;
+}
 
 struct SolveOut {
     double res;
@@ -31,6 +59,9 @@ struct SolveArgs {
     TailArgs<T> tail;
     int nd;                                           // levels above the tail (0: the tail is the hierarchy)
     int flat;                                         // one level, solved by the coarsest level's sweeps
+    int win[CL_LEVELS];                               // windows: offsets in values behind the words; win[0] < 0: none
+    int win_values;
+    int kp[CL_LEVELS + 1], wo[CL_LEVELS + 2];         // pairs a thread keeps of each level, and where their words lie
     Grid g[CL_LEVELS + 1];
     T* x[CL_LEVELS + 1];
     T* b[CL_LEVELS + 1];                              // b[nd]: the tail's right-hand side
@@ -57,7 +88,10 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
     constexpr bool MIXED = sizeof(T) == 4;
     extern __shared__ __align__(16) unsigned char tail_raw[];
     T* sm = reinterpret_cast<T*>(tail_raw);
-    unsigned* words = reinterpret_cast<unsigned*>(sm + a.tail.values) + a.tail.words;   // CL_PAIRS * TAIL_WORDS a thread and level
+    unsigned* words = reinterpret_cast<unsigned*>(sm + a.tail.values) + a.tail.words;   // kp * CL_WORDS a thread and level
+    T* windows = reinterpret_cast<T*>(words + a.wo[a.nd + 1]);
+    __shared__ int wlo[CL_LEVELS][CL_MAX], whi[CL_LEVELS][CL_MAX];
+    __shared__ int greach[CL_LEVELS][3][2];   // blocks whose windows hold this block's copies across a wrap, by direction
     __shared__ T mean_s, red[2][TAIL_THREADS];
     __shared__ unsigned long long red_max;
     __shared__ double sc[4];
@@ -75,6 +109,12 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
         asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     };
+    // the same for windows alone, which other blocks write directly: nothing has to reach L2
+    auto wsync = [&]() {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    };
+    const bool windowed = D == 2 && a.win[0] >= 0;
     auto cells = [&](const Grid& g, auto&& f) {
         const int nx = g.n[0] - 2, ny = g.n[1] - 2, nz = D == 3 ? g.n[2] - 2 : 1, n = nx * ny * nz;
         for (int t = t0; t < n; t += stride) {
@@ -123,38 +163,81 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
     auto smooth = [&](int l, int mode) {
         const bool post = mode == POST;
         const Grid& g = a.g[l];
-        T* xv = keep(a.x[l]);
-        const T* b = keep(a.b[l]);
+        T* const xg = keep(a.x[l]);
+        T* const win = windows + a.win[l];                                  // (windowed)
+        T* const xv = windowed ? win - wlo[l][rank] : xg;
+        T* b = keep(a.b[l]);
         const T* __restrict__ L = keep(a.L[l]);
         const T* __restrict__ iD = keep(a.iD[l]);
         const T om = mode == FLAT ? T(1) : a.omega;
         const int N = keep(int(g.N)), r1 = keep(int(g.s[1])), r2 = keep(int(g.s[2])), conflicts = keep(wrap_conflicts(g));
         const Wraps wr(g);
-        const unsigned* w = words + l * CL_PAIRS * TAIL_WORDS * TAIL_THREADS + tid;
+        const unsigned* w = words + a.wo[l] + tid;
+        const int kp = a.kp[l];
         PairCells pc[CL_PAIRS];
+        unsigned in[CL_PAIRS];
+        T bv[2 * CL_PAIRS];   // right-hand side of the red and the black cell
 #pragma unroll
         for (int k = 0; k < CL_PAIRS; ++k) {
-            const unsigned w0 = w[(k * TAIL_WORDS) * TAIL_THREADS];
-            if (w0) pc[k] = PairCells(w0, w[(k * TAIL_WORDS + 1) * TAIL_THREADS]);
+            const unsigned w0 = k < kp ? w[(k * CL_WORDS) * TAIL_THREADS] : 0u;
+            if (w0) pc[k] = PairCells(w0, w[(k * CL_WORDS + 1) * TAIL_THREADS]);
+            in[k] = w0 ? pc[k].order(w[(k * CL_WORDS + TAIL_WORDS) * TAIL_THREADS]) : 0u;
+            bv[2 * k] = pc[k].red ? b[pc[k].red] : T(0);
+            bv[2 * k + 1] = pc[k].black ? b[pc[k].black] : T(0);
+            if (mode == FLAT) {   // mean-free, here and in memory
+                const T mean = T(sc[2]);
+                if (pc[k].red) b[pc[k].red] = bv[2 * k] -= mean;
+                if (pc[k].black) b[pc[k].black] = bv[2 * k + 1] -= mean;
+            }
         }
+        // v into cell I (flags f) and its ghost copies: in this block's window and those in mask m that hold it too
+        auto store = [&](unsigned I, unsigned f, unsigned m, T v) {
+            if (!windowed) {
+                tail_store<T, D>(wr, xv, I, f, v);
+                return;
+            }
+            const int gx = f & 1u ? wr.w0 : f & 2u ? -wr.w0 : 0;   // both at a single cell: the other copy below
+            xv[I] = v;
+            if (gx) xv[int(I) + gx] = v;
+            for (; m; m &= m - 1) {
+                const int r = __ffs(m) - 1;
+                T* p = cl.map_shared_rank(win, r) + (int(I) - wlo[l][r]);
+                *p = v;
+                if (gx) p[gx] = v;
+            }
+            if (!(f & 12u) && (f & 3u) != 3u) return;
+            auto ghost = [&](int J, int q) {
+                for (int r = greach[l][q][0]; r <= greach[l][q][1]; ++r)
+                    if (J >= wlo[l][r] && J <= whi[l][r]) cl.map_shared_rank(win, r)[J - wlo[l][r]] = v;
+            };
+            if ((f & 3u) == 3u) ghost(int(I) - wr.w0, 0);
+            if (f & 4u) ghost(int(I) + wr.w1, 1);
+            if (f & 8u) ghost(int(I) - wr.w1, 2);
+        };
+        auto stage = [&]() {
+            if (windowed) wsync();
+            else sync();
+        };
         const T* xc = post ? keep(a.x[l + 1]) : nullptr;
+        // From zero, the first red half-sweep reads no neighbour, and no black cell is read before its own half-sweep
+        // unless cells of a colour touch across a wrap.
+        const bool direct = mode == PRE || (mode == FLAT && !conflicts);
 #pragma unroll
         for (int k = 0; k < CL_PAIRS; ++k) {
             const int r = pc[k].red, c = pc[k].black;
+            T vr = T(0), vc = T(0);
             if (post) {
-                const unsigned par = pc[k].order(w[(k * TAIL_WORDS + 2) * TAIL_THREADS]);
-                const T vr = r ? xv[r] + xc[par & 0xFFFFu] : T(0), vc = c ? xv[c] + xc[par >> 16] : T(0);
-                if (r) tail_store<T, D>(wr, xv, r, pc[k].fl & 0xFFFFu, vr);
-                if (c) tail_store<T, D>(wr, xv, c, pc[k].fl >> 16, vc);
-            } else if (mode == FLAT) {
-                if (r) tail_store<T, D>(wr, xv, r, pc[k].fl & 0xFFFFu, T(0));
-                if (c) tail_store<T, D>(wr, xv, c, pc[k].fl >> 16, T(0));
-            } else {   // the first red half-sweep from zero; black cells are zero
-                if (r) tail_store<T, D>(wr, xv, r, pc[k].fl & 0xFFFFu, om * (b[r] * __ldg(iD + r)));
-                if (c) tail_store<T, D>(wr, xv, c, pc[k].fl >> 16, T(0));
+                const unsigned par = r || c ? pc[k].order(w[(k * CL_WORDS + 2) * TAIL_THREADS]) : 0u;
+                if (r) vr = xv[r] + xc[par & 0xFFFFu];
+                if (c) vc = xv[c] + xc[par >> 16];
+            } else if (direct && r) {
+                vr = om * (bv[2 * k] * __ldg(iD + r));
             }
+            if (r) store(r, pc[k].fl & 0xFFFFu, in[k] & 0xFFFFu, vr);
+            if (c && (post || !direct || conflicts || !windowed)) store(c, pc[k].fl >> 16, in[k] >> 16, vc);
+            else if (c) xv[c] = T(0);
         }
-        sync();
+        stage();
         auto ld = [](const T* p, unsigned o) { return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o); };
         auto nc = [](const T* p, unsigned o) { return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + o)); };
         // b - Σ c x_nb of the cell at byte offset o, and Σ c when asked for
@@ -180,7 +263,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
             return r;
         };
         const int nh = mode == FLAT ? keep(a.tail.nuc) + 1 : post ? 2 * keep(a.nu2[l]) : 2 * keep(a.nu1[l]);
-        for (int s = mode == PRE ? 1 : 0; s < nh; ++s) {
+        for (int s = direct ? 1 : 0; s < nh; ++s) {
             const int color = (s + (post ? 1 : 0)) & 1, sh = 16 * color;
             for (int cls = 0; cls <= conflicts; ++cls) {
                 if (cls & ~conflicts) continue;
@@ -190,19 +273,29 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
                 for (int k = 0; k < CL_PAIRS; ++k) {
                     const unsigned I = color ? pc[k].black : pc[k].red, o = I * unsigned(sizeof(T));
                     if (!I) continue;
-                    const T xo = ld(xv, o), d = nc(iD, o), r = gather(o, ld(b, o), nullptr);
+                    const T xo = ld(xv, o), d = nc(iD, o), r = gather(o, color ? bv[2 * k + 1] : bv[2 * k], nullptr);
                     nv[k] = om == T(1) ? r * d : fma(om, fma(r, d, -xo), xo);
                 }
 #pragma unroll
                 for (int k = 0; k < CL_PAIRS; ++k) {
                     const int I = color ? pc[k].black : pc[k].red;
                     const unsigned f = pc[k].fl >> sh & 0xFFFFu;
-                    if (I && int(f >> 6 & 7u) == cls) tail_store<T, D>(wr, xv, I, f, nv[k]);
+                    if (I && int(f >> 6 & 7u) == cls) store(I, f, in[k] >> sh & 0xFFFFu, nv[k]);
+                }
+                stage();
+            }
+        }
+        if (mode != PRE) {
+            if (windowed) {   // the finer level's prolongation and the CG read x in memory
+#pragma unroll
+                for (int k = 0; k < CL_PAIRS; ++k) {
+                    if (pc[k].red) xg[pc[k].red] = xv[pc[k].red];
+                    if (pc[k].black) xg[pc[k].black] = xv[pc[k].black];
                 }
                 sync();
             }
+            return;
         }
-        if (mode != PRE) return;
         T* res = keep(a.r[l]);
 #pragma unroll
         for (int k = 0; k < CL_PAIRS; ++k)
@@ -211,18 +304,20 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
                 const unsigned I = c ? pc[k].black : pc[k].red, o = I * unsigned(sizeof(T));
                 if (!I) continue;
                 T dd;
-                const T r = gather(o, ld(b, o), &dd);
+                const T r = gather(o, bv[2 * k + c], &dd);
                 res[I] = fma(dd, ld(xv, o), r);
             }
         sync();
         // the next level's right-hand side: its words are those of this slot's threads, the tail's of the first ones
         T* bc = keep(a.b[l + 1]);
-        const unsigned* wc = words + (l + 1) * CL_PAIRS * TAIL_WORDS * TAIL_THREADS + tid;
+        const unsigned* wc = words + a.wo[l + 1] + tid;
+        const int kc = a.kp[l + 1];
 #pragma unroll
         for (int k = 0; k < CL_PAIRS; ++k) {
-            const unsigned w0 = wc[(k * TAIL_WORDS) * TAIL_THREADS], f = wc[(k * TAIL_WORDS + 1) * TAIL_THREADS], I = w0 & 0x3FFFFFFFu;
+            if (k >= kc) continue;
+            const unsigned w0 = wc[(k * CL_WORDS) * TAIL_THREADS], f = wc[(k * CL_WORDS + 1) * TAIL_THREADS], I = w0 & 0x3FFFFFFFu;
             if (!w0) continue;
-            const T* r = res + wc[(k * TAIL_WORDS + 3) * TAIL_THREADS];
+            const T* r = res + wc[(k * CL_WORDS + 3) * TAIL_THREADS];
             bc[I] = tail_children<T, D>(r, f & 0xFFFFu, r1, r2);
             if (w0 >> 31) bc[I + 1] = tail_children<T, D>(r + (f & 512u ? 2 : 1), f >> 16, r1, r2);
         }
@@ -239,8 +334,6 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
                 if (tid == 0) sc[2] = sum / double((g0.n[0] - 2) * (g0.n[1] - 2) * (D == 3 ? g0.n[2] - 2 : 1));
             }
             __syncthreads();
-            const T mean = T(sc[2]);
-            cells(g0, [&](int, int, int, int I) { a.b[0][I] -= mean; });
             smooth(0, FLAT);
             return;
         }
@@ -285,18 +378,57 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
         return __longlong_as_double((long long)cluster_max(m));
     };
 
+    // windows: their bounds, and zeros (the ghosts of walls stay so)
+    const int tops = windowed ? a.nd + a.flat : 0;
+    if (tid < tops * CL_MAX) {
+        const int l = tid / CL_MAX, r = tid - l * CL_MAX;
+        int lo = 0, hi = -1;
+        if (r < C) cl_window<D>(a.g[l], C, r, lo, hi);
+        wlo[l][r] = lo;
+        whi[l][r] = hi;
+    }
+    if (tid < CL_LEVELS * 3) {
+        greach[tid / 3][tid % 3][0] = CL_MAX;
+        greach[tid / 3][tid % 3][1] = -1;
+    }
+    if (windowed)
+        for (int i = tid; i < a.win_values; i += TAIL_THREADS) windows[i] = T(0);
+    __syncthreads();
     // the words of this thread's pairs of every level (the last: the tail's largest, for its right-hand side)
     for (int l = 0; l <= a.nd; ++l) {
         const Grid& g = a.g[l];
-        const int n = (g.n[0] - 1) / 2 * (g.n[1] - 2) * (D == 3 ? g.n[2] - 2 : 1);
-        for (int k = 0; k < CL_PAIRS; ++k) {
-            unsigned* w = words + (l * CL_PAIRS + k) * TAIL_WORDS * TAIL_THREADS + tid;
-            if (t0 + k * stride < n)
-                tail_words<D>(g, l < a.nd ? &a.g[l + 1] : nullptr, l > 0 ? &a.g[l - 1] : nullptr, t0 + k * stride, w, TAIL_THREADS);
-            else
-                for (int q = 0; q < TAIL_WORDS; ++q) w[q * TAIL_THREADS] = 0u;
+        const int n = cl_pairs<D>(g), share = (n + C - 1) / C;
+        for (int k = 0; k < a.kp[l]; ++k) {
+            unsigned* w = words + a.wo[l] + k * CL_WORDS * TAIL_THREADS + tid;
+            const int t = rank * share + k * TAIL_THREADS + tid;
+            for (int q = 0; q < CL_WORDS; ++q) w[q * TAIL_THREADS] = 0u;
+            if (k * TAIL_THREADS + tid >= share || t >= n) continue;
+            tail_words<D>(g, l < a.nd ? &a.g[l + 1] : nullptr, l > 0 ? &a.g[l - 1] : nullptr, t, w, TAIL_THREADS);
+            if (l >= tops) continue;
+            const int I = int(w[0] & 0x3FFFFFFFu);
+            unsigned m = 0u;
+            for (int r = 0; r < C; ++r) {
+                if (r == rank) continue;
+                if (I >= wlo[l][r] && I <= whi[l][r]) m |= 1u << r;
+                if (I + 1 >= wlo[l][r] && I + 1 <= whi[l][r]) m |= 0x10000u << r;
+            }
+            w[TAIL_WORDS * TAIL_THREADS] = m;
+            const Wraps wr(g);
+            for (int c = 0; c < 2; ++c) {
+                const unsigned f = w[TAIL_THREADS] >> (16 * c) & 63u;
+                for (int q = 0; q < 3; ++q) {
+                    if (!(q == 0 ? (f & 3u) == 3u : (f >> (q + 1) & 1u) != 0u)) continue;
+                    const int J = I + c + (q == 0 ? -wr.w0 : q == 1 ? wr.w1 : -wr.w1);
+                    for (int r = 0; r < C; ++r)
+                        if (J >= wlo[l][r] && J <= whi[l][r]) {
+                            atomicMin(&greach[l][q][0], r);
+                            atomicMax(&greach[l][q][1], r);
+                        }
+                }
+            }
         }
     }
+    sync();
     if (rank == 0 && !a.flat) tail_setup<T, D>(a.tail, sm);
     T* rv = a.b[0];
     T* sv = a.x[0];
