@@ -59,7 +59,7 @@ ROOF = {
     # its unit is the whole-level half-sweep, 5 per V-cycle at nu = (2, 2) with over-relaxation (2 in the
     # pre-smoothing after the fused first one, 3 in the post-smoothing)
     "mg_fine_rbgs": dict(bytes=18, traffic=15.0, per_vcycle=5,
-                         kernel="rbgs_pair_k<float> (finest-level red-black half-sweep)"),
+                         kernel="rb_half_k (finest-level red-black half-sweep)"),
 }
 
 
@@ -588,16 +588,21 @@ def run_vof(args, world, local_rank):
     for _ in range(10):
         one()
     intf.handle.call("ia_timing", 0, T, Lc, 16)
-    bulk_ms = T[0] / max(1, Lc[0])
+    # one call: the scan of the whole grid and the three sweeps' passes over the tiles that it lists (large grids: 81 B a
+    # cell, f, u and u⁰ read, ρuf and c̄ written once), or three passes over the whole grid (33 B a cell each)
+    scan = Lc[0] == 40
+    bulk_ms, cell_bytes = T[0] / 10, 81 if scan else 99
     peak, peak_kind = measured_peak_hbm()
-    ach = 33 * N ** 3 / (bulk_ms / 1e3) / 1e9
+    ach = cell_bytes * N ** 3 / (bulk_ms / 1e3) / 1e9
     return {"workload": f"VOF-only sphere r=0.15 at (0.35,0.35,0.35), LeVeque deformation, {N}^3, CFL 0.5, "
                         f"full period T=3 ({steps} advect! steps, all timed)",
             "value": world * N ** 3 * steps / (ms / 1e3) / 1e6, "ms_per_step": ms / steps, "steps": steps,
             "l1_shape_error": l1, "mass_drift": drift, "status_codes": sorted(codes),
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                         "traffic": 31.1 * N ** 3, "kernel": "vof_bulk (read f, u_d, u⁰_d, c̄; write ρuf_d: 33 B)",
-                         "peak_kind": peak_kind, "avg_launch_ms": bulk_ms}}
+                         "traffic": (92.6 if scan else 93.3) * N ** 3,
+                         "kernel": "vof_scan and vof_bulk_tiles (81 B a cell and call)" if scan else
+                                   "vof_bulk (read f, u_d, u⁰_d, c̄; write ρuf_d: 33 B a sweep)",
+                         "peak_kind": peak_kind, "ms_per_call": bulk_ms, "avg_launch_ms": T[0] / max(1, Lc[0])}}
 
 
 def main():

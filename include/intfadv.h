@@ -340,14 +340,16 @@ int ia_poisson_smoother(ia_handle* h, int32_t kind);
 /* relaxation factor omega in (0, 2) of the V-cycle's red-black half-sweeps, x += omega (x_GS - x)
  * (no reference counterpart; default 1.15, which takes the rising-bubble solves from 12 to 10 FCG
  * iterations per step; 1 is plain Gauss-Seidel); the coarsest-level sweeps stay at 1.  The blocked
- * smoother runs only at omega = 1 (the half-sweeps are used otherwise) */
+ * smoother runs only at omega = 1 (the half-sweeps are used otherwise).  Small grids (up to 65536
+ * cells in FP32, 4096 in FP64) are solved in one launch, by half-sweeps at any omega but 1 */
 int ia_poisson_mg_relax(ia_handle* h, double omega);
 /* coefficient storage of the finest level's V-cycle smoother in the MIXED / LEARNED modes (no reference
  * counterpart): 1 = an FP16 copy of the FP32 face coefficients (relative precision 2^-11) for the
  * red-black half-sweeps and the residual restriction of that level, 0 = the FP32 coefficients.  The inner
  * FCG's operator, the coarse levels and the FP64 defect correction are not affected, so the solve still
  * stops on the FP64 true residual.  Default 1 when the coefficients 1/ρ (between 1/max(λρ,1) and
- * 1/min(λρ,1)) fit FP16's range, which IA_ERR_UNSUPPORTED reports otherwise. */
+ * 1/min(λρ,1)) fit FP16's range, which IA_ERR_UNSUPPORTED reports otherwise.  Grids solved in one launch
+ * read the FP32 coefficients. */
 int ia_poisson_coef16(ia_handle* h, int32_t on);
 /* 1: the momentum and viscous flux bulk passes use their 64-bit cell-offset variants whatever the grid
  * size; 0 (default): the 32-bit variants wherever every vector entry index fits 32 bits (fewer
@@ -363,7 +365,8 @@ int ia_poisson_mg_fine(ia_handle* h, int32_t nu1, int32_t nu2);
  * half-sweep one row behind the previous, so that the later half-sweeps read the slab from L2.  Same
  * results as whole-level half-sweeps, bit for bit.  0 = whole-level half-sweeps; otherwise at least 8.
  * Applies in 3D with walls in y.  Default 0: with two z planes per half-sweep thread the wavefront no
- * longer shortens the step (a slab within about 3/5 of L2, 64 rows at 256x512x256, ties). */
+ * longer shortens the step (a slab within about 3/5 of L2, 64 rows at 256x512x256, ties).  Grids solved in
+ * one launch have no slabs. */
 int ia_poisson_slab_rows(ia_handle* h, int32_t rows);
 /* counters since the handle's creation: [0] net applications, [1] V-cycles, [2] fallbacks
  * to the V-cycle, [3] inner FCG iterations, [4] outer corrections */
