@@ -287,7 +287,12 @@ __device__ void normal_cc(const Stencil& S, int dc, const double ref[3], double 
     }
     for (int d = 0; d < D; ++d) out[d] /= s;
 }
-// mixed Youngs–centred (src/normalEstimation.jl:185-202)
+// mixed Youngs–centred (src/normalEstimation.jl:185-202).  Candidates that are equal but for rounding count as equal, and
+// the earlier one stands, as in exact arithmetic: along an interface that varies neither in y nor in z, the y and the z
+// candidate have the same leading component, and a comparison of the two as they are takes the sign of their rounding (and
+// of what the pressure solve leaves in f), a normal that points elsewhere by a component of order one, in some cells and
+// not in others.  The candidates' components are sums of at most 9 fractions over their own 1-norm.
+constexpr double MYC_TIE = 1e-12;
 template <int D>
 __device__ void normal_myc(const Stencil& S, double n[3]) {
     normal_young<D>(S, n);
@@ -297,7 +302,7 @@ __device__ void normal_myc(const Stencil& S, double n[3]) {
     int cz = 0;
     for (int iz = 0; iz < D; ++iz) {
         normal_cc<D>(S, iz, n, tmp);
-        if (fabs(tmp[iz]) > prev) cz = iz;
+        if (fabs(tmp[iz]) > prev + MYC_TIE) cz = iz;
         prev = fabs(tmp[iz]);
     }
     normal_cc<D>(S, cz, n, tmp);

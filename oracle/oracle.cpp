@@ -309,7 +309,8 @@ void nrm_cci(const G& g, const double* f, long I, int dc, const double n[3], dou
     }
     for (int d = 0; d < g.D; ++d) out[d] /= s;
 }
-// _MYC!, normalEstimation.jl:185-202
+// _MYC!, normalEstimation.jl:185-202; candidates equal but for rounding count as equal (the first one stands, as in
+// exact arithmetic)
 void nrm_myc(const G& g, const double* f, long I, double n[3]) {
     nrm_y(g, f, I, n);
     double mx = 0;
@@ -318,7 +319,7 @@ void nrm_myc(const G& g, const double* f, long I, double n[3]) {
     double tmp[3];
     for (int iz = 0; iz < g.D; ++iz) {
         nrm_cci(g, f, I, iz, n, tmp);
-        if (std::fabs(tmp[iz]) > cur0) cz = iz;
+        if (std::fabs(tmp[iz]) > cur0 + 1e-12) cz = iz;
         cur0 = std::fabs(tmp[iz]);
     }
     nrm_cci(g, f, I, cz, n, tmp);
