@@ -210,9 +210,14 @@ __device__ __forceinline__ ff limiter_corr_ff(const FluxFF& Q, ff u, ff c, ff d)
     if (LIM == IA_LIMITER_MINMOD)   // median((3c - u)/2, c, (c + d)/2) = c + median(δ₁, 0, δ₂)/2
         return ff_scale2(ff_minmod(d1, d2), 0.5f);
     if (LIM == IA_LIMITER_VANALBADA1) {   // c + max(δ₁δ₂, 0)(δ₁ + δ₂)/(δ₁² + δ₂²)/2
-        const ff fac = (ff_zero(d1) && ff_zero(d2)) ? ff_from(0.0f)
-                                                    : ff_div(ff_add(d1, d2), ff_add(ff_mul(d1, d1), ff_mul(d2, d2)));
-        return ff_scale2(ff_mul(ff_max(ff_mul(d1, d2), ff_from(0.0f)), fac), 0.5f);
+        // The form is homogeneous of degree 1.  Differences below 2^-40 (a component that is rounding alone) are taken
+        // 2^100 times as large: their squares would leave the FP32 range, below 1e-23 to a quotient 0/0.
+        const bool tiny = fabsf(d1.hi) < 0x1p-40f && fabsf(d2.hi) < 0x1p-40f;
+        const float up = tiny ? 0x1p100f : 1.0f, down = tiny ? 0x1p-101f : 0.5f;
+        const ff a = ff_scale2(d1, up), b = ff_scale2(d2, up);
+        const ff fac = (ff_zero(a) && ff_zero(b)) ? ff_from(0.0f)
+                                                  : ff_div(ff_add(a, b), ff_add(ff_mul(a, a), ff_mul(b, b)));
+        return ff_scale2(ff_mul(ff_max(ff_mul(a, b), ff_from(0.0f)), fac), down);
     }
     if (LIM == IA_LIMITER_SWEBY || LIM == IA_LIMITER_SUPERBEE || LIM == IA_LIMITER_TVDCEN ||
         LIM == IA_LIMITER_TVDDOWN) {
