@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "capi_internal.cuh"
@@ -702,25 +703,43 @@ inline int nblk(long long n) {
     return int(b < 4096 ? (b < 1 ? 1 : b) : 4096);
 }
 
-// a convolution (flip: a data gradient) on the tile that fills the device: 32 x 8 x 4 cells, 2 planes where 4 leave
-// fewer than two blocks for a multiprocessor, 16 cells along x on short rows
+// a data gradient on the tile that fills the device: 32 x 8 x 4 cells, 2 planes where 4 leave fewer than two blocks
+// for a multiprocessor, 16 cells along x on short rows
 template <int CI, int CO, int TX, int TZ>
-cudaError_t conv32_tile(const nn::Dims& d, const float* X, const float* W, int flip, const float* b, float* Z, float* A,
-                        const float* skip, int relu, cudaStream_t st) {
+cudaError_t conv32_tile(const nn::Dims& d, const float* dY, const float* W, float* dX, cudaStream_t st) {
     using C = nn::Conv32<CI, CO, TX, TZ>;
     const long long blocks = (long long)((d.nx + TX - 1) / TX) * ((d.ny + nn::CONV_TY - 1) / nn::CONV_TY) * ((d.nz + TZ - 1) / TZ) * d.B;
     const cudaError_t e = cudaFuncSetAttribute(nn::conv32_k<CI, CO, TX, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES);
     if (e != cudaSuccess) return e;
-    { nn::conv32_k<CI, CO, TX, TZ><<<unsigned(blocks), C::THREADS, C::BYTES, st>>>(d, X, W, flip, b, Z, A, skip, relu); ia::note_launch(); }
+    { nn::conv32_k<CI, CO, TX, TZ><<<unsigned(blocks), C::THREADS, C::BYTES, st>>>(d, dY, W, dX); ia::note_launch(); }
     return cudaGetLastError();
 }
 template <int CI, int CO>
-cudaError_t conv32(const NNState* s, const nn::Dims& d, const float* X, const float* W, int flip, const float* b, float* Z,
-                   float* A, const float* skip, int relu, cudaStream_t st) {
-    if (d.nx <= 16) return conv32_tile<CI, CO, 16, 2>(d, X, W, flip, b, Z, A, skip, relu, st);
+cudaError_t conv32(const NNState* s, const nn::Dims& d, const float* dY, const float* W, float* dX, cudaStream_t st) {
+    if (d.nx <= 16) return conv32_tile<CI, CO, 16, 2>(d, dY, W, dX, st);
     const long long blocks = (long long)((d.nx + 31) / 32) * ((d.ny + nn::CONV_TY - 1) / nn::CONV_TY) * ((d.nz + 3) / 4) * d.B;
-    if (blocks < 2 * s->sms) return conv32_tile<CI, CO, 32, 2>(d, X, W, flip, b, Z, A, skip, relu, st);
-    return conv32_tile<CI, CO, 32, 4>(d, X, W, flip, b, Z, A, skip, relu, st);
+    if (blocks < 2 * s->sms) return conv32_tile<CI, CO, 32, 2>(d, dY, W, dX, st);
+    return conv32_tile<CI, CO, 32, 4>(d, dY, W, dX, st);
+}
+// a layer's forward convolution: 32 x 8 x 4 cells, 2 planes where 4 leave more than half of the multiprocessors without a
+// block (the layers together, 4 samples of 64^3: 1412 us, 1440 by the data gradient's rule; one sample 546 and 571)
+template <int CI, int CO, int TX, int TZ>
+cudaError_t fwd32_tile(const nn::Dims& d, const float* X, const float* W, const float* b, float* Z, float* A, const float* skip,
+                       int relu, cudaStream_t st) {
+    using C = nn::Fwd32<CI, CO, TX, TZ>;
+    const long long blocks = (long long)((d.nx + TX - 1) / TX) * ((d.ny + nn::CONV_TY - 1) / nn::CONV_TY) * ((d.nz + TZ - 1) / TZ) * d.B;
+    const cudaError_t e = cudaFuncSetAttribute(nn::fwd32_k<CI, CO, TX, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES);
+    if (e != cudaSuccess) return e;
+    { nn::fwd32_k<CI, CO, TX, TZ><<<unsigned(blocks), C::THREADS, C::BYTES, st>>>(d, X, W, b, Z, A, skip, relu); ia::note_launch(); }
+    return cudaGetLastError();
+}
+template <int CI, int CO>
+cudaError_t fwd32(const NNState* s, const nn::Dims& d, const float* X, const float* W, const float* b, float* Z, float* A,
+                  const float* skip, int relu, cudaStream_t st) {
+    if (d.nx <= 16) return fwd32_tile<CI, CO, 16, 2>(d, X, W, b, Z, A, skip, relu, st);
+    const long long blocks = (long long)((d.nx + 31) / 32) * ((d.ny + nn::CONV_TY - 1) / nn::CONV_TY) * ((d.nz + 3) / 4) * d.B;
+    if (2 * blocks < s->sms) return fwd32_tile<CI, CO, 32, 2>(d, X, W, b, Z, A, skip, relu, st);
+    return fwd32_tile<CI, CO, 32, 4>(d, X, W, b, Z, A, skip, relu, st);
 }
 // gradients of the weights and the bias of a layer into g (W[27][CO][CI], then b[CO])
 template <int CI, int CO>
@@ -742,16 +761,16 @@ inline float4* v4(float* p) { return reinterpret_cast<float4*>(p); }
 cudaError_t forward_f32(const NNState* s, const Graph& G, cudaStream_t st) {
     using namespace nn;
     const float* w = s->w;
-    cudaError_t e = conv32<4, 16>(s, G.f, G.x0, w + layer_w(0), 0, w + layer_b(0), G.z1, G.a1, nullptr, 1, st);
+    cudaError_t e = fwd32<4, 16>(s, G.f, G.x0, w + layer_w(0), w + layer_b(0), G.z1, G.a1, nullptr, 1, st);
     { pool_fwd_k<<<nblk(G.hf.cells() * 4), 256, 0, st>>>(G.hf, 4, v4(G.a1), v4(G.p1)); ia::note_launch(); }
-    e = e ? e : conv32<16, 32>(s, G.hf, G.p1, w + layer_w(1), 0, w + layer_b(1), G.z2, G.a2, nullptr, 1, st);
+    e = e ? e : fwd32<16, 32>(s, G.hf, G.p1, w + layer_w(1), w + layer_b(1), G.z2, G.a2, nullptr, 1, st);
     { pool_fwd_k<<<nblk(G.qt.cells() * 8), 256, 0, st>>>(G.qt, 8, v4(G.a2), v4(G.p2)); ia::note_launch(); }
-    e = e ? e : conv32<32, 32>(s, G.qt, G.p2, w + layer_w(2), 0, w + layer_b(2), G.z3, G.a3, nullptr, 1, st);
+    e = e ? e : fwd32<32, 32>(s, G.qt, G.p2, w + layer_w(2), w + layer_b(2), G.z3, G.a3, nullptr, 1, st);
     { up_fwd_k<<<nblk(G.hf.cells() * 8), 256, 0, st>>>(G.hf, 8, v4(G.a3), v4(G.a2), v4(G.u2)); ia::note_launch(); }
-    e = e ? e : conv32<32, 32>(s, G.hf, G.u2, w + layer_w(3), 0, w + layer_b(3), G.z4, G.a4, nullptr, 1, st);
+    e = e ? e : fwd32<32, 32>(s, G.hf, G.u2, w + layer_w(3), w + layer_b(3), G.z4, G.a4, nullptr, 1, st);
     { up_fwd_k<<<nblk(G.f.cells() * 8), 256, 0, st>>>(G.f, 8, v4(G.a4), nullptr, v4(G.u1)); ia::note_launch(); }
-    e = e ? e : conv32<32, 16>(s, G.f, G.u1, w + layer_w(4), 0, w + layer_b(4), G.z5, G.a5, G.a1, 1, st);
-    e = e ? e : conv32<16, 1>(s, G.f, G.a5, w + layer_w(5), 0, w + layer_b(5), nullptr, G.out, nullptr, 0, st);
+    e = e ? e : fwd32<32, 16>(s, G.f, G.u1, w + layer_w(4), w + layer_b(4), G.z5, G.a5, G.a1, 1, st);
+    e = e ? e : fwd32<16, 1>(s, G.f, G.a5, w + layer_w(5), w + layer_b(5), nullptr, G.out, nullptr, 0, st);
     return e ? e : cudaGetLastError();
 }
 
@@ -762,20 +781,20 @@ cudaError_t backward_f32(const NNState* s, const Graph& G, cudaStream_t st) {
     // data gradient of layer l
     auto W = [&](int l) { return w + layer_w(l); };
     cudaError_t e = wgrad<16, 1>(s, G.f, G.a5, G.dout, g + layer_w(5), st);
-    e = e ? e : conv32<1, 16>(s, G.f, G.dout, W(5), 1, nullptr, nullptr, G.da5, nullptr, 0, st);
+    e = e ? e : conv32<1, 16>(s, G.f, G.dout, W(5), G.da5, st);
     { relu_bwd_k<<<nblk(G.f.cells() * 4), 256, 0, st>>>(G.f, 4, v4(G.z5), v4(G.da5), v4(G.dz5)); ia::note_launch(); }
     e = e ? e : wgrad<32, 16>(s, G.f, G.u1, G.dz5, g + layer_w(4), st);
-    e = e ? e : conv32<16, 32>(s, G.f, G.dz5, W(4), 1, nullptr, nullptr, G.du1, nullptr, 0, st);
+    e = e ? e : conv32<16, 32>(s, G.f, G.dz5, W(4), G.du1, st);
     { up_bwd_relu_k<<<nblk(G.hf.cells() * 8), 256, 0, st>>>(G.hf, 8, v4(G.du1), v4(G.z4), v4(G.dz4)); ia::note_launch(); }
     e = e ? e : wgrad<32, 32>(s, G.hf, G.u2, G.dz4, g + layer_w(3), st);
-    e = e ? e : conv32<32, 32>(s, G.hf, G.dz4, W(3), 1, nullptr, nullptr, G.du2, nullptr, 0, st);
+    e = e ? e : conv32<32, 32>(s, G.hf, G.dz4, W(3), G.du2, st);
     { up_bwd_relu_k<<<nblk(G.qt.cells() * 8), 256, 0, st>>>(G.qt, 8, v4(G.du2), v4(G.z3), v4(G.dz3)); ia::note_launch(); }
     e = e ? e : wgrad<32, 32>(s, G.qt, G.p2, G.dz3, g + layer_w(2), st);
-    e = e ? e : conv32<32, 32>(s, G.qt, G.dz3, W(2), 1, nullptr, nullptr, G.dp2, nullptr, 0, st);
+    e = e ? e : conv32<32, 32>(s, G.qt, G.dz3, W(2), G.dp2, st);
     // a2 feeds the skip connection (du2) and the pooling (dp2)
     { pool_bwd_relu_k<<<nblk(G.hf.cells() * 8), 256, 0, st>>>(G.hf, 8, v4(G.du2), v4(G.dp2), v4(G.z2), v4(G.dz2)); ia::note_launch(); }
     e = e ? e : wgrad<16, 32>(s, G.hf, G.p1, G.dz2, g + layer_w(1), st);
-    e = e ? e : conv32<32, 16>(s, G.hf, G.dz2, W(1), 1, nullptr, nullptr, G.dp1, nullptr, 0, st);
+    e = e ? e : conv32<32, 16>(s, G.hf, G.dz2, W(1), G.dp1, st);
     // a1 feeds the skip connection (da5) and the pooling (dp1)
     { pool_bwd_relu_k<<<nblk(G.f.cells() * 4), 256, 0, st>>>(G.f, 4, v4(G.da5), v4(G.dp1), v4(G.z1), v4(G.dz1)); ia::note_launch(); }
     e = e ? e : wgrad<4, 16>(s, G.f, G.x0, G.dz1, g + layer_w(0), st);

@@ -1,28 +1,27 @@
-// FP32 training kernels of the learned preconditioner's network (included by nn.cu): the 3x3x3 convolution and
+// FP32 training kernels of the learned preconditioner's network (included by nn.cu): the 3x3x3 convolution,
 // its data gradient, the weight gradient, and the pooling / upsampling / ReLU passes between them.
 //
 // The contractions run on the FP32 pipes: the gradients are checked against FP64 at 5e-5 and the BF16 and TF32
 // tensor formats round their inputs to 8 and 11 bits.  The bound is therefore the FMA rate, and the kernels are
 // built so that a multiply-add costs little else: 64 (convolution) or 48 (weight gradient) accumulators a thread,
-// operands read from shared memory as 16-byte vectors and used 19 or 24 times each.
+// operands read from shared memory as vectors and used 12 to 24 times each.
 // Measured on GB300, 4 samples of 64^3 (136 GFLOP in all, 1.8 ms at the measured FMA rate): 38.4 ms for one
-// gradient with a thread per cell and scalar loads, 4.2 ms with these kernels.
+// gradient with a thread per cell and scalar loads, 4.3 ms with these kernels.
 #pragma once
 
 namespace ia {
 namespace nn {
 
-// ------------------------------------------------------------------ convolution and data gradient
-// out[p][o] = bias[o] + Σ_t Σ_c w[t][c][o] X[p + off(t)][c] on a tile of TX x 8 x TZ cells.  A thread owns 8
-// consecutive cells of a row and COT output channels.  The input tile (with its halo) is staged channel by channel,
+// ------------------------------------------------------------------ data gradient
+// dX[p][o] = Σ_t Σ_c W[26 - t][c][o] dY[p + off(t)][c] on a tile of TX x 8 x TZ cells (CI: channels of dY).  A thread owns
+// 8 consecutive cells of a row and COT channels of dX.  The tile of dY (with its halo) is staged channel by channel,
 // x fastest, CC channels at a time: for one channel and one (dy, dz) a thread reads 10 values and multiplies them
 // by the 3 x COT weights of the row, which are the same for its whole warp.
-// FLIP (the data gradient): weights of tap 26 - t with the channels exchanged.
 constexpr int CONV_TY = 8;
 template <int CI, int CO, int TX, int TZ>
 struct Conv32 {
     static constexpr int CC = CI < 8 ? CI : 8;
-    static constexpr int COT = CO < 8 ? CO : 8;
+    static constexpr int COT = 8;
     static constexpr int PX = TX + 4;                                  // row pitch: 16-byte rows, no bank conflicts at TX = 32
     static constexpr int XN = CC * (TZ + 2) * (CONV_TY + 2) * PX;      // staged inputs (floats)
     static constexpr int WN = 27 * CC * CO;                            // staged weights
@@ -32,8 +31,7 @@ struct Conv32 {
 
 template <int CI, int CO, int TX, int TZ>
 __global__ void __launch_bounds__(Conv32<CI, CO, TX, TZ>::THREADS, 512 / Conv32<CI, CO, TX, TZ>::THREADS)
-conv32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, int flip, const float* __restrict__ bias,
-         float* __restrict__ Z, float* __restrict__ A, const float* __restrict__ skip, int relu) {
+conv32_k(Dims d, const float* __restrict__ dY, const float* __restrict__ W, float* __restrict__ dX) {
     using C = Conv32<CI, CO, TX, TZ>;
     constexpr int CC = C::CC, COT = C::COT, PX = C::PX, RX = TX + 2, RY = CONV_TY + 2, RZ = TZ + 2;
     extern __shared__ __align__(16) float conv_sm[];
@@ -52,11 +50,9 @@ conv32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, int f
     const int z0 = t % ntz * TZ, b = t / ntz;
     float acc[8][COT];
 #pragma unroll
-    for (int o = 0; o < COT; ++o) {
-        const float v = bias ? __ldg(bias + o0 + o) : 0.f;
+    for (int o = 0; o < COT; ++o)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i][o] = v;
-    }
+        for (int i = 0; i < 8; ++i) acc[i][o] = 0.f;
     for (int c0 = 0; c0 < CI; c0 += CC) {
         if (c0) __syncthreads();
         for (int e = tid; e < RX * RY * RZ; e += C::THREADS) {
@@ -64,7 +60,7 @@ conv32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, int f
             const bool in = x0 + rx < d.nx + 2 && y0 + ry < d.ny + 2 && z0 + rz < d.nz + 2;   // the padded tensor
             float v[CC];
             if (in) {
-                const float* src = X + d.pos(b, x0 + rx - 1, y0 + ry - 1, z0 + rz - 1) * CI + c0;
+                const float* src = dY + d.pos(b, x0 + rx - 1, y0 + ry - 1, z0 + rz - 1) * CI + c0;
                 if (CC % 4 == 0) {
 #pragma unroll
                     for (int q = 0; q < CC / 4; ++q) {
@@ -85,7 +81,7 @@ conv32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, int f
         // weights as ws[(row (dz, dy) * CC + c) * 3 + dx][o]
         for (int e = tid; e < C::WN; e += C::THREADS) {
             const int o = e % CO, r = e / CO, dx = r % 3, rc = r / 3, c = rc % CC, tap = rc / CC * 3 + dx;
-            ws[e] = flip ? __ldg(W + ((26 - tap) * CI + c0 + c) * CO + o) : __ldg(W + (tap * CO + o) * CI + c0 + c);
+            ws[e] = __ldg(W + ((26 - tap) * CI + c0 + c) * CO + o);
         }
         __syncthreads();
 #pragma unroll 1
@@ -101,13 +97,8 @@ conv32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, int f
 #pragma unroll
                 for (int dx = 0; dx < 3; ++dx) {
                     float wv[COT];
-                    if (COT == 8) {
-                        *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(wr + dx * CO);
-                        *reinterpret_cast<float4*>(wv + 4) = *reinterpret_cast<const float4*>(wr + dx * CO + 4);
-                    } else {
-#pragma unroll
-                        for (int o = 0; o < COT; ++o) wv[o] = wr[dx * CO + o];
-                    }
+                    *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(wr + dx * CO);
+                    *reinterpret_cast<float4*>(wv + 4) = *reinterpret_cast<const float4*>(wr + dx * CO + 4);
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -116,6 +107,150 @@ conv32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, int f
                 xr += RZ * RY * PX;
                 wr += 3 * CO;
             }
+        }
+    }
+    const int y = y0 + ty, z = z0 + tz;
+    if (y >= d.ny || z >= d.nz) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int x = x0 + 8 * j + i;
+        if (x >= d.nx) break;
+        const long long q = d.pos(b, x, y, z) * CO + o0;
+#pragma unroll
+        for (int h = 0; h < 8; h += 4)
+            *reinterpret_cast<float4*>(dX + q + h) = make_float4(acc[i][h], acc[i][h + 1], acc[i][h + 2], acc[i][h + 3]);
+    }
+}
+
+// ------------------------------------------------------------------ forward convolution
+// out[p][o] = bias[o] + Σ_t Σ_c W[t][o][c] X[p + off(t)][c], summed in that order: one chain of multiply-adds from the bias,
+// tap by tap with the channels inside.  The order decides the ReLU units whose input is zero but for rounding, and a few
+// such units move a gradient by 1e-6 to 1e-5 of its norm, so that it is part of the result; the data gradient, which
+// decides nothing, takes the channels in chunks.
+// A thread owns 8 cells and COT channels as above.  All channels are staged at once, the planes of one dz at a time: TZ
+// planes in a ring (a further dz replaces one of them), and the weights of its 9 taps.  A tap reads its own 8 values of
+// the row, 1.6 times the loads of the chunked order, which still issue beside the multiply-adds; with few channels the
+// rows stay in registers for three taps.  The forward convolutions of 4 samples of 64^3: 1.41 ms so, 1.30 ms in chunks of
+// channels; of the first, whose loads are few, 126 and 124 us, of 32 -> 16 channels at full resolution (8 warps a
+// multiprocessor, as many as 32 channels leave room for) 795 and 712.
+template <int CI, int CO, int TX, int TZ>
+struct Fwd32 {
+    static constexpr int COT = CO < 8 ? CO : 8;
+    static constexpr int PX = TX + 4;
+    static constexpr int PLANE = (CONV_TY + 2) * PX;                   // one channel of one plane (floats)
+    static constexpr int XN = CI * TZ * PLANE;
+    static constexpr int WN = 9 * CI * CO;
+    static constexpr int THREADS = TX / 8 * CONV_TY * TZ * (CO / COT);
+    static constexpr int BYTES = 4 * (XN + WN);
+    // channels whose rows a thread holds at once: all of them where 10 values each fit beside the 8·COT sums
+    static constexpr int ROWS = CI * 10 + 8 * COT <= 176 && (COT == 1 || CI == 4) ? CI : 1;
+    static constexpr int UNROLL = ROWS == CI ? CI : 8;
+    // blocks on a multiprocessor: 512 threads, or what shared memory leaves
+    static constexpr int FIT = 220 * 1024 / BYTES, BLOCKS = 512 / THREADS < FIT ? 512 / THREADS : FIT < 1 ? 1 : FIT;
+};
+
+template <int CI, int CO, int TX, int TZ>
+__global__ void __launch_bounds__(Fwd32<CI, CO, TX, TZ>::THREADS, Fwd32<CI, CO, TX, TZ>::BLOCKS)
+fwd32_k(Dims d, const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ bias,
+        float* __restrict__ Z, float* __restrict__ A, const float* __restrict__ skip, int relu) {
+    using C = Fwd32<CI, CO, TX, TZ>;
+    constexpr int COT = C::COT, PX = C::PX, RX = TX + 2, RY = CONV_TY + 2, ROWS = C::ROWS;
+    extern __shared__ __align__(16) float conv_sm[];
+    float* xs = conv_sm;                 // [channel][plane mod TZ][row][x]
+    float* ws = conv_sm + C::XN;         // [tap of the plane][channel][output]
+    const int tid = threadIdx.x;
+    const int j = tid % (TX / 8), ty = tid / (TX / 8) % CONV_TY, tz = tid / (TX / 8 * CONV_TY) % TZ;
+    const int o0 = tid / (TX / 8 * CONV_TY * TZ) * COT;
+    const int ntx = (d.nx + TX - 1) / TX, nty = (d.ny + CONV_TY - 1) / CONV_TY, ntz = (d.nz + TZ - 1) / TZ;
+    int t = blockIdx.x;
+    const int x0 = t % ntx * TX;
+    t /= ntx;
+    const int y0 = t % nty * CONV_TY;
+    t /= nty;
+    const int z0 = t % ntz * TZ, b = t / ntz;
+    float acc[8][COT];
+#pragma unroll
+    for (int o = 0; o < COT; ++o) {
+        const float v = __ldg(bias + o0 + o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i][o] = v;
+    }
+    // np planes of the padded tile from plane p0 on
+    auto stage = [&](auto NP, int p0) {
+        constexpr int cells = decltype(NP)::value * RX * RY;
+#pragma unroll 4
+        for (int e = tid; e < cells * (CI / 4); e += C::THREADS) {
+            const int q = e / cells, cell = e - q * cells, rx = cell % RX, r = cell / RX, ry = r % RY, p = p0 + r / RY;
+            const bool in = x0 + rx < d.nx + 2 && y0 + ry < d.ny + 2 && z0 + p < d.nz + 2;   // the padded tensor
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in) v = __ldg(reinterpret_cast<const float4*>(X + d.pos(b, x0 + rx - 1, y0 + ry - 1, z0 + p - 1) * CI) + q);
+            float* dst = xs + (4 * q * TZ + p % TZ) * C::PLANE + ry * PX + rx;
+            dst[0] = v.x;
+            dst[TZ * C::PLANE] = v.y;
+            dst[2 * TZ * C::PLANE] = v.z;
+            dst[3 * TZ * C::PLANE] = v.w;
+        }
+    };
+    for (int dz = 0; dz < 3; ++dz) {
+        // planes dz .. dz + TZ - 1; all but the last are there from the dz before
+        if (dz) {
+            __syncthreads();
+            stage(std::integral_constant<int, 1>(), dz + TZ - 1);
+        } else {
+            stage(std::integral_constant<int, TZ>(), 0);
+        }
+        for (int e = tid; e < C::WN; e += C::THREADS) {
+            const int o = e % CO, r = e / CO, c = r % CI, tap = r / CI;
+            ws[e] = __ldg(W + ((9 * dz + tap) * CO + o) * CI + c);
+        }
+        __syncthreads();
+        const float* xp = xs + (tz + dz) % TZ * C::PLANE + ty * PX + 8 * j;
+        const float* wr = ws + o0;
+#pragma unroll 1
+        for (int dy = 0; dy < 3; ++dy) {
+            // the 8 + 2 values of a channel's row; of a few channels they stay in registers for the three taps
+            float xv[ROWS][10];
+            auto row = [&](int k, const float* xr) {
+                *reinterpret_cast<float4*>(xv[k]) = *reinterpret_cast<const float4*>(xr);
+                *reinterpret_cast<float4*>(xv[k] + 4) = *reinterpret_cast<const float4*>(xr + 4);
+                *reinterpret_cast<float2*>(xv[k] + 8) = *reinterpret_cast<const float2*>(xr + 8);
+            };
+            if (ROWS == CI) {
+#pragma unroll
+                for (int c = 0; c < ROWS; ++c) row(c, xp + dy * PX + c * TZ * C::PLANE);
+            }
+            auto tap = [&](auto DX) {
+                constexpr int dx = decltype(DX)::value;
+                const float* xr = xp + dy * PX;
+#pragma unroll C::UNROLL
+                for (int c = 0; c < CI; ++c) {
+                    const int k = ROWS == CI ? c : 0;
+                    if (ROWS != CI) {   // the tap's 8 alone
+                        if (dx == 2) *reinterpret_cast<float2*>(xv[k] + 2) = *reinterpret_cast<const float2*>(xr + 2);
+                        else *reinterpret_cast<float4*>(xv[k]) = *reinterpret_cast<const float4*>(xr);
+                        *reinterpret_cast<float4*>(xv[k] + 4) = *reinterpret_cast<const float4*>(xr + 4);
+                        if (dx == 1) xv[k][8] = xr[8];
+                        if (dx == 2) *reinterpret_cast<float2*>(xv[k] + 8) = *reinterpret_cast<const float2*>(xr + 8);
+                        xr += TZ * C::PLANE;
+                    }
+                    float wv[COT];
+                    if (COT == 8) {
+                        *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(wr + c * CO);
+                        *reinterpret_cast<float4*>(wv + 4) = *reinterpret_cast<const float4*>(wr + c * CO + 4);
+                    } else {
+#pragma unroll
+                        for (int o = 0; o < COT; ++o) wv[o] = wr[c * CO + o];
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int o = 0; o < COT; ++o) acc[i][o] = fmaf(wv[o], xv[k][i + dx], acc[i][o]);
+                }
+                wr += CI * CO;
+            };
+            tap(std::integral_constant<int, 0>());
+            tap(std::integral_constant<int, 1>());
+            tap(std::integral_constant<int, 2>());
         }
     }
     const int y = y0 + ty, z = z0 + tz;
