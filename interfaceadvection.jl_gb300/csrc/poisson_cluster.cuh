@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
         return warp_sum(lane < C ? __ldcg(a.partial + slot * CL_MAX + lane) : 0.0);
     };
     // A thread's pairs of level l: pre-smoothing (from x = 0) and the residual (PRE), prolongation and post-smoothing
-    // (POST), or the coarsest level's sweeps from x = 0 on the mean-free right-hand side (FLAT).
+    // (POST), or the coarsest level's sweeps from x = 0 on the right-hand side less its mean (FLAT).
     // What a thread needs of its cells is in shared memory (tail_words); every operand of a cell lies at its byte
     // offset from a pointer that is the same for all threads, as copies of the cells across a periodic wrap are kept in
     // x's ghosts (tail_store).
@@ -184,10 +184,14 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
             in[k] = w0 ? pc[k].order(w[(k * CL_WORDS + TAIL_WORDS) * TAIL_THREADS]) : 0u;
             bv[2 * k] = pc[k].red ? b[pc[k].red] : T(0);
             bv[2 * k + 1] = pc[k].black ? b[pc[k].black] : T(0);
-            if (mode == FLAT) {   // mean-free, here and in memory
+            if (mode == FLAT) {
+                // mean-free.  In FP64 the right-hand side in memory is the CG's residual, which the stopping test reads:
+                // it keeps its mean.  The mixed mode's inner residual loses it there, too (the outer one is formed anew).
                 const T mean = T(sc[2]);
-                if (pc[k].red) b[pc[k].red] = bv[2 * k] -= mean;
-                if (pc[k].black) b[pc[k].black] = bv[2 * k + 1] -= mean;
+                if (pc[k].red) bv[2 * k] -= mean;
+                if (pc[k].black) bv[2 * k + 1] -= mean;
+                if (MIXED && pc[k].red) b[pc[k].red] = bv[2 * k];
+                if (MIXED && pc[k].black) b[pc[k].black] = bv[2 * k + 1];
             }
         }
         // v into cell I (flags f) and its ghost copies: in this block's window and those in mask m that hold it too
