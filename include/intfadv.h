@@ -283,7 +283,8 @@ int ia_metrics(ia_handle* h, const double* u, const double* f, const double* ome
  * 11 momentum update, 12 update/projection, 13 finest-level red-black
  * half-sweeps, 14 learned preconditioner, 15 finest-level first half-sweeps),
  * then, if enable >= 0, resets the totals and switches recording on (1) or
- * off (0). */
+ * off (0).  While recording, small grids are solved by the same iteration in
+ * launches of their own (not in one); a solve on one level stays one launch, of family 4. */
 int ia_timing(ia_handle* h, int32_t enable, double* ms_out, int64_t* launches_out, int32_t n);
 
 /* Measured FMA throughput of the current device, FP64 and FP32, in fused multiply-adds per second
@@ -341,7 +342,8 @@ int ia_poisson_smoother(ia_handle* h, int32_t kind);
  * (no reference counterpart; default 1.15, which takes the rising-bubble solves from 12 to 10 FCG
  * iterations per step; 1 is plain Gauss-Seidel); the coarsest-level sweeps stay at 1.  The blocked
  * smoother runs only at omega = 1 (the half-sweeps are used otherwise).  Small grids (up to 65536
- * cells in FP32, 4096 in FP64) are solved in one launch, by half-sweeps at any omega but 1 */
+ * cells in FP32, 4096 in FP64) are solved in one launch, by half-sweeps at any omega but 1.  2D grids
+ * of up to about 65000 cells with an odd extent and a side above 96 have one level, swept as the coarsest one */
 int ia_poisson_mg_relax(ia_handle* h, double omega);
 /* coefficient storage of the finest level's V-cycle smoother in the MIXED / LEARNED modes (no reference
  * counterpart): 1 = an FP16 copy of the FP32 face coefficients (relative precision 2^-11) for the

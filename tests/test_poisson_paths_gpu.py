@@ -1,0 +1,67 @@
+"""The forms that a pressure solve of a small grid takes: one launch, or many while launch times are recorded.
+
+On one level (2D, odd, a side above 96 cells) there is one form alone, whatever is recorded and however the smoother is
+set, and the bits are the same.  On a hierarchy the two do the same iteration: after three Krylov steps the pressures
+differ by rounding alone, some 50 operations a V-cycle and cell over up to six levels (2e-5 of the largest pressure in
+FP32, 1e-13 in FP64), and a solve takes as many steps, but for one where a residual lies at the tolerance.
+"""
+import ctypes as C
+
+import pytest
+import torch
+
+import intfadv as ia
+from intfadv import _lib
+from intfadv.fields import fzeros, ptr
+from test_ragged_multigrid_gpu import system
+
+pytestmark = pytest.mark.gpu
+
+
+def solve(dims, perdir, poisson, sys_, tol, itmx, timing=False, smoother=None):
+    L, z, _ = sys_
+    h = ia.Handle(ia.make_config(dims, perdir=perdir, poisson=poisson, lrho=0.05))
+    if poisson == "mixed":
+        ia.set_poisson_coef16(h, False)     # the one-launch form reads FP32 coefficients
+    if smoother:
+        ia.set_smoother(h, *smoother)
+    if timing:
+        _lib.check(h.call("ia_timing", 1, None, None, 0), "ia_timing")
+    x, it, res = fzeros(z.shape), C.c_int32(), C.c_double()
+    n0 = _lib.load().ia_launch_count()
+    h.call("ia_poisson_solve", ptr(x), ptr(z), ptr(L), tol, itmx, C.byref(it), C.byref(res))
+    x = x[(slice(1, -1),) * len(dims)]
+    return x - x.mean(), it.value, _lib.load().ia_launch_count() - n0
+
+
+ONE_LEVEL = [((161, 97), ()), ((99, 8), ()), ((131, 98), (1,)), ((255, 255), ())]
+
+
+@pytest.mark.parametrize("poisson", ["fp64", "mixed"])
+@pytest.mark.parametrize("dims,perdir", ONE_LEVEL)
+def test_one_level_whatever_is_set(cuda, dims, perdir, poisson):
+    sys_ = system(dims, perdir, lrho=0.05)
+    x, it, n = solve(dims, perdir, poisson, sys_, 1e-8, 3000)
+    assert n == solve(dims, perdir, poisson, sys_, 1e-8, 5)[2]      # one launch, however many iterations
+    for kw in (dict(timing=True), dict(smoother=("halfsweep", 1.0)), dict(smoother=("blocked", 1.0))):
+        y, jt, m = solve(dims, perdir, poisson, sys_, 1e-8, 3000, **kw)
+        assert jt == it and m == n and torch.equal(x, y)
+
+
+HIERARCHY = [
+    ((160, 96), (), "mixed"), ((61, 87), (), "mixed"), ((254, 250), (1,), "mixed"), ((41, 35, 30), (), "mixed"),
+    ((32, 64, 32), (0, 2), "mixed"), ((33, 36, 50), (1,), "mixed"), ((60, 50), (0,), "fp64"), ((61, 55), (), "fp64"),
+    ((16, 15, 14), (), "fp64"), ((12, 18, 16), (0, 1, 2), "fp64"),
+]
+
+
+@pytest.mark.parametrize("dims,perdir,poisson", HIERARCHY)
+def test_one_launch_and_many(cuda, dims, perdir, poisson):
+    sys_ = system(dims, perdir, lrho=0.05)
+    a, ita, n = solve(dims, perdir, poisson, sys_, 1e-30, 3)
+    b, itb, m = solve(dims, perdir, poisson, sys_, 1e-30, 3, timing=True)
+    assert ita == itb == 3 and n < m
+    assert n == solve(dims, perdir, poisson, sys_, 1e-30, 6)[2]     # the one-launch form was taken
+    assert float((a - b).abs().max()) <= (1e-4 if poisson == "mixed" else 1e-12) * float(b.abs().max())
+    ita, itb = (solve(dims, perdir, poisson, sys_, 1e-10, 400, timing=t)[1] for t in (False, True))
+    assert abs(ita - itb) <= 1
