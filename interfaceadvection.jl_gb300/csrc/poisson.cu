@@ -2081,11 +2081,20 @@ static cudaError_t vcycle(ia_handle* h, PoissonMG* mg, int l, cudaStream_t st, i
             }
         }
     };
-    // pre-smoothing: first (black with the red values in place), then (red, black) nu1 - 1 times
-    chain(2 * nu1_here - 1, [&](int s, int y0, int y1) {
-        if (s == 0) first(false, y0, y1);
-        else half((s & 1) ? 0 : 1, y0, y1);
-    }, true);
+    if (conf) {
+        // cells of one colour touch across a wrap, and the fused first half-sweep would take a black neighbour there for
+        // a red one: (red, black) nu1 times from x = 0
+        cudaError_t e = cudaMemsetAsync(x, 0, sizeof(T) * (size_t)L.g.N, st);
+        if (e != cudaSuccess) return e;
+        for (int s = 0; s < 2 * nu1_here; ++s) half(s & 1, 1, L.g.n[1] - 1);
+        restrict_rows(1, C.g.n[1] - 1);
+    } else {
+        // pre-smoothing: first (black with the red values in place), then (red, black) nu1 - 1 times
+        chain(2 * nu1_here - 1, [&](int s, int y0, int y1) {
+            if (s == 0) first(false, y0, y1);
+            else half((s & 1) ? 0 : 1, y0, y1);
+        }, true);
+    }
     cudaError_t e = vcycle<T>(h, mg, l + 1, st, nu1, nu2, nuc);
     if (e != cudaSuccess) return e;
     if (nu2_here == 0 || conf) {

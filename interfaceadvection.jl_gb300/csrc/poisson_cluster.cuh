@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
         const T* xc = post ? keep(a.x[l + 1]) : nullptr;
         // From zero, the first red half-sweep reads no neighbour, and no black cell is read before its own half-sweep
         // unless cells of a colour touch across a wrap.
-        const bool direct = mode == PRE || (mode == FLAT && !conflicts);
+        const bool direct = !post && !conflicts;
 #pragma unroll
         for (int k = 0; k < CL_PAIRS; ++k) {
             const int r = pc[k].red, c = pc[k].black;
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) solve_cluster_k(const __grid_con
                 vr = om * (bv[2 * k] * __ldg(iD + r));
             }
             if (r) store(r, pc[k].fl & 0xFFFFu, in[k] & 0xFFFFu, vr);
-            if (c && (post || !direct || conflicts || !windowed)) store(c, pc[k].fl >> 16, in[k] >> 16, vc);
+            if (c && (!direct || !windowed)) store(c, pc[k].fl >> 16, in[k] >> 16, vc);
             else if (c) xv[c] = T(0);
         }
         stage();

@@ -53,9 +53,12 @@ HIERARCHY = [
     ((32, 64, 32), (0, 2), "mixed"), ((33, 36, 50), (1,), "mixed"), ((60, 50), (0,), "fp64"), ((61, 55), (), "fp64"),
     ((16, 15, 14), (), "fp64"), ((12, 18, 16), (0, 1, 2), "fp64"),
 ]
+# odd periodic extents: cells of one colour touch across the wrap
+ODD_WRAPS = [((25, 26, 23), (0, 2), "mixed"), ((33, 17), (0, 1), "mixed"), ((95, 64), (0,), "mixed"), ((33, 17), (0, 1), "fp64"),
+             ((27, 21, 7), (0, 1, 2), "fp64"), ((10, 35, 11), (1,), "fp64")]
 
 
-@pytest.mark.parametrize("dims,perdir,poisson", HIERARCHY)
+@pytest.mark.parametrize("dims,perdir,poisson", HIERARCHY + ODD_WRAPS)
 def test_one_launch_and_many(cuda, dims, perdir, poisson):
     sys_ = system(dims, perdir, lrho=0.05)
     a, ita, n = solve(dims, perdir, poisson, sys_, 1e-30, 3)
