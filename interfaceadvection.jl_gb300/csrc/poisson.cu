@@ -1398,7 +1398,7 @@ __device__ void fcg_alpha(FcgDev* S, double pq) {
 }
 
 // ---- FP64 Krylov kernels (IA_POISSON_FP64).  As the FP32 ones below, with the scalars on the device; the vectors
-// are the library's, whose ghost entries stay zero, so they are streamed whole.
+// are the library's, whose ghost entries are zero here, so they are streamed whole.
 // q = A p and partial sums of p·q, ZT planes a thread, one chain of multiply-adds a cell; the rows follow one another
 // through the lanes
 template <int D, int ZT>
@@ -1571,8 +1571,8 @@ __global__ void __launch_bounds__(256, MV_RESIDENT) matvec32_tile_k(Grid g, Ends
 }
 
 // Whole-array FP32 vector kernels of the inner solve.  Only interior cells of these vectors are
-// ever written, so their ghost entries stay zero and sums and updates over all N entries equal
-// those over the interior; the arrays are streamed as 16-byte vectors (cudaMalloc alignment),
+// written (the one-launch solver's copies in ghosts are cleared: clear_wrap_copies), so their ghost
+// entries stay zero and sums and updates over all N entries equal those over the interior; the arrays are streamed as 16-byte vectors (cudaMalloc alignment),
 // the N mod 4 tail by the first threads.
 __global__ void __launch_bounds__(256, VB_RESIDENT) dot2_32_k(long long n, const float* __restrict__ sv, const float* __restrict__ q,
                           const float* __restrict__ r, double* __restrict__ partial, FcgDev* S, int first) {
@@ -2610,6 +2610,7 @@ static cudaError_t cluster_solve(ia_handle* h, double* xv, const double* zz, con
         tail_layout<T>(mg, l0).bytes() + cl_layout<D>(mg, lt, C, nullptr, nullptr) > (size_t)CL_BYTES)
         return cudaSuccess;
     *done = true;
+    mg->wrap_copies = true;
     SolveArgs<T> a;
     const size_t words = cl_layout<D>(mg, lt, C, a.kp, a.wo);
     a.tail = tail_args<T>(mg, l0, mg->nu1, mg->nu2, mg->nuc);
@@ -2718,6 +2719,31 @@ int poisson_residual(ia_handle* h, double* r, const double* x, const double* z, 
 }
 
 // Solve A x = z to L∞(z - A x) <= tol (x holds the initial guess); L = μ₀.
+// The many-launch solvers stream whole vectors, whose ghost entries have to be zero.  The one-launch solver keeps copies of
+// cells across a wrap in the ghosts of x and takes them into p and e: they are cleared when the other form follows (a copy
+// of an infinity or a NaN would otherwise stay in its sums for good).
+static cudaError_t clear_wrap_copies(ia_handle* h) {
+    PoissonMG* mg = h->mg;
+    if (!mg->wrap_copies) return cudaSuccess;
+    const bool fp64 = h->cfg.poisson_mode == IA_POISSON_FP64;
+    cudaError_t e = cudaSuccess;
+    auto clear = [&](void* v, size_t bytes) { e = e ? e : cudaMemsetAsync(v, 0, bytes, h->stream); };
+    for (int l = 0; l < mg->nlev; ++l) {
+        const size_t n = (size_t)mg->lev[l].g.N;
+        if (fp64) clear(mg->lev[l].x, 8 * n);
+        else clear(mg->lev[l].x32, 4 * n);
+    }
+    const size_t N = (size_t)h->g.N;
+    if (fp64) {
+        clear(mg->p, 8 * N);
+    } else {
+        clear(mg->p32, 4 * N);
+        clear(mg->e32, 4 * N);
+    }
+    if (e == cudaSuccess) mg->wrap_copies = false;
+    return e;
+}
+
 int poisson_solve(ia_handle* h, double* xv, const double* zz, const double* L, double tol, int itmx, int* iters,
                   double* resid) {
     PoissonMG* mg = h->mg;
@@ -2734,6 +2760,7 @@ int poisson_solve(ia_handle* h, double* xv, const double* zz, const double* L, d
                             : cluster_solve<float, 2>(h, xv, zz, L, tol, itmx, iters, resid, &done);
         if (e != cudaSuccess) return IA_ERR_CUDA;
         if (done) return (*resid <= tol) ? IA_OK : IA_WARN_NOT_CONVERGED;
+        if (clear_wrap_copies(h) != cudaSuccess) return IA_ERR_CUDA;
     }
     if (h->cfg.poisson_mode != IA_POISSON_FP64) {
         if (h->cfg.poisson_mode == IA_POISSON_LEARNED && mg_setup(h, L) != cudaSuccess) return IA_ERR_CUDA;

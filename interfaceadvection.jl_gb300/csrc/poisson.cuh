@@ -80,6 +80,7 @@ struct PoissonMG {
     int slab_rows = 0;                                                // finest-level wavefront slab (rows; 0 off)
     int nsm = 0;                                                      // multiprocessors of the device
     int cluster = -1;                                                 // blocks of the one-launch solver's cluster
+    bool wrap_copies = false;                                         // it has left copies across wraps in ghost cells
     // each precision's finest-level V-cycle is captured once into a CUDA graph (its launch
     // sequence and arguments are fixed for the handle) and replayed; recaptured when the
     // smoothing parameters change
