@@ -343,7 +343,8 @@ int ia_poisson_smoother(ia_handle* h, int32_t kind);
  * iterations per step; 1 is plain Gauss-Seidel); the coarsest-level sweeps stay at 1.  The blocked
  * smoother runs only at omega = 1 (the half-sweeps are used otherwise).  Small grids (up to 65536
  * cells in FP32, 4096 in FP64) are solved in one launch, by half-sweeps at any omega but 1.  2D grids
- * of up to about 65000 cells with an odd extent and a side above 96 have one level, swept as the coarsest one */
+ * of up to about 65000 cells with an odd extent and a side above 96 are solved on one level, swept as the
+ * coarsest one, for at most three quarters of the allowed iterations */
 int ia_poisson_mg_relax(ia_handle* h, double omega);
 /* coefficient storage of the finest level's V-cycle smoother in the MIXED / LEARNED modes (no reference
  * counterpart): 1 = an FP16 copy of the FP32 face coefficients (relative precision 2^-11) for the
