@@ -53,6 +53,9 @@ HIERARCHY = [
     ((160, 96), (), "mixed"), ((61, 87), (), "mixed"), ((254, 250), (1,), "mixed"), ((41, 35, 30), (), "mixed"),
     ((32, 64, 32), (0, 2), "mixed"), ((33, 36, 50), (1,), "mixed"), ((60, 50), (0,), "fp64"), ((61, 55), (), "fp64"),
     ((16, 15, 14), (), "fp64"), ((12, 18, 16), (0, 1, 2), "fp64"),
+    # levels that halve evenly, whose launches have kernels of their own
+    ((32, 34, 38), (), "mixed"), ((40, 32, 32), (0, 1, 2), "mixed"), ((64, 8, 72), (1,), "mixed"), ((72, 64, 8), (2,), "mixed"),
+    ((4, 80, 112), (0,), "mixed"),
 ]
 # odd periodic extents: cells of one colour touch across the wrap
 ODD_WRAPS = [((25, 26, 23), (0, 2), "mixed"), ((33, 17), (0, 1), "mixed"), ((95, 64), (0,), "mixed"), ((33, 17), (0, 1), "fp64"),
@@ -82,3 +85,24 @@ def test_density_ratio_of_a_thousand_beside_the_limits(cuda, dims, most, poisson
     _lib.check(h.call("ia_poisson_solve", ptr(x), ptr(z), ptr(L), 1e-10, max(most, 200), C.byref(it), C.byref(res)), "ia_poisson_solve")
     assert it.value <= most
     assert float((z[1:-1, 1:-1] - apply(Li, x[1:-1, 1:-1])).abs().max()) <= 2e-10
+
+
+SIZES = [((66, 34, 38), ()), ((64, 48, 40), (0, 1, 2)), ((128, 8, 72), (1,)), ((72, 128, 8), (2,)), ((130, 66, 10), (0, 1))]
+
+
+@pytest.mark.parametrize("nu,omega", [((2, 2), 1.15), ((1, 1), 1.15), ((1, 1), 1.0), ((1, 2), 1.0)])
+@pytest.mark.parametrize("dims,perdir", SIZES)
+def test_fp16_coefficients_that_are_exact(cuda, dims, perdir, nu, omega):
+    # coefficients 1/4, 1/2, 1: their FP16 copies are exact, and the kernels that read those do the same arithmetic
+    L, z, _ = system(dims, perdir)
+    L.copy_(torch.where(L > 0, torch.exp2(-torch.floor(torch.log2(L.clamp_min(1.0)) / 4)), 0.0))
+    got = []
+    for on in (False, True):
+        h = ia.Handle(ia.make_config(dims, perdir=perdir, poisson="mixed", lrho=0.05))
+        ia.set_poisson_coef16(h, on)
+        ia.set_smoother(h, "halfsweep", omega)
+        _lib.check(h.call("ia_poisson_mg_params", nu[0], nu[1], 16), "ia_poisson_mg_params")
+        x, it, res = fzeros(z.shape), C.c_int32(), C.c_double()
+        h.call("ia_poisson_solve", ptr(x), ptr(z), ptr(L), 1e-30, 4, C.byref(it), C.byref(res))
+        got.append((x, res.value))
+    assert got[0][1] == got[1][1] and torch.equal(got[0][0], got[1][0])
