@@ -211,7 +211,8 @@ int ia_bc_velocity(ia_handle* h, double* a);
 /* Pressure solve of inproject!(::MultiLevelPoisson) — src/flow.jl:343-347
  * (WaterLily solver!): A x = z with the face coefficients L (μ₀), x holding the
  * initial guess; stops when the L-infinity FP64 residual is <= tol or after itmx
- * iterations (IA_WARN_NOT_CONVERGED). */
+ * iterations (IA_WARN_NOT_CONVERGED).  The residual is z - A x in the MIXED and LEARNED
+ * modes and the CG's own in FP64, which differs from it by rounding. */
 int ia_poisson_solve(ia_handle* h, double* x, const double* z, const double* L, double tol,
                      int32_t itmx, int32_t* iters, double* resid);
 

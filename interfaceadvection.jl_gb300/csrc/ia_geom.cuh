@@ -18,8 +18,9 @@ namespace ia {
 // cubics of the plane constant are one.  Faces of a sphere in 256^3 cells, one sweep: 56 us with every division and two
 // cubics, 44 us so.
 
-// x / y from r = 1/y (correctly rounded): Markstein's final step, the quotient that the division gives; the division
-// itself where r is near the ends of the range (a velocity or a difference of fractions below 1e-290)
+// x / y from r = 1/y: Markstein's final step.  With r correctly rounded it is the quotient that the division gives; with a
+// reciprocal that is a product (of 6 m3 from that of m3) it can be the neighbouring number.  The division itself where r is
+// near the ends of the range (a velocity or a difference of fractions below 1e-290)
 __device__ __forceinline__ double quot(double x, double y, double r) {
     const int e = __double2hiint(r) & 0x7FF00000;
     if (e < (64 << 20) || e > ((2047 - 64) << 20)) return x / y;

@@ -14,16 +14,18 @@
 //    before and ν₂ black→red after, so the V-cycle is a symmetric
 //    preconditioner; the coarsest level is solved by one block with a fixed
 //    number of symmetric sweeps on the mean-free right-hand side;
-//  * flexible CG in FP64 around it (β from the residual change, so an
-//    inexact FP32 V-cycle stays admissible), stopping on the L∞ norm of the
-//    FP64 true residual of the dt-scaled system.
+//  * flexible CG around it (β from the residual change, so an inexact
+//    V-cycle stays admissible).
 //
-// IA_POISSON_FP64 runs the V-cycle in FP64; IA_POISSON_MIXED runs it in FP32
-// (FP32 copies of every level's operator), the defect correction, matvec,
-// dot products and updates staying FP64.  IA_POISSON_LEARNED keeps the MIXED
-// structure and preconditions the inner FCG with the conv net (nn.cu), composed
-// with the V-cycle (hybrid) or alone; an outer correction that fails to halve
-// the FP64 true residual switches the rest of the solve to the plain V-cycle.
+// IA_POISSON_FP64 runs all of it in FP64 and stops on the L∞ norm of the CG's
+// residual, which starts as the true one of the dt-scaled system and follows
+// its recurrence (apart by rounding alone).  IA_POISSON_MIXED corrects in FP64
+// with inner CG solves in FP32 (FP32 copies of every level's operator) and
+// stops on the FP64 true residual, formed anew after every correction.
+// IA_POISSON_LEARNED keeps the MIXED structure and preconditions the inner FCG
+// with the conv net (nn.cu), composed with the V-cycle (hybrid) or alone; an
+// outer correction that fails to halve the FP64 true residual switches the
+// rest of the solve to the plain V-cycle.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1043,8 +1045,10 @@ template <class T> constexpr long long tail_pairs() { return sizeof(T) == 4 ? TA
 
 // ---- the one-launch solver of small grids (poisson_cluster.cuh)
 // Interior cells up to which it is used, and pairs of cells of its tail's largest level.  Measured on GB300, a step
-// with the multi-launch solver and on this path: FP32 (mixed) 41x35x30 4.3 and 2.8 ms, 32x64x32 4.9 and 4.2 ms; FP64
-// 128x64 2.4 and 2.6 ms (16 multiprocessors have a tenth of the device's FP64 pipes), 64x64 the same.
+// with the multi-launch solver and on this path: FP32 (mixed) 41x35x30 4.3 and 2.8 ms, 32x64x32 4.9 and 4.2 ms.  The FP64
+// limit is from before x lay in shared memory in 2D and the iteration in one cluster (128x64 2.4 and 2.6 ms then; 16
+// multiprocessors have a tenth of the device's FP64 pipes) and is low by now: 128x64 2.32 and 2.15 ms, 128x128 2.50 and
+// 2.27, 192x128 2.20 and 2.25, 256x192 2.91 and 3.36; 24x20x16 3.16 and 2.41, 32x32x16 3.72 and 2.95.
 template <class T> constexpr long long cluster_cells() { return sizeof(T) == 4 ? 65536 : 4096; }
 template <class T> constexpr long long cluster_tail_pairs() { return sizeof(T) == 4 ? 512 : 128; }
 
