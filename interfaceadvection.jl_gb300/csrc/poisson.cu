@@ -1050,6 +1050,7 @@ template <class T> constexpr long long tail_pairs() { return sizeof(T) == 4 ? TA
 // multiprocessors have a tenth of the device's FP64 pipes) and is low by now: 128x64 2.32 and 2.15 ms, 128x128 2.50 and
 // 2.27, 192x128 2.20 and 2.25, 256x192 2.91 and 3.36; 24x20x16 3.16 and 2.41, 32x32x16 3.72 and 2.95.
 template <class T> constexpr long long cluster_cells() { return sizeof(T) == 4 ? 65536 : 4096; }
+constexpr int CL_ITERATIONS = 2000;   // a launch: up to 0.3 s
 template <class T> constexpr long long cluster_tail_pairs() { return sizeof(T) == 4 ? 512 : 128; }
 
 // ------------------------------------------------------------------ Krylov kernels
@@ -2650,7 +2651,6 @@ static cudaError_t cluster_solve(ia_handle* h, bool flat, double* xv, const doub
     a.diag64 = mg->diag64;
     a.tol = tol;
     a.inner_rtol = mg->inner_rtol;
-    a.itmx = itmx;
     a.inner_max = mg->inner_max;
     a.partial = mg->partial;
     a.out = reinterpret_cast<SolveOut*>(mg->dsc);
@@ -2689,21 +2689,27 @@ static cudaError_t cluster_solve(ia_handle* h, bool flat, double* xv, const doub
     cfg.stream = h->stream;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    const int tk = timing_begin(h, TK_MG_SMOOTH);   // (on one level: all of the solve)
-    cudaError_t e = cudaLaunchKernelEx(&cfg, solve_cluster_k<T, D>, a);
-    ia::note_launch();
-    timing_end(h, tk);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(mg->hsc, a.out, sizeof(SolveOut), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return e;
+    // at most CL_ITERATIONS a launch: a solve that is allowed any number of them and does not converge must not hold the
+    // device in one kernel
     SolveOut o;
-    std::memcpy(&o, mg->hsc, sizeof(o));
-    mg->stats[1] += o.vcycles;
-    if (sizeof(T) == 4) {
-        mg->stats[3] += o.total;
-        mg->stats[4] += o.outer;
-    }
-    *iters = o.total;
+    *iters = 0;
+    do {
+        a.itmx = std::min(itmx - *iters, CL_ITERATIONS);
+        const int tk = timing_begin(h, TK_MG_SMOOTH);   // (on one level: all of the solve)
+        cudaError_t e = cudaLaunchKernelEx(&cfg, solve_cluster_k<T, D>, a);
+        ia::note_launch();
+        timing_end(h, tk);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(mg->hsc, a.out, sizeof(SolveOut), cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        if (e != cudaSuccess) return e;
+        std::memcpy(&o, mg->hsc, sizeof(o));
+        mg->stats[1] += o.vcycles;
+        if (sizeof(T) == 4) {
+            mg->stats[3] += o.total;
+            mg->stats[4] += o.outer;
+        }
+        *iters += o.total;
+    } while (!(o.res <= tol) && *iters < itmx && o.total == a.itmx);   // (less: a breakdown)
     *resid = o.res;
     return cudaSuccess;
 }

@@ -106,3 +106,14 @@ def test_fp16_coefficients_that_are_exact(cuda, dims, perdir, nu, omega):
         h.call("ia_poisson_solve", ptr(x), ptr(z), ptr(L), 1e-30, 4, C.byref(it), C.byref(res))
         got.append((x, res.value))
     assert got[0][1] == got[1][1] and torch.equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("dims,perdir", [((20, 18, 16), (0, 2)), ((60, 50), ()), ((99, 8), ())])
+def test_many_iterations_take_launches_of_two_thousand(cuda, dims, perdir):
+    # a tolerance out of reach: all allowed iterations, and no launch that holds the device for all of them
+    sys_ = system(dims, perdir, lrho=0.05)
+    a, ita, n = solve(dims, perdir, "mixed", sys_, 1e-30, 100)
+    b, itb, m = solve(dims, perdir, "mixed", sys_, 1e-30, 4100)
+    assert ita == 100 and itb == 4100
+    assert m == n + (2 if len(dims) == 3 or dims[0] % 2 == 0 else 1)   # one level: 3075 of them, then 1025 on the hierarchy
+    assert float((a - b).abs().max()) <= 1e-9 * float(b.abs().max())
